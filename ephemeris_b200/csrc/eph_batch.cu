@@ -1,14 +1,12 @@
-// eph_batch.cu - batched ensembles: many independent systems integrated in one persistent launch.
+// eph_batch.cu - batched ensembles: many independent systems integrated in one call.
 //
 // Each system runs the reference's msystem::integrate (mass.cpp:399-442) on its own dt, step count and
 // ephemeris time. Systems whose bodies are all point-like (no tide, rotational deformation, static
 // harmonics, spin, luminosity, radiation receptance, geopotential or ring: the Newtonian + 1PN systems of
-// an ensemble) run in `ensemble_kernel`: one CTA integrates one whole system, so a stage needs only
-// CTA barriers, and persistent CTAs take systems from an atomic queue, heaviest (bodies^2 x steps) first.
-// The bodies' stage data sit in shared memory as structure-of-arrays rows; the stage values f_j and the
-// start-of-step state sit in global scratch (L2-resident for ensemble sizes), and each body's thread
-// forms sum_j a_kj f_j at its state update (independent loads, ascending j as in the reference). Any other system
-// of the batch (a full-physics body, or more bodies than one CTA's shared memory holds) is integrated by
+// an ensemble) run in `ensemble_kernel`: a system is integrated by one CTA, or by the CTAs of one thread-block
+// cluster, so a stage needs only CTA or cluster barriers, and persistent CTAs take systems from an atomic
+// queue, longest first. The bodies' stage data, and the stage accelerations where they fit, sit in shared memory.
+// Any other system of the batch (a full-physics body, or more bodies than shared memory holds) is integrated by
 // the per-system persistent kernel of eph_step.cu through a context, one after another.
 //
 // Physics per pair (the point-class branches of the reference):
@@ -17,11 +15,11 @@
 //   prepare beta = v / c, beta^2, phi / c^2, a_N / c^2 (PREPARE_RELATIVITY, mass.impl:76-80)
 //   pass B  EIH 1PN (RELATIVITY, mass.impl:82-97) and the per-pair maxima of 1/r and GM_j/r^3
 //           (RungeKutta.cu:229-230), recomputed exactly for the extremal pair; in the mixed-precision form
-//           (eph_batch_set_precision) the 1PN terms in FP32 (pair_point_b32)
+//           (eph_batch_set_precision) the 1PN terms in FP32 (sweep_point_b32)
 //   final   phi c^2, a_N c^2 (FINALIZE_RELATIVITY, mass.impl:133-135); f = (gaccel + daccel) + naccel
 // For such bodies the reference's angular velocity, G*L and harmonics stay constant (w = G*L = 0), the
 // frame rotations are the identity and only the end-of-step orthogonalisation of the frame acts
-// (mass.h:147-150); the RK12 combination and state update are those of RungeKutta.impl:148-186.
+// (mass.h:147-150); the RK12 combination is RungeKutta.impl:148-186 in second-order form (integrate_system).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -44,382 +42,265 @@ namespace eph {
 namespace {
 
 constexpr int kBThreads = 256;          // threads per ensemble CTA
-constexpr int kCluster = 4;             // CTAs of a thread-block cluster that share one large system
-constexpr int kCoopMin = 96;            // default: bodies from which a system is shared by a cluster
+constexpr int kCoopMin = 32;            // default: bodies from which a system may be shared by a cluster
 constexpr double kCB = 299792458.0;     // src/math/basic_math.h:10,18
-constexpr int kAcc = 9;                 // stored values per (body, stage): velocity dd (hi 3, lo 3), acceleration 3
+constexpr int kStore = 3 * kStages + 12;   // stored values per body: f_j of every stage, r0 and v0 (hi, lo)
+constexpr int kMaxSplit = 32;           // most parts a body's j range is cut into
 
-__constant__ double b_rk_hi[EPH_RK12_NCOEF];
-__constant__ double b_rk_lo[EPH_RK12_NCOEF];
-__constant__ double b_dtk[kStages + 1];
+// The Feagin table in second-order form: v_j = v0 + dt sum_l a_jl f_l, so sum_j a_kj v_j = c_k v0 +
+// dt sum_l Abar_kl f_l with Abar = A A. Entry k(k-1)/2 + l: Abar_kl as hi + lo, a_kl rounded. The CTAs read the
+// entries from shared memory: the rows are walked whole (a zero entry adds nothing), so no load depends on another.
+__constant__ double b_ab_hi[EPH_RK12_NCOEF];
+__constant__ double b_ab_lo[EPH_RK12_NCOEF];
+__constant__ double b_a[EPH_RK12_NCOEF];
+__constant__ double b_ck_hi[kStages + 1];   // c_k = sum_j a_kj, hi + lo
+__constant__ double b_ck_lo[kStages + 1];
+__constant__ double b_dtk[kStages + 1];     // c_k as the reference sums it (stage times)
+struct RkTable {
+    double2 ab[EPH_RK12_NCOEF];   // {Abar hi, a}
+    double lo[EPH_RK12_NCOEF];    // Abar lo
+};
 
 struct BatchSys {
     int n;                // bodies
-    int pad;
+    int split;            // parts that a body's j range is cut into (batch_split)
     long long n_step;     // steps (>= 1)
     double dt;            // signed step
     double t_eph;         // double(t_eph) at the start
     double *planes;       // [EPH_NPLANES][n], in and out
-    double *acc;          // [kStages][kAcc][n] stage values f_j: velocity (hi 3, lo 3), acceleration 3
-    double *x0;           // [12][n] start-of-step r, v (hi, lo)
+    double *store;        // [kStore][n] stage accelerations and start-of-step state, when shared memory has no room
 };
 
-// shared-memory rows of one system, stride `ld` bodies
-enum BRow { BR_R_HI = 0, BR_R_LO = 3, BR_GM = 6, BR_SR2 = 7, BR_PHI = 8, BR_NACC = 9, BR_BETA = 12, BR_BETA2 = 15,
-            BR_V_HI = 16, BR_V_LO = 19, BR_FA = 22, BR_GA = 25, BR_MIND = 28, BR_MAXI = 29, BR_GM0 = 30, BR_DGM = 31,
-            BR_F32 = 32, BR_ROWS = 37 };
-// FP32 rows of the mixed-precision form (single-precision copies of what its pass-B pair terms read of body
-// j), packed two to a double row from BR_F32 on
-enum FRow { F_GM = 0, F_PHI = 1, F_NACC = 2, F_BETA = 5, F_BETA2 = 8, F_ROWS = 9 };
-static_assert((F_ROWS + 1) / 2 <= BR_ROWS - BR_F32, "FP32 rows do not fit");
+// What a pair term reads of a body lies in records of 64 bytes, 80 apart, so that a thread fetches a body j with four
+// 16-byte shared-memory loads; the lanes of a warp work on different bodies i and the same j, which makes every
+// one of them a broadcast.
+enum RecA { RA_R_HI = 0, RA_R_LO = 3, RA_GM = 6, RA_SR2 = 7, kRecA = 10 };          // state of the stage
+enum RecB { RB_NACC = 0, RB_BETA = 3, RB_K = 6, RB_PHI = 7, kRecB = 10 };           // pass-A outputs; K = phi + 2 beta^2
+// The mixed-precision form reads single-precision copies instead of RecB.
+enum RecF { RF_NACC = 0, RF_GM = 3, RF_BETA = 4, RF_PHI = 7, RF_BETA2 = 8, kRecF = 12 };
+enum OwnRow { OR_V_HI = 0, OR_V_LO = 3, OR_M = 6, OR_MAXI = 7, OR_GM0 = 8, OR_DGM = 9, kOwnRows = 10 };
+constexpr int kPartA = 4, kPartB = 6;   // values of a unit's sums: {phi, a_N}; {gaccel, m_min, tq, j of tq}
 
-struct BatchView {
-    double *T;    // rows
+// One CTA's share of a system: the bodies [lo, lo + cnt) of n, and its shared memory. Every CTA of a cluster has
+// the same layout for the arrays that its peers write (A, and what pass B reads of all bodies: B, or F in mixed
+// precision).
+struct View {
+    double *A[2];    // [n][kRecA], by stage parity when shared by a cluster (else the same array twice)
+    double *B;       // [kRecB] records, of all bodies (FP64) or of the own bodies (mixed precision), from body b0
+    float *F;        // [n][kRecF] (mixed precision only)
+    double *own;     // [kOwnRows][cnt]
+    double *part;    // [kPartB][split * cnt] sums of the (body, part) units
+    double *store;   // [kStore] rows `ld` apart, own bodies from 0: f_l component c at row 3 l + c, then r0, v0
     int ld;
+    int n, lo, cnt, b0;
+    int split;       // parts of a body's j range
 };
+__device__ __forceinline__ double &own_row(const View &V, int r, int b) { return V.own[r * V.cnt + b]; }
+__device__ __forceinline__ double *rec_b(const View &V, int i) { return V.B + (size_t)(i - V.b0) * kRecB; }
 
-__device__ __forceinline__ double &row(const BatchView &V, int r, int i) { return V.T[r * V.ld + i]; }
-__device__ __forceinline__ float &frow(const BatchView &V, int r, int i) {
-    return reinterpret_cast<float *>(V.T + BR_F32 * V.ld)[r * V.ld + i];
+// Shared memory (doubles) of each CTA when `peers` share a system of n bodies: room for the largest share. The
+// stage store is in it while two CTAs still fit an SM; larger shares keep it in global memory (L2).
+constexpr int kPairSmem = (113 * 1024 - (int)sizeof(RkTable) - 128) / 8;
+__host__ __device__ inline int batch_smem_doubles(int n, int peers, int split, bool mixed, bool *store_in_smem) {
+    const int most = (n + peers - 1) / peers;
+    const int base = n * ((peers > 1 ? 2 : 1) * kRecA + (mixed ? kRecF / 2 : kRecB)) +
+                     most * (split * kPartB + kOwnRows + (mixed ? kRecB : 0));
+    *store_in_smem = base + most * kStore <= kPairSmem;
+    return *store_in_smem ? base + most * kStore : base;
+}
+template <bool MIXED>
+__device__ __forceinline__ View make_view(const BatchSys &Y, double *smem, int lo, int cnt, int peers) {
+    const bool coop = peers > 1;
+    const int n = Y.n;
+    View V;
+    V.n = n; V.lo = lo; V.cnt = cnt; V.split = Y.split;
+    double *p = smem;   // every array a multiple of 16 bytes
+    V.A[0] = p; p += (size_t)n * kRecA;
+    V.A[1] = coop ? p : smem; p += coop ? (size_t)n * kRecA : 0;
+    V.F = reinterpret_cast<float *>(p); p += MIXED ? (size_t)n * (kRecF / 2) : 0;
+    V.b0 = MIXED ? lo : 0;
+    V.B = p; p += (size_t)(MIXED ? cnt : n) * kRecB;
+    V.part = p; p += (size_t)cnt * V.split * kPartB;
+    V.own = p; p += (size_t)cnt * kOwnRows;
+    bool in_smem;
+    batch_smem_doubles(n, peers, Y.split, MIXED, &in_smem);
+    V.store = in_smem ? p : Y.store + lo;
+    V.ld = in_smem ? cnt : n;
+    return V;
 }
 
-// pass A pair (i, j): acc = {phi, a_N}
-__device__ __forceinline__ void pair_point_a(const BatchView &V, int i, int j, double acc[4]) {
-    const v3 r = mk(sep_diff(row(V, BR_R_HI + 0, j), row(V, BR_R_LO + 0, j), row(V, BR_R_HI + 0, i), row(V, BR_R_LO + 0, i)),
-                    sep_diff(row(V, BR_R_HI + 1, j), row(V, BR_R_LO + 1, j), row(V, BR_R_HI + 1, i), row(V, BR_R_LO + 1, i)),
-                    sep_diff(row(V, BR_R_HI + 2, j), row(V, BR_R_LO + 2, j), row(V, BR_R_HI + 2, i), row(V, BR_R_LO + 2, i)));
-    const double q = dot(r, r), sm = row(V, BR_SR2, i) + row(V, BR_SR2, j);
-    const double rr = rsqrt((q < sm) ? sm : q);
-    const double rr2 = rr * rr;
-    const double tp_dphi = rr * row(V, BR_GM, j);
-    const double tp_dg = rr2 * tp_dphi;
-    acc[0] -= tp_dphi;
-    acc[1] += tp_dg * r.x;
-    acc[2] += tp_dg * r.y;
-    acc[3] += tp_dg * r.z;
+struct BodyA {   // a body's stage state
+    double hx, hy, hz, lx, ly, lz, gm, sr2;
+};
+__device__ __forceinline__ BodyA load_a(const double *A, int i) {
+    const double2 *p = reinterpret_cast<const double2 *>(A + (size_t)i * kRecA);
+    const double2 a = p[0], b = p[1], c = p[2], d = p[3];
+    return BodyA{a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
+}
+__device__ __forceinline__ v3 separation(const BodyA &j, const BodyA &i) {
+    return mk(sep_diff(j.hx, j.lx, i.hx, i.lx), sep_diff(j.hy, j.ly, i.hy, i.ly), sep_diff(j.hz, j.lz, i.hz, i.lz));
 }
 
-struct PairMax {
-    double m_min;            // smallest floored r^2
-    double tq, tq_m, tq_gm;  // largest GM_j/r^3 seen, with its r^2 and GM_j
-};
-
-// pass B pair (i, j): acc = gaccel (EIH 1PN) and the maxima bookkeeping
-__device__ __forceinline__ void pair_point_b(const BatchView &V, int i, int j, double acc[3], PairMax &x) {
-    const v3 r = mk(sep_diff(row(V, BR_R_HI + 0, j), row(V, BR_R_LO + 0, j), row(V, BR_R_HI + 0, i), row(V, BR_R_LO + 0, i)),
-                    sep_diff(row(V, BR_R_HI + 1, j), row(V, BR_R_LO + 1, j), row(V, BR_R_HI + 1, i), row(V, BR_R_LO + 1, i)),
-                    sep_diff(row(V, BR_R_HI + 2, j), row(V, BR_R_LO + 2, j), row(V, BR_R_HI + 2, i), row(V, BR_R_LO + 2, i)));
-    const double GMj = row(V, BR_GM, j);
-    const double q = dot(r, r), sm = row(V, BR_SR2, i) + row(V, BR_SR2, j);
-    const double m = (q < sm) ? sm : q;
-    const double rr = rsqrt(m);
-    const double rr2 = rr * rr;
-    const double tp_dphi = rr * GMj;
-    const double tp_dg = rr2 * tp_dphi;
-    if (x.m_min == x.m_min) x.m_min = (m != m || m < x.m_min) ? m : x.m_min;
-    if (x.tq == x.tq) {
-        if (tp_dg != tp_dg) x.tq = tp_dg;
-        else if (tp_dg > x.tq) { x.tq = tp_dg; x.tq_m = m; x.tq_gm = GMj; }
+// pass A over j in [j0, j1): s = {phi, a_N}. The body itself takes part with GM = 0 at unit distance, so the
+// loop has no branch that differs between lanes.
+__device__ __forceinline__ void sweep_point_a(const double *A, int i, int j0, int j1, double s[kPartA]) {
+    const BodyA bi = load_a(A, i);
+    s[0] = s[1] = s[2] = s[3] = 0;
+#pragma unroll 2
+    for (int j = j0; j < j1; ++j) {
+        const BodyA bj = load_a(A, j);
+        const v3 r = separation(bj, bi);
+        const double q = dot(r, r), sm = bi.sr2 + bj.sr2;
+        const double m = (q < sm) ? sm : q;
+        const double rr = inv_sqrt(j == i ? 1.0 : m);
+        const double tp_dphi = rr * (j == i ? 0.0 : bj.gm);
+        const double tp_dg = (rr * rr) * tp_dphi;
+        s[0] -= tp_dphi;
+        s[1] += tp_dg * r.x;
+        s[2] += tp_dg * r.y;
+        s[3] += tp_dg * r.z;
     }
-    const v3 bj = mk(row(V, BR_BETA + 0, j), row(V, BR_BETA + 1, j), row(V, BR_BETA + 2, j));
-    const v3 bi = mk(row(V, BR_BETA + 0, i), row(V, BR_BETA + 1, i), row(V, BR_BETA + 2, i));
-    const double rbj = dot(r, bj);
-    double tp = rbj * rr;
-    tp *= tp;
-    const v3 naj = mk(row(V, BR_NACC + 0, j), row(V, BR_NACC + 1, j), row(V, BR_NACC + 2, j));
-    const double delta1 = 4 * row(V, BR_PHI, i) + row(V, BR_PHI, j) + row(V, BR_BETA2, i) + 2 * row(V, BR_BETA2, j) -
-                          4 * dot(bi, bj) + (dot(r, naj) - 3 * tp) / 2;
-    const v3 b = bj - bi;
-    const v3 g = (7 * tp_dphi / 2) * naj + (tp_dg * delta1) * r + (tp_dg * (rbj - dot(r, b) * 4)) * b;
-    acc[0] += g.x;
-    acc[1] += g.y;
-    acc[2] += g.z;
 }
 
-// Mixed-precision form of the pass-B pair: the separation and its floored square stay FP64 (so the per-pair
+// pass B over j in [j0, j1): s = {EIH 1PN acceleration less the terms common to all j, smallest floored r^2,
+// largest GM_j/r^3 and its j}. mass.impl:82-97 with the sums over j regrouped: the coefficient 4 phi_i + beta_i^2
+// multiplies the Newtonian sum that pass A has formed already (point_b_common adds it), and with b = beta_j -
+// beta_i the last term's coefficient is r.beta_j - 4 r.b = 4 r.beta_i - 3 r.beta_j =: c, its sum over j
+// sum c beta_j - beta_i sum c: 57 FP64 operations and a reciprocal square root per pair, not 77.
+__device__ __forceinline__ void sweep_point_b(const double *A, const double *B, int i, int j0, int j1, double s[kPartB]) {
+    const BodyA bi = load_a(A, i);
+    const double2 *pi = reinterpret_cast<const double2 *>(B + (size_t)i * kRecB);
+    const double bix = pi[1].y, biy = pi[2].x, biz = pi[2].y;
+    double gx = 0, gy = 0, gz = 0, cs = 0;
+    double m_min = __longlong_as_double(0x7ff0000000000000ll), tq = 0;
+    int tj = -1;
+#pragma unroll 2
+    for (int j = j0; j < j1; ++j) {
+        const BodyA bj = load_a(A, j);
+        const double2 *pj = reinterpret_cast<const double2 *>(B + (size_t)j * kRecB);
+        const double2 p0 = pj[0], p1 = pj[1], p2 = pj[2];
+        const double K = pj[3].x;
+        const double nx = p0.x, ny = p0.y, nz = p1.x, bx = p1.y, by = p2.x, bz = p2.y;
+        const v3 r = separation(bj, bi);
+        const double q = dot(r, r), sm = bi.sr2 + bj.sr2;
+        const double m = (q < sm) ? sm : q;
+        const double rr = inv_sqrt(j == i ? 1.0 : m);
+        const double tp_dphi = rr * (j == i ? 0.0 : bj.gm);
+        const double tp_dg = (rr * rr) * tp_dphi;
+        if (m < m_min && j != i) m_min = m;
+        if (tp_dg > tq) { tq = tp_dg; tj = j; }
+        const double rbj = r.x * bx + r.y * by + r.z * bz;
+        const double rbi = r.x * bix + r.y * biy + r.z * biz;
+        const double rn = r.x * nx + r.y * ny + r.z * nz;
+        const double bb = bix * bx + biy * by + biz * bz;
+        double tp = rbj * rr;
+        tp *= tp;
+        const double w = tp_dg * (((K - 4 * bb) + 0.5 * rn) - 1.5 * tp);
+        const double c = tp_dg * (4 * rbi - 3 * rbj);
+        const double h = 3.5 * tp_dphi;
+        cs += c;
+        gx += h * nx + w * r.x + c * bx;
+        gy += h * ny + w * r.y + c * by;
+        gz += h * nz + w * r.z + c * bz;
+    }
+    s[0] = gx - cs * bix;
+    s[1] = gy - cs * biy;
+    s[2] = gz - cs * biz;
+    s[3] = m_min;
+    s[4] = tq;
+    s[5] = __longlong_as_double(tj);
+}
+
+// Mixed-precision form of the pass-B sweep: the separation and its floored square stay FP64 (so the per-pair
 // maxima keep the reference's exact recomputation of the extremal pair), the EIH 1PN acceleration (about
 // 1e-8 of the Newtonian one for solar-system speeds and potentials, so FP32's 6e-8 relative rounding is
 // ~1e-15 of the total) is formed in FP32 from FP32 copies of the pass-A outputs and summed with a
-// compensated FP32 sum (Fast2Sum after each add), which the caller converts into its FP64 totals. The
+// compensated FP32 sum (Fast2Sum after each add), which is converted into the FP64 totals. The
 // extremal pair of max_influence is chosen on the FP32 value of GM/r^3, so in a near-tie (within FP32
 // rounding) another pair's value may be the one recomputed.
-struct BodyF32 {   // body i's FP32 pass-B inputs
-    float phi, beta2, bx, by, bz;
+struct Comp32 {    // a compensated FP32 sum
+    float s, c;
 };
-struct Comp32 {    // compensated FP32 sums of the three 1PN components
-    float s[3], c[3];
-};
-struct PairMax32 {
-    double m_min;          // smallest floored r^2 (FP64)
-    float tq;              // largest FP32 GM_j/r^3 seen
-    double tq_m, tq_gm;    // its r^2 and GM_j
-};
-__device__ __forceinline__ void comp_add(float &s, float &c, float x) {
-    const float t = __fadd_rn(s, x);
-    const float big = fabsf(s) >= fabsf(x) ? s : x, small = fabsf(s) >= fabsf(x) ? x : s;
-    c = __fadd_rn(c, __fadd_rn(__fsub_rn(big, t), small));
-    s = t;
+__device__ __forceinline__ void comp_add(Comp32 &a, float x) {
+    const float t = __fadd_rn(a.s, x);
+    const bool keep = fabsf(a.s) >= fabsf(x);
+    const float big = keep ? a.s : x, small = keep ? x : a.s;
+    a.c = __fadd_rn(a.c, __fadd_rn(__fsub_rn(big, t), small));
+    a.s = t;
 }
-__device__ __forceinline__ void pair_point_b32(const BatchView &V, int i, int j, const BodyF32 &bi, Comp32 &acc,
-                                               PairMax32 &x) {
-    const v3 r = mk(sep_diff(row(V, BR_R_HI + 0, j), row(V, BR_R_LO + 0, j), row(V, BR_R_HI + 0, i), row(V, BR_R_LO + 0, i)),
-                    sep_diff(row(V, BR_R_HI + 1, j), row(V, BR_R_LO + 1, j), row(V, BR_R_HI + 1, i), row(V, BR_R_LO + 1, i)),
-                    sep_diff(row(V, BR_R_HI + 2, j), row(V, BR_R_LO + 2, j), row(V, BR_R_HI + 2, i), row(V, BR_R_LO + 2, i)));
-    const double q = dot(r, r), sm = row(V, BR_SR2, i) + row(V, BR_SR2, j);
-    const double m = (q < sm) ? sm : q;
-    if (x.m_min == x.m_min) x.m_min = (m != m || m < x.m_min) ? m : x.m_min;
-    const float rr = rsqrtf((float)m);
-    const float rr2 = rr * rr;
-    const float tp_dphi = rr * frow(V, F_GM, j);
-    const float tp_dg = rr2 * tp_dphi;
-    if (x.tq == x.tq) {
-        if (tp_dg != tp_dg) x.tq = tp_dg;
-        else if (tp_dg > x.tq) { x.tq = tp_dg; x.tq_m = m; x.tq_gm = row(V, BR_GM, j); }
+__device__ __forceinline__ void sweep_point_b32(const double *A, const float *F, int i, int j0, int j1,
+                                                double s[kPartB]) {
+    const BodyA bi = load_a(A, i);
+    const float4 *fi = reinterpret_cast<const float4 *>(F + (size_t)i * kRecF);
+    const float bix = fi[1].x, biy = fi[1].y, biz = fi[1].z;
+    const float phi_i = fi[1].w, beta2_i = fi[2].x;
+    Comp32 gx{0, 0}, gy{0, 0}, gz{0, 0};
+    double m_min = __longlong_as_double(0x7ff0000000000000ll);
+    float tq = 0;
+    int tj = -1;
+#pragma unroll 2
+    for (int j = j0; j < j1; ++j) {
+        const BodyA bj = load_a(A, j);
+        const float4 *fj = reinterpret_cast<const float4 *>(F + (size_t)j * kRecF);
+        const float4 a = fj[0], b = fj[1];   // {a_N, GM}, {beta, phi}
+        const v3 r = separation(bj, bi);
+        const double q = dot(r, r), sm = bi.sr2 + bj.sr2;
+        const double m = (q < sm) ? sm : q;
+        if (m < m_min && j != i) m_min = m;
+        const float rr = rsqrtf(j == i ? 1.0f : (float)m);
+        const float tp_dphi = rr * (j == i ? 0.0f : a.w);
+        const float tp_dg = (rr * rr) * tp_dphi;
+        if (tp_dg > tq) { tq = tp_dg; tj = j; }
+        const float rx = (float)r.x, ry = (float)r.y, rz = (float)r.z;
+        const float rbj = rx * b.x + ry * b.y + rz * b.z;
+        float tp = rbj * rr;
+        tp *= tp;
+        const float delta1 = 4 * phi_i + b.w + beta2_i + 2 * fj[2].x - 4 * (bix * b.x + biy * b.y + biz * b.z) +
+                             ((rx * a.x + ry * a.y + rz * a.z) - 3 * tp) / 2;
+        const float bx = b.x - bix, by = b.y - biy, bz = b.z - biz;
+        const float c1 = 7 * tp_dphi / 2, c2 = tp_dg * delta1, c3 = tp_dg * (rbj - (rx * bx + ry * by + rz * bz) * 4);
+        comp_add(gx, c1 * a.x + c2 * rx + c3 * bx);
+        comp_add(gy, c1 * a.y + c2 * ry + c3 * by);
+        comp_add(gz, c1 * a.z + c2 * rz + c3 * bz);
     }
-    const float rx = (float)r.x, ry = (float)r.y, rz = (float)r.z;
-    const float bjx = frow(V, F_BETA + 0, j), bjy = frow(V, F_BETA + 1, j), bjz = frow(V, F_BETA + 2, j);
-    const float rbj = rx * bjx + ry * bjy + rz * bjz;
-    float tp = rbj * rr;
-    tp *= tp;
-    const float nax = frow(V, F_NACC + 0, j), nay = frow(V, F_NACC + 1, j), naz = frow(V, F_NACC + 2, j);
-    const float delta1 = 4 * bi.phi + frow(V, F_PHI, j) + bi.beta2 + 2 * frow(V, F_BETA2, j) -
-                         4 * (bi.bx * bjx + bi.by * bjy + bi.bz * bjz) + ((rx * nax + ry * nay + rz * naz) - 3 * tp) / 2;
-    const float bx = bjx - bi.bx, by = bjy - bi.by, bz = bjz - bi.bz;
-    const float c1 = 7 * tp_dphi / 2, c2 = tp_dg * delta1, c3 = tp_dg * (rbj - (rx * bx + ry * by + rz * bz) * 4);
-    comp_add(acc.s[0], acc.c[0], c1 * nax + c2 * rx + c3 * bx);
-    comp_add(acc.s[1], acc.c[1], c1 * nay + c2 * ry + c3 * by);
-    comp_add(acc.s[2], acc.c[2], c1 * naz + c2 * rz + c3 * bz);
-}
-__device__ __forceinline__ BodyF32 body_f32(const BatchView &V, int i) {
-    return BodyF32{frow(V, F_PHI, i), frow(V, F_BETA2, i), frow(V, F_BETA + 0, i), frow(V, F_BETA + 1, i),
-                   frow(V, F_BETA + 2, i)};
+    s[0] = (double)gx.s + (double)gx.c;
+    s[1] = (double)gy.s + (double)gy.c;
+    s[2] = (double)gz.s + (double)gz.c;
+    s[3] = m_min;
+    s[4] = (double)tq;
+    s[5] = __longlong_as_double(tj);
 }
 
-// Threads of a pass: with n <= blockDim bodies, G consecutive lanes of a warp share body i and split its j
-// range (G = the largest power of two <= min(32, blockDim / n)); their partial sums are combined by warp
-// shuffles. With more bodies than threads each thread takes whole bodies.
-struct PassMap {
-    int G, i, sub;
-    bool grouped, active;
-};
-__device__ __forceinline__ PassMap pass_map(int lo, int hi) {
-    const int cnt = hi - lo;
-    PassMap m;
-    m.grouped = cnt <= (int)blockDim.x;
-    int g = 1;
-    if (m.grouped)
-        while (g < 32 && 2 * g * cnt <= (int)blockDim.x) g *= 2;
-    m.G = g;
-    m.i = lo + (int)threadIdx.x / g;
-    m.sub = threadIdx.x % g;
-    m.active = m.grouped && m.i < hi;
-    return m;
-}
-// sum (or NaN-propagating maximum) over the G lanes of a group; every lane of the warp takes part
-__device__ __forceinline__ double group_sum(double v, int G) {
-    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-__device__ __forceinline__ double group_max(double v, int G) {
-    for (int o = G / 2; o > 0; o >>= 1) {
-        const double u = __shfl_xor_sync(0xffffffffu, v, o);
-        checked_maximize(v, u);
-    }
-    return v;
-}
-
-// pass A for body i over j ≡ sub (mod G), then PREPARE_RELATIVITY by whoever holds the total
-__device__ __forceinline__ void prepare_body(const BatchView &V, int i, const double s[4]) {
-    const double c2 = kCB * kCB;
-    const v3 beta = vdiv(mk(dd_val(dd{row(V, BR_V_HI + 0, i), row(V, BR_V_LO + 0, i)}),
-                            dd_val(dd{row(V, BR_V_HI + 1, i), row(V, BR_V_LO + 1, i)}),
-                            dd_val(dd{row(V, BR_V_HI + 2, i), row(V, BR_V_LO + 2, i)})), kCB);
-    row(V, BR_BETA + 0, i) = beta.x;
-    row(V, BR_BETA + 1, i) = beta.y;
-    row(V, BR_BETA + 2, i) = beta.z;
-    row(V, BR_BETA2, i) = dot(beta, beta);
-    row(V, BR_PHI, i) = s[0] / c2;
-    const v3 na = vdiv(mk(s[1], s[2], s[3]), c2);
-    row(V, BR_NACC + 0, i) = na.x;
-    row(V, BR_NACC + 1, i) = na.y;
-    row(V, BR_NACC + 2, i) = na.z;
-    // FP32 copies for the mixed-precision pass B (written in both forms; unused by the FP64 one)
-    frow(V, F_PHI, i) = (float)row(V, BR_PHI, i);
-    frow(V, F_BETA2, i) = (float)row(V, BR_BETA2, i);
-    for (int c = 0; c < 3; ++c) {
-        frow(V, F_NACC + c, i) = (float)row(V, BR_NACC + c, i);
-        frow(V, F_BETA + c, i) = (float)row(V, BR_BETA + c, i);
+// Running extremes of a body over all stages (RungeKutta.cu:229-230: the largest 1/r and GM_j/r^3 over the floored
+// separations), with the reference's expressions rr2 = 1/m, rr = sqrt(rr2) (mass.impl:84-89). The smallest m = r^2
+// is kept as it is (sqrt(1/m) does not decrease as m falls, so it is formed once, at the end). The stage's pair of
+// the largest GM_j/r^3 is recomputed exactly only when its swept value, good to `slack`, may exceed the largest so far.
+__device__ __forceinline__ void extremes_add(const View &V, const double *A, int b, double m_min, double tq, int tj,
+                                             double slack) {
+    if (m_min < own_row(V, OR_M, b)) own_row(V, OR_M, b) = m_min;
+    const double top = own_row(V, OR_MAXI, b);
+    if (tj >= 0 && tq >= top * (1 - slack)) {   // (false once the maximum is a NaN)
+        const BodyA bi = load_a(A, V.lo + b), bj = load_a(A, tj);
+        const v3 r = separation(bj, bi);
+        const double q = dot(r, r), sm = bi.sr2 + bj.sr2;
+        const double rr2 = 1.0 / ((q < sm) ? sm : q), t = rr2 * (sqrt(rr2) * bj.gm);
+        if (t > top) own_row(V, OR_MAXI, b) = t;
     }
 }
-
-// pass A (and PREPARE_RELATIVITY) of the bodies i in [lo, hi) against all n bodies
-__device__ void pass_point_a(const BatchView &V, int n, int lo, int hi) {
-    const PassMap m = pass_map(lo, hi);
-    if (m.grouped) {
-        // two independent pair chains per thread (j and j + G), added at the end
-        double acc[4] = {0, 0, 0, 0}, acc2[4] = {0, 0, 0, 0};
-        if (m.active) {
-            int j = m.sub;
-#pragma unroll 1
-            for (; j + m.G < n; j += 2 * m.G) {
-                if (j != m.i) pair_point_a(V, m.i, j, acc);
-                if (j + m.G != m.i) pair_point_a(V, m.i, j + m.G, acc2);
-            }
-            if (j < n && j != m.i) pair_point_a(V, m.i, j, acc);
-        }
-        double s[4];
-        for (int c = 0; c < 4; ++c) s[c] = group_sum(acc[c] + acc2[c], m.G);
-        if (m.active && m.sub == 0) prepare_body(V, m.i, s);
-    } else {
-        // whole bodies per thread: prepare_body writes only rows pass A does not read (it reads r, GM, sR2)
-#pragma unroll 1
-        for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-            double s[4] = {0, 0, 0, 0}, s2[4] = {0, 0, 0, 0};
-            int j = 0;
-#pragma unroll 1
-            for (; j + 1 < n; j += 2) {
-                if (j != i) pair_point_a(V, i, j, s);
-                if (j + 1 != i) pair_point_a(V, i, j + 1, s2);
-            }
-            if (j < n && j != i) pair_point_a(V, i, j, s);
-            for (int c = 0; c < 4; ++c) s[c] += s2[c];
-            prepare_body(V, i, s);
-        }
+// The same when one of the body's sums is not a number: the sweeps' comparisons drop a NaN, the reference's
+// maxima keep it (checked_maximize), so the pairs are walked again one by one.
+__device__ __noinline__ void extremes_nan(const View &V, const double *A, int b) {
+    const int i = V.lo + b;
+    const BodyA bi = load_a(A, i);
+    for (int j = 0; j < V.n; ++j) {
+        if (j == i) continue;
+        const BodyA bj = load_a(A, j);
+        const v3 r = separation(bj, bi);
+        const double q = dot(r, r), sm = bi.sr2 + bj.sr2;
+        const double m = (q < sm) ? sm : q, rr2 = 1.0 / m;
+        if (m != m || m < own_row(V, OR_M, b)) own_row(V, OR_M, b) = m;
+        checked_maximize(own_row(V, OR_MAXI, b), rr2 * (sqrt(rr2) * bj.gm));
     }
-    __syncthreads();
-}
-
-// finalisation of body i from its pass-B totals {gaccel, 1/r max, GM/r^3 max}
-__device__ __forceinline__ void finish_body(const BatchView &V, int i, const double s[5]) {
-    const double c2 = kCB * kCB;
-    checked_maximize(row(V, BR_MIND, i), s[3]);
-    checked_maximize(row(V, BR_MAXI, i), s[4]);
-    const v3 ga = mk(s[0], s[1], s[2]);
-    const v3 da = mk(0, 0, 0);
-    const v3 na = c2 * mk(row(V, BR_NACC + 0, i), row(V, BR_NACC + 1, i), row(V, BR_NACC + 2, i));
-    const v3 fa = (ga + da) + na;
-    row(V, BR_GA + 0, i) = ga.x;
-    row(V, BR_GA + 1, i) = ga.y;
-    row(V, BR_GA + 2, i) = ga.z;
-    row(V, BR_FA + 0, i) = fa.x;
-    row(V, BR_FA + 1, i) = fa.y;
-    row(V, BR_FA + 2, i) = fa.z;
-}
-
-// exact extremes with the reference's expressions (rr2 = 1/m, rr = sqrt(rr2), mass.impl:84-89)
-__device__ __forceinline__ void extremes_of(const PairMax &x, double &inv_r, double &infl) {
-    inv_r = sqrt(1.0 / x.m_min);   // +inf -> 0 when no pair was seen
-    if (x.tq != x.tq) infl = x.tq;
-    else if (x.tq > 0) {
-        const double r2 = 1.0 / x.tq_m;
-        infl = r2 * (sqrt(r2) * x.tq_gm);
-    } else infl = 0.0;
-}
-
-// exact extremes of the mixed form's tracking (the same expressions on the tracked FP64 values)
-__device__ __forceinline__ void extremes_of32(const PairMax32 &x, double &inv_r, double &infl) {
-    inv_r = sqrt(1.0 / x.m_min);
-    if (x.tq != x.tq) infl = (double)x.tq;
-    else if (x.tq > 0) {
-        const double r2 = 1.0 / x.tq_m;
-        infl = r2 * (sqrt(r2) * x.tq_gm);
-    } else infl = 0.0;
-}
-
-// mixed-precision pass B: two pair chains per thread like the FP64 form, FP32 1PN sums converted into FP64
-__device__ void pass_point_b32(const BatchView &V, int n, int lo, int hi) {
-    const PassMap m = pass_map(lo, hi);
-    const double inf = __longlong_as_double(0x7ff0000000000000ll);
-    auto sweep = [&](int i, int j0, int step, double s[5]) {
-        const BodyF32 bi = body_f32(V, i);
-        Comp32 a{{0, 0, 0}, {0, 0, 0}}, a2{{0, 0, 0}, {0, 0, 0}};
-        PairMax32 x{inf, 0.0f, 0.0, 0.0}, x2{inf, 0.0f, 0.0, 0.0};
-        int j = j0;
-#pragma unroll 1
-        for (; j + step < n; j += 2 * step) {
-            if (j != i) pair_point_b32(V, i, j, bi, a, x);
-            if (j + step != i) pair_point_b32(V, i, j + step, bi, a2, x2);
-        }
-        if (j < n && j != i) pair_point_b32(V, i, j, bi, a, x);
-        for (int c = 0; c < 3; ++c)
-            s[c] = ((double)a.s[c] + (double)a.c[c]) + ((double)a2.s[c] + (double)a2.c[c]);
-        double f0, f1;
-        extremes_of32(x, s[3], s[4]);
-        extremes_of32(x2, f0, f1);
-        checked_maximize(s[3], f0);
-        checked_maximize(s[4], f1);
-    };
-    if (m.grouped) {
-        double s[5] = {0, 0, 0, 0, 0};
-        if (m.active) sweep(m.i, m.sub, m.G, s);
-        else {
-            const PairMax32 none{inf, 0.0f, 0.0, 0.0};
-            extremes_of32(none, s[3], s[4]);
-        }
-        for (int c = 0; c < 3; ++c) s[c] = group_sum(s[c], m.G);
-        s[3] = group_max(s[3], m.G);
-        s[4] = group_max(s[4], m.G);
-        if (m.active && m.sub == 0) finish_body(V, m.i, s);
-    } else {
-#pragma unroll 1
-        for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-            double s[5];
-            sweep(i, 0, 1, s);
-            finish_body(V, i, s);
-        }
-    }
-    __syncthreads();
-}
-
-// pass B and finalisation of the bodies i in [lo, hi) against all n bodies
-__device__ void pass_point_b(const BatchView &V, int n, int lo, int hi) {
-    const PassMap m = pass_map(lo, hi);
-    const double inf = __longlong_as_double(0x7ff0000000000000ll);
-    if (m.grouped) {
-        double acc[3] = {0, 0, 0}, acc2[3] = {0, 0, 0};
-        PairMax x{inf, 0.0, 0.0, 0.0}, x2{inf, 0.0, 0.0, 0.0};
-        if (m.active) {
-            int j = m.sub;
-#pragma unroll 1
-            for (; j + m.G < n; j += 2 * m.G) {
-                if (j != m.i) pair_point_b(V, m.i, j, acc, x);
-                if (j + m.G != m.i) pair_point_b(V, m.i, j + m.G, acc2, x2);
-            }
-            if (j < n && j != m.i) pair_point_b(V, m.i, j, acc, x);
-        }
-        double e0, e1, f0, f1;
-        extremes_of(x, e0, e1);
-        extremes_of(x2, f0, f1);
-        checked_maximize(e0, f0);
-        checked_maximize(e1, f1);
-        double s[5];
-        for (int c = 0; c < 3; ++c) s[c] = group_sum(acc[c] + acc2[c], m.G);
-        s[3] = group_max(e0, m.G);
-        s[4] = group_max(e1, m.G);
-        if (m.active && m.sub == 0) finish_body(V, m.i, s);
-    } else {
-        // finish_body writes only rows pass B does not read (GA, FA, MIND, MAXI)
-#pragma unroll 1
-        for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-            double acc[3] = {0, 0, 0}, acc2[3] = {0, 0, 0};
-            PairMax x{inf, 0.0, 0.0, 0.0}, x2{inf, 0.0, 0.0, 0.0};
-            int j = 0;
-#pragma unroll 1
-            for (; j + 1 < n; j += 2) {
-                if (j != i) pair_point_b(V, i, j, acc, x);
-                if (j + 1 != i) pair_point_b(V, i, j + 1, acc2, x2);
-            }
-            if (j < n && j != i) pair_point_b(V, i, j, acc, x);
-            double s[5] = {acc[0] + acc2[0], acc[1] + acc2[1], acc[2] + acc2[2], 0, 0};
-            double f0, f1;
-            extremes_of(x, s[3], s[4]);
-            extremes_of(x2, f0, f1);
-            checked_maximize(s[3], f0);
-            checked_maximize(s[4], f1);
-            finish_body(V, i, s);
-        }
-    }
-    __syncthreads();
 }
 
 // mass::orthogonalize (mass.h:147-150) of body i's frame, in place in the planes
@@ -447,224 +328,381 @@ __device__ void orthogonalize_frame(double *pl, int n, int i) {
 
 namespace cg = cooperative_groups;
 
-// Copy rows [row0, row0 + nrows) of the bodies [lo, hi) into the shared memory of every other CTA of the
-// cluster (distributed shared memory); the cluster barrier that follows publishes them.
-__device__ void broadcast_rows(const BatchView &V, int row0, int nrows, int lo, int hi, int rank) {
-    cg::cluster_group cl = cg::this_cluster();
-    const int cnt = hi - lo;
-    for (int q = 0; q < kCluster; ++q) {
-        if (q == rank) continue;
-        double *peer = cl.map_shared_rank(V.T, q);
-        for (int idx = threadIdx.x; idx < nrows * cnt; idx += blockDim.x) {
-            const int r = row0 + idx / cnt, i = lo + idx % cnt;
-            peer[r * V.ld + i] = V.T[r * V.ld + i];
-        }
+// Copies `count` 16-byte words at p (16-byte aligned, the same place in every CTA's shared memory) to the other CTAs of
+// the cluster (distributed shared memory), consecutive threads consecutive words; the cluster barrier that follows
+// publishes them. Stored by the threads that formed them, 8 bytes at a time and 64 apart, the records of 38 bodies
+// took 1800 cycles to seven peers.
+__device__ __forceinline__ void send_all(double *p, int count, int peers, int rank) {
+    const double2 *from = reinterpret_cast<const double2 *>(p);
+#pragma unroll 1
+    for (int q = threadIdx.x; q < count * (peers - 1); q += blockDim.x) {
+        const int hop = q / count, w = q - hop * count;
+        const int to = rank + 1 + hop < peers ? rank + 1 + hop : rank + 1 + hop - peers;
+        reinterpret_cast<double2 *>(cg::this_cluster().map_shared_rank(p, to))[w] = from[w];
     }
 }
 
-// The same for FP32 rows [row0, row0 + nrows).
-__device__ void broadcast_frows(const BatchView &V, int row0, int nrows, int lo, int hi, int rank) {
-    cg::cluster_group cl = cg::this_cluster();
-    const int cnt = hi - lo;
-    float *mine = reinterpret_cast<float *>(V.T + BR_F32 * V.ld);
-    for (int q = 0; q < kCluster; ++q) {
-        if (q == rank) continue;
-        float *peer = reinterpret_cast<float *>(cl.map_shared_rank(V.T, q) + BR_F32 * V.ld);
-        for (int idx = threadIdx.x; idx < nrows * cnt; idx += blockDim.x) {
-            const int r = row0 + idx / cnt, i = lo + idx % cnt;
-            peer[r * V.ld + i] = mine[r * V.ld + i];
-        }
-    }
-}
-
-// One system on one CTA (coop = false) or on the kCluster CTAs of a cluster (coop = true), this CTA
-// owning bodies [lo, hi): every CTA holds all bodies' rows, computes its own bodies' stages and passes,
-// and sends the rows the other CTAs read (positions and GM after the state update, the pass-A outputs
-// after pass A) to their shared memory.
+// One system on one CTA (peers = 1) or on the CTAs of a cluster, this CTA (number `rank`) owning bodies
+// [lo, lo + cnt): every CTA holds the records of all bodies, computes its own bodies' stages and passes, and
+// stores what the other CTAs read (state after the state update, pass-A outputs after pass A) to all of them.
+//
+// What bounds it: latency, of the dependent FP64 chains in the sweeps at 8 to 16 warps an SM (FP64 pipe 51 % and
+// issue 52 % busy with two CTAs of 95 bodies on each SM) and of the stage's four dependent phases for small
+// systems. Hence one thread per (body, component) in the state update, whose sum is one addition deep per term, one
+// thread per (body, part of its j range) in the sweeps, records that a warp reads without bank conflicts, and as
+// many CTAs per system as the batch needs to finish together. Stage times on one B200, one system alone, before
+// (one thread per body, power-of-two lane groups, at most 4 CTAs) and now: 8 bodies 6.5 / 2.9 us, 33 9.3 / 4.6,
+// 95 28.7 / 7.8, 128 16.6 / 7.5, 300 80.3 / 13.3 us.
 template <bool MIXED>
-__device__ void integrate_system(const BatchSys &Y, const BatchView &V, bool coop, int rank) {
+__device__ void integrate_system(const BatchSys &Y, const RkTable &rk, double *smem, int peers, int rank) {
     const int n = Y.n;
-    const int lo = coop ? (int)((long long)rank * n / kCluster) : 0;
-    const int hi = coop ? (int)((long long)(rank + 1) * n / kCluster) : n;
+    const int lo = (int)((long long)rank * n / peers);
+    const int cnt = (int)((long long)(rank + 1) * n / peers) - lo;
+    const View V = make_view<MIXED>(Y, smem, lo, cnt, peers);
     double *pl = Y.planes;
+    const double c2 = kCB * kCB;
 #define PLV(p, i) pl[(size_t)(p) * n + (i)]
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        for (int c = 0; c < 3; ++c) {
-            row(V, BR_R_HI + c, i) = PLV(EPH_P_R_HI + c, i);
-            row(V, BR_R_LO + c, i) = PLV(EPH_P_R_LO + c, i);
-            row(V, BR_V_HI + c, i) = PLV(EPH_P_V_HI + c, i);
-            row(V, BR_V_LO + c, i) = PLV(EPH_P_V_LO + c, i);
-            row(V, BR_NACC + c, i) = PLV(EPH_P_NACCEL + c, i);
-            row(V, BR_GA + c, i) = PLV(EPH_P_GACCEL + c, i);
+    auto sync = [&]() {
+        if (peers > 1) cg::this_cluster().sync();
+        else __syncthreads();
+    };
+    // One pass over the units (body b, part `sub` of its j range), unit u = sub * cnt + b on thread u mod 256:
+    // sweep(i, j0, j1, slot of the unit's sums) by the unit's thread, then take(b, value, the body's first slot) by
+    // one thread per (body, value). A body's parts are summed in ascending j, so how many CTAs share a system changes
+    // no result. The takes are not followed by a barrier.
+    const int units = cnt * V.split;
+    auto for_units = [&](auto &&sweep, auto &&take) {
+#pragma unroll 1
+        for (int u = threadIdx.x; u < units; u += kBThreads) {
+            const int sub = u / cnt, b = u - sub * cnt;
+            sweep(lo + b, sub * n / V.split, (sub + 1) * n / V.split, V.part + u);
         }
-        row(V, BR_GM, i) = PLV(EPH_P_GM, i);
-        frow(V, F_GM, i) = (float)PLV(EPH_P_GM, i);
-        row(V, BR_SR2, i) = PLV(EPH_P_SR2, i);
-        row(V, BR_GM0, i) = PLV(EPH_P_GM0, i);
-        row(V, BR_DGM, i) = PLV(EPH_P_DGM, i);
-        row(V, BR_PHI, i) = PLV(EPH_P_PHI, i);
+        __syncthreads();
+#pragma unroll 1
+        for (int idx = threadIdx.x; idx < 4 * cnt; idx += kBThreads) {
+            const int c = idx / cnt, b = idx - c * cnt;
+            take(b, c, V.part + b);
+        }
+    };
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        for (int h = 0; h < (peers > 1 ? 2 : 1); ++h) {
+            double *a = V.A[h] + (size_t)i * kRecA;
+            for (int c = 0; c < 3; ++c) {
+                a[RA_R_HI + c] = PLV(EPH_P_R_HI + c, i);
+                a[RA_R_LO + c] = PLV(EPH_P_R_LO + c, i);
+            }
+            a[RA_GM] = PLV(EPH_P_GM, i);
+            a[RA_SR2] = PLV(EPH_P_SR2, i);
+        }
+    }
+    for (int b = threadIdx.x; b < cnt; b += blockDim.x) {
+        const int i = lo + b;
+        for (int c = 0; c < 3; ++c) {
+            own_row(V, OR_V_HI + c, b) = PLV(EPH_P_V_HI + c, i);
+            own_row(V, OR_V_LO + c, b) = PLV(EPH_P_V_LO + c, i);
+        }
+        own_row(V, OR_GM0, b) = PLV(EPH_P_GM0, i);
+        own_row(V, OR_DGM, b) = PLV(EPH_P_DGM, i);
+        own_row(V, OR_M, b) = __longlong_as_double(0x7ff0000000000000ll);   // msystem::integrate resets the
+        own_row(V, OR_MAXI, b) = 0.0;                                         // maxima (mass.cpp:406)
         // the loaded auxiliaries are f_0 of the first step (RungeKutta.impl:110-116)
         const v3 fa = (mk(PLV(EPH_P_GACCEL, i), PLV(EPH_P_GACCEL + 1, i), PLV(EPH_P_GACCEL + 2, i)) +
                        mk(PLV(EPH_P_DACCEL, i), PLV(EPH_P_DACCEL + 1, i), PLV(EPH_P_DACCEL + 2, i))) +
                       mk(PLV(EPH_P_NACCEL, i), PLV(EPH_P_NACCEL + 1, i), PLV(EPH_P_NACCEL + 2, i));
-        row(V, BR_FA + 0, i) = fa.x;
-        row(V, BR_FA + 1, i) = fa.y;
-        row(V, BR_FA + 2, i) = fa.z;
-        row(V, BR_MIND, i) = 0.0;   // msystem::integrate resets the maxima (mass.cpp:406)
-        row(V, BR_MAXI, i) = 0.0;
+        V.store[b] = fa.x;
+        V.store[V.ld + b] = fa.y;
+        V.store[2 * V.ld + b] = fa.z;
     }
-    __syncthreads();
+    sync();   // the peers' copies are loaded too before the first store to them
     const double dt = Y.dt;
+    int buf = 0;   // parity of the state records in use
 #pragma unroll 1
     for (long long step = 0; step < Y.n_step; ++step) {
 #pragma unroll 1
         for (int s = 0; s < kStages; ++s) {
-            // f_s of every body into the stage store; at s == 0 also x0 = x (RungeKutta.impl:113-121).
-            // Each thread keeps the same bodies throughout, so what it stores it reads back itself.
             const int k = s + 1;
             const double t = Y.t_eph + dt * (b_dtk[k] + (double)step);
-            const int ci0 = k * (k - 1) / 2;
+            const bool last = k == kStages && step + 1 == Y.n_step;
+            double *A = V.A[buf ^ 1];
+            // At s == 0 x0 = x (RungeKutta.impl:113-121). Then the state of stage k (RungeKutta.impl:148-186):
+            // r = r0 + dt (c_k v0 + dt sum_l Abar_kl f_l), the sums in double-double, v = v0 + dt sum_l a_kl f_l.
 #pragma unroll 1
-            for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-                double *F = Y.acc + (size_t)s * kAcc * n + i;   // [stage][component][body]
-                for (int c = 0; c < 3; ++c) {
-                    F[(size_t)c * n] = row(V, BR_V_HI + c, i);
-                    F[(size_t)(3 + c) * n] = row(V, BR_V_LO + c, i);
-                    F[(size_t)(6 + c) * n] = row(V, BR_FA + c, i);
+            for (int idx = threadIdx.x; idx < 3 * cnt; idx += blockDim.x) {
+                const int b = idx / 3, c = idx - 3 * b, i = lo + b, ld = V.ld;
+                double *x0 = V.store + (size_t)(3 * kStages + c) * ld + b;
+                dd r0, v0;
+                if (s == 0) {
+                    const double *a = V.A[buf] + (size_t)i * kRecA;
+                    r0 = dd{a[RA_R_HI + c], a[RA_R_LO + c]};
+                    v0 = dd{own_row(V, OR_V_HI + c, b), own_row(V, OR_V_LO + c, b)};
+                    x0[0] = r0.hi;
+                    x0[3 * ld] = r0.lo;
+                    x0[6 * ld] = v0.hi;
+                    x0[9 * ld] = v0.lo;
+                } else {
+                    r0 = dd{x0[0], x0[3 * ld]};
+                    v0 = dd{x0[6 * ld], x0[9 * ld]};
                 }
-                if (s == 0)
-                    for (int c = 0; c < 3; ++c) {
-                        Y.x0[(0 + c) * n + i] = row(V, BR_R_HI + c, i);
-                        Y.x0[(3 + c) * n + i] = row(V, BR_R_LO + c, i);
-                        Y.x0[(6 + c) * n + i] = row(V, BR_V_HI + c, i);
-                        Y.x0[(9 + c) * n + i] = row(V, BR_V_LO + c, i);
-                    }
-                // state of stage k: sum_j a_kj f_j in ascending j, zero coefficients skipped
-                // (RungeKutta.impl:148-162), then r = r0 + dt v, v = v0 + dt a (RungeKutta.impl:164-186)
-                dd sv[3] = {dd_make(0), dd_make(0), dd_make(0)};
-                double sa[3] = {0.0, 0.0, 0.0};
+                // r0 + dt c_k v0 does not wait for the sum
+                const dd rv = dd_add(r0, dd_mul(dd_make(dt), dd_mul(dd{b_ck_hi[k], b_ck_lo[k]}, v0)));
+                // sum_l Abar_kl f_l as a compensated dot product (Ogita, Rump and Oishi 2005, Dot2: the result of
+                // twice the working precision): one dependent addition per term instead of a double-double one
+                double s1 = 0, e1 = 0, s2 = 0;
+                const double *f = V.store + c * ld + b;
+                const int row = k * (k - 1) / 2;
 #pragma unroll 4
-                for (int j = 0; j < k; ++j) {
-                    const dd a = dd{b_rk_hi[ci0 + j], b_rk_lo[ci0 + j]};
-                    if (a.hi == 0) continue;
-                    const double fa = dd_val(a);
-                    const double *Fj = Y.acc + (size_t)j * kAcc * n + i;
-                    for (int c = 0; c < 3; ++c) {
-                        sv[c] = dd_add(sv[c], dd_mul(a, dd{Fj[(size_t)c * n], Fj[(size_t)(3 + c) * n]}));
-                        sa[c] = __dadd_rn(sa[c], __dmul_rn(fa, Fj[(size_t)(6 + c) * n]));
+                for (int l = 0; l < k; ++l) {
+                    const double2 ab = rk.ab[row + l];
+                    const double fl = f[3 * l * ld], h = ab.x;
+                    const double p = __dmul_rn(h, fl), pe = __fma_rn(rk.lo[row + l], fl, __fma_rn(h, fl, -p));
+                    double sum, se;
+                    two_sum(s1, p, sum, se);
+                    s1 = sum;
+                    e1 = __dadd_rn(e1, __dadd_rn(se, pe));
+                    s2 = __dadd_rn(s2, __dmul_rn(ab.y, fl));
+                }
+                dd sf;
+                two_sum_quick(s1, e1, sf.hi, sf.lo);
+                const dd r = dd_add(rv, dd_mul(dd_make(dt), dd_mul(dd_make(dt), sf)));
+                const dd v = dd_add(v0, dd_make(dt * s2));
+                double *a = A + (size_t)i * kRecA;
+                a[RA_R_HI + c] = r.hi;
+                a[RA_R_LO + c] = r.lo;
+                own_row(V, OR_V_HI + c, b) = v.hi;
+                own_row(V, OR_V_LO + c, b) = v.lo;
+                if (c == 0) {
+                    const double gm = own_row(V, OR_GM0, b) + own_row(V, OR_DGM, b) * t;
+                    a[RA_GM] = gm;
+                }
+            }
+            if (k == kStages)
+                for (int b = threadIdx.x; b < cnt; b += blockDim.x) orthogonalize_frame(pl, n, lo + b);
+            buf ^= 1;
+            if (peers > 1) {
+                __syncthreads();
+                send_all(A + (size_t)lo * kRecA, cnt * (kRecA / 2), peers, rank);
+            }
+            // The state records alternate between two arrays when a cluster shares the system: a peer that is
+            // still in the previous stage's pass B reads the other one, so one barrier per exchange is enough
+            sync();
+            // pass A (DAMPED_TIDAL_DEFORMATION_MATRIX_NK2, mass.impl:38-46), then PREPARE_RELATIVITY
+            // (mass.impl:76-80), one thread per (body, value)
+            for_units([&](int i, int j0, int j1, double *part) {
+                double p[kPartA];
+                sweep_point_a(A, i, j0, j1, p);
+                for (int c = 0; c < kPartA; ++c) part[c * units] = p[c];
+            }, [&](int b, int c, const double *part) {
+                double sum = 0;
+#pragma unroll 8
+                for (int q = 0; q < V.split; ++q) sum += part[c * units + q * cnt];
+                double *rec = rec_b(V, lo + b);
+                float *frec = V.F + (size_t)(lo + b) * kRecF;
+                auto beta = [&](int d) {
+                    return dd_val(dd{own_row(V, OR_V_HI + d, b), own_row(V, OR_V_LO + d, b)}) * (1.0 / kCB);
+                };
+                if (c == 0) {
+                    const v3 be = mk(beta(0), beta(1), beta(2));
+                    const double phi = sum / c2, b2 = dot(be, be);
+                    rec[RB_PHI] = phi;
+                    rec[RB_K] = phi + 2 * b2;
+                    if (MIXED) {
+                        frec[RF_PHI] = (float)phi;
+                        frec[RF_BETA2] = (float)b2;
+                        frec[RF_GM] = (float)A[(size_t)(lo + b) * kRecA + RA_GM];
+                    }
+                } else {
+                    const double na = sum * (1.0 / c2), be = beta(c - 1);
+                    rec[RB_NACC + c - 1] = na;
+                    rec[RB_BETA + c - 1] = be;
+                    if (MIXED) {
+                        frec[RF_NACC + c - 1] = (float)na;
+                        frec[RF_BETA + c - 1] = (float)be;
                     }
                 }
-                const dd ddt = dd_make(dt);
-                for (int c = 0; c < 3; ++c) {
-                    const dd r = dd_add(dd{Y.x0[(0 + c) * n + i], Y.x0[(3 + c) * n + i]}, dd_mul(ddt, sv[c]));
-                    const dd v = dd_add(dd{Y.x0[(6 + c) * n + i], Y.x0[(9 + c) * n + i]}, dd_make(dt * sa[c]));
-                    row(V, BR_R_HI + c, i) = r.hi;
-                    row(V, BR_R_LO + c, i) = r.lo;
-                    row(V, BR_V_HI + c, i) = v.hi;
-                    row(V, BR_V_LO + c, i) = v.lo;
+            });
+            if (peers > 1) {
+                __syncthreads();
+                if (MIXED) send_all(reinterpret_cast<double *>(V.F + (size_t)lo * kRecF), cnt * (kRecF / 4), peers, rank);
+                else send_all(V.B + (size_t)lo * kRecB, cnt * (kRecB / 2), peers, rank);
+            }
+            sync();
+            // pass B (RELATIVITY, mass.impl:82-97), then FINALIZE_RELATIVITY (mass.impl:133-135): f = (gaccel +
+            // daccel) + naccel, kept as f_k
+            for_units([&](int i, int j0, int j1, double *part) {
+                double p[kPartB];
+                if (MIXED) sweep_point_b32(A, V.F, i, j0, j1, p);
+                else sweep_point_b(A, V.B, i, j0, j1, p);
+                for (int c = 0; c < kPartB; ++c) part[c * units] = p[c];
+            }, [&](int b, int c, const double *part) {
+                if (c < 3) {
+                    double ga = 0;
+#pragma unroll 8
+                    for (int q = 0; q < V.split; ++q) ga += part[c * units + q * cnt];
+                    const double *rec = rec_b(V, lo + b);
+                    const double na = c2 * rec[RB_NACC + c];
+                    if (!MIXED) {
+                        const v3 be = mk(rec[RB_BETA], rec[RB_BETA + 1], rec[RB_BETA + 2]);
+                        ga += (4 * rec[RB_PHI] + dot(be, be)) * na;   // the terms common to all j
+                    }
+                    V.store[(3 * (k % kStages) + c) * V.ld + b] = ga + na;
+                    if (last) PLV(EPH_P_GACCEL + c, lo + b) = ga;
+                } else {
+                    double nan = 0, m_min = __longlong_as_double(0x7ff0000000000000ll), tq = 0;
+                    int tj = -1;
+#pragma unroll 4
+                    for (int q = 0; q < V.split; ++q) {
+                        const double *p = part + q * cnt;
+                        const double p0 = p[0], pm = p[3 * units], pt = p[4 * units];
+                        const int pj = __double2loint(p[5 * units]);
+                        nan += p0;
+                        m_min = pm < m_min ? pm : m_min;
+                        tj = pt > tq ? pj : tj;
+                        tq = pt > tq ? pt : tq;
+                    }
+                    if (nan != nan) extremes_nan(V, A, b);
+                    else extremes_add(V, A, b, m_min, tq, tj, MIXED ? 0x1p-18 : 0x1p-48);
                 }
-                row(V, BR_GM, i) = row(V, BR_GM0, i) + row(V, BR_DGM, i) * t;
-                frow(V, F_GM, i) = (float)row(V, BR_GM, i);
-                if (k == kStages) orthogonalize_frame(pl, n, i);
-            }
+            });
             __syncthreads();
-            if (coop) {
-                // every CTA of the cluster has finished the previous stage's pass B, which reads these rows
-                // in its own shared memory, before they are overwritten there
-                cg::this_cluster().sync();
-                broadcast_rows(V, BR_R_HI, BR_GM + 1 - BR_R_HI, lo, hi, rank);
-                if (MIXED) broadcast_frows(V, F_GM, 1, lo, hi, rank);
-                cg::this_cluster().sync();
-            }
-            pass_point_a(V, n, lo, hi);
-            if (coop) {
-                broadcast_rows(V, BR_PHI, BR_BETA2 + 1 - BR_PHI, lo, hi, rank);
-                if (MIXED) broadcast_frows(V, F_PHI, F_ROWS - F_PHI, lo, hi, rank);
-                cg::this_cluster().sync();
-            }
-            if (MIXED) pass_point_b32(V, n, lo, hi);
-            else pass_point_b(V, n, lo, hi);
         }
     }
     // store (cuda_rungekutta_kernel_config::save of RungeKutta.cu:124-133); min_distance inverted (mass.cpp:436)
-    const double c2 = kCB * kCB;
-    for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) {
+    for (int b = threadIdx.x; b < cnt; b += blockDim.x) {
+        const int i = lo + b;
+        const double *a = V.A[buf] + (size_t)i * kRecA, *rec = rec_b(V, i);
         for (int c = 0; c < 3; ++c) {
-            PLV(EPH_P_R_HI + c, i) = row(V, BR_R_HI + c, i);
-            PLV(EPH_P_R_LO + c, i) = row(V, BR_R_LO + c, i);
-            PLV(EPH_P_V_HI + c, i) = row(V, BR_V_HI + c, i);
-            PLV(EPH_P_V_LO + c, i) = row(V, BR_V_LO + c, i);
-            PLV(EPH_P_NACCEL + c, i) = c2 * row(V, BR_NACC + c, i);
-            PLV(EPH_P_GACCEL + c, i) = row(V, BR_GA + c, i);
+            PLV(EPH_P_R_HI + c, i) = a[RA_R_HI + c];
+            PLV(EPH_P_R_LO + c, i) = a[RA_R_LO + c];
+            PLV(EPH_P_V_HI + c, i) = own_row(V, OR_V_HI + c, b);
+            PLV(EPH_P_V_LO + c, i) = own_row(V, OR_V_LO + c, b);
+            PLV(EPH_P_NACCEL + c, i) = c2 * rec[RB_NACC + c];
             PLV(EPH_P_DACCEL + c, i) = 0.0;
             PLV(EPH_P_DTORQUE + c, i) = 0.0;
-            PLV(EPH_P_BETA + c, i) = row(V, BR_BETA + c, i);
+            PLV(EPH_P_BETA + c, i) = rec[RB_BETA + c];
         }
-        PLV(EPH_P_GM, i) = row(V, BR_GM, i);
-        PLV(EPH_P_PHI, i) = c2 * row(V, BR_PHI, i);
-        PLV(EPH_P_BETA2, i) = row(V, BR_BETA2, i);
-        PLV(EPH_P_MIN_DISTANCE, i) = 1 / row(V, BR_MIND, i);
-        PLV(EPH_P_MAX_INFLUENCE, i) = row(V, BR_MAXI, i);
+        PLV(EPH_P_GM, i) = a[RA_GM];
+        PLV(EPH_P_PHI, i) = c2 * rec[RB_PHI];
+        const v3 be = mk(rec[RB_BETA], rec[RB_BETA + 1], rec[RB_BETA + 2]);
+        PLV(EPH_P_BETA2, i) = dot(be, be);
+        PLV(EPH_P_MIN_DISTANCE, i) = 1 / sqrt(1.0 / own_row(V, OR_M, b));   // no pair seen: 1 / 0
+        PLV(EPH_P_MAX_INFLUENCE, i) = own_row(V, OR_MAXI, b);
     }
 #undef PLV
     __syncthreads();
 }
 
-// Persistent CTAs in clusters of kCluster. Jobs [0, n_coop) of the queue (the large systems) are taken a
-// cluster at a time and shared by its CTAs; once a cluster draws a job past them, its CTAs take the
-// remaining jobs one CTA each.
+// Persistent CTAs: every CTA (peers = 1) or thread-block cluster of `peers` CTAs takes systems from the queue
+// until it is empty.
 template <bool MIXED>
-__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kBThreads, 2)
-    ensemble_kernel(const BatchSys *sys, const int *order, int n_sys, int n_coop, int *next, int ld) {
+__global__ void __launch_bounds__(kBThreads, 2)
+    ensemble_kernel(const BatchSys *sys, const int *order, int n_jobs, int *next, int peers) {
     extern __shared__ __align__(16) double bsm[];
+    __shared__ RkTable rk;
     __shared__ int s_job;
-    const BatchView V{bsm, ld};
     cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    bool together = true;
+    for (int q = threadIdx.x; q < EPH_RK12_NCOEF; q += blockDim.x) {
+        rk.ab[q] = make_double2(b_ab_hi[q], b_a[q]);
+        rk.lo[q] = b_ab_lo[q];
+    }
+    __syncthreads();
+    const int rank = peers > 1 ? (int)cl.block_rank() : 0;
 #pragma unroll 1
     for (;;) {
         int job;
-        if (together) {
+        if (peers > 1) {
             cl.sync();   // every CTA of the cluster is done with the previous job and its shared memory
             if (rank == 0 && threadIdx.x == 0) s_job = atomicAdd(next, 1);
             cl.sync();
             job = *cl.map_shared_rank(&s_job, 0);
-            cl.sync();   // read by all before rank 0 may reuse s_job
-            if (job >= n_sys) return;
-            if (job < n_coop) {
-                integrate_system<MIXED>(sys[order[job]], V, true, rank);
-                continue;
-            }
-            together = false;
-            if (rank != 0) continue;   // rank 0 keeps this job, the others draw their own
+            cl.sync();   // read by all before rank 0 may reuse s_job, or leave
         } else {
             if (threadIdx.x == 0) s_job = atomicAdd(next, 1);
             __syncthreads();
             job = s_job;
             __syncthreads();
-            if (job >= n_sys) return;
         }
-        integrate_system<MIXED>(sys[order[job]], V, false, 0);
+        if (job >= n_jobs) return;
+        integrate_system<MIXED>(sys[order[job]], rk, bsm, peers, rank);
     }
 }
 
-size_t ensemble_smem(int ld) { return (size_t)BR_ROWS * ld * sizeof(double); }
-constexpr size_t kBMaxSmem = 227 * 1024 - 1024;
-int ensemble_max_bodies() { return (int)(kBMaxSmem / sizeof(double) / BR_ROWS) / kPad * kPad; }
+constexpr size_t kBMaxSmem = 227 * 1024 - sizeof(RkTable) - 256;
+// ---- how many CTAs share a system
+constexpr int kShares = 5;
+constexpr int kSharePeers[kShares] = {16, 8, 4, 2, 1};
+constexpr int kMinOwn = 12;  // bodies per CTA below which sharing a system further does not pay
+
+// Time of one stage (us) of a system of n bodies on `peers` CTAs, its j ranges cut into `split` parts: a model
+// of measurements on one B200 (single systems of 8-400 bodies on 1-16 CTAs): 2.6 us for the state update and the
+// phases per body, 1.3 us for the two cluster exchanges, and per unit of a thread 0.36 us a pair (both passes;
+// FP64 latency at 8 warps) and 0.3 us.
+float stage_us(int n, int peers, int split) {
+    const int per_thread = ((n + peers - 1) / peers * split + kBThreads - 1) / kBThreads;
+    return 2.6f + (peers > 1 ? 1.3f : 0.0f) + (float)per_thread * (0.36f * (float)((n + split - 1) / split) + 0.3f);
+}
+// Parts that each body's j range is cut into: the number that keeps the threads busiest over the CTA counts the
+// system may be shared by. It depends on n alone, so that a system's sums are the same however it is shared.
+constexpr int kMaxPerThread = 4;   // units per thread, by the shared memory of their sums
+int batch_split(int n) {
+    int best = 1;
+    float best_cost = 1e30f;
+    for (int g = 1; g <= kMaxSplit && g <= n; ++g) {
+        float cost = 0;
+        for (int peers : kSharePeers) {
+            const int cnt = (n + peers - 1) / peers;
+            if ((peers > 1 && n < kMinOwn * peers) || cnt * g > kMaxPerThread * kBThreads) continue;
+            cost += stage_us(n, peers, g) / stage_us(n, peers, std::max(1, std::min(n, kBThreads / cnt)));
+        }
+        // (the same CTA counts enter every candidate's mean)
+        int counted = 0;
+        for (int peers : kSharePeers)
+            counted += !((peers > 1 && n < kMinOwn * peers) || (n + peers - 1) / peers * g > kMaxPerThread * kBThreads);
+        if (counted && cost / counted < best_cost) { best_cost = cost / counted; best = g; }
+    }
+    return best;
+}
+bool share_fits(int n, int peers, int split) { return (n + peers - 1) / peers * split <= kMaxPerThread * kBThreads; }
+
+size_t system_smem(int n, int peers, int split, bool mixed) {
+    bool in_smem;
+    return batch_smem_doubles(n, peers, split, mixed, &in_smem) * sizeof(double);
+}
+constexpr int kMaxBodies = 768;   // bodies of a system of the ensemble launch: shared memory holds it on one CTA
 
 bool g_batch_ready[64];
 cudaError_t batch_setup(int device) {
     if (device >= 0 && device < 64 && g_batch_ready[device]) return cudaSuccess;
     double hi[EPH_RK12_NCOEF], lo[EPH_RK12_NCOEF], dtk[kStages + 1];
     rk12_expand(hi, lo, dtk);
-    cudaError_t e = cudaMemcpyToSymbol(b_rk_hi, hi, sizeof(hi));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(b_rk_lo, lo, sizeof(lo));
+    double ab_hi[EPH_RK12_NCOEF] = {0}, ab_lo[EPH_RK12_NCOEF] = {0}, aa[EPH_RK12_NCOEF] = {0};
+    double ck_hi[kStages + 1] = {0}, ck_lo[kStages + 1] = {0};
+    auto coef = [&](int k, int j) { return (long double)hi[k * (k - 1) / 2 + j] + lo[k * (k - 1) / 2 + j]; };
+    auto split = [](long double x, double &h, double &l) { h = (double)x; l = (double)(x - h); };
+    for (int k = 1; k <= kStages; ++k) {
+        long double c = 0;
+        for (int l = 0; l < k; ++l) {
+            const int q = k * (k - 1) / 2 + l;
+            long double acc = 0;   // Abar_kl = sum_{l<j<k} a_kj a_jl
+            for (int j = l + 1; j < k; ++j) acc += coef(k, j) * coef(j, l);
+            split(acc, ab_hi[q], ab_lo[q]);
+            aa[q] = hi[q] + lo[q];
+            c += coef(k, l);
+        }
+        split(c, ck_hi[k], ck_lo[k]);
+    }
+    cudaError_t e = cudaMemcpyToSymbol(b_ab_hi, ab_hi, sizeof(ab_hi));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(b_ab_lo, ab_lo, sizeof(ab_lo));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(b_a, aa, sizeof(aa));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(b_ck_hi, ck_hi, sizeof(ck_hi));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(b_ck_lo, ck_lo, sizeof(ck_lo));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(b_dtk, dtk, sizeof(dtk));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(ensemble_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBMaxSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(ensemble_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBMaxSmem);
+    // clusters of 16 CTAs: twice the portable size
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(ensemble_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(ensemble_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess && device >= 0 && device < 64) g_batch_ready[device] = true;
     return e;
 }
@@ -678,6 +716,8 @@ struct eph_batch {
     int device = 0;
     cudaStream_t stream = nullptr;     // work stream (own_stream unless eph_batch_set_stream chose another)
     cudaStream_t own_stream = nullptr;
+    cudaStream_t side[kShares] = {};   // the launches of one integration run beside each other
+    cudaEvent_t ev_begin = nullptr, ev_end[kShares] = {};
     int mixed = 0;                     // 1: EIH 1PN terms of the ensemble kernel in FP32 (eph_batch_set_precision)
     int coop_min = kCoopMin;           // bodies from which a system is shared by a cluster (eph_batch_set_coop_min)
     std::mutex mu;
@@ -685,15 +725,15 @@ struct eph_batch {
     int n_sys = 0;
     std::vector<int64_t> n_body;
     std::vector<int> point;                    // 1: ensemble kernel, 0: per-system context path
+    std::vector<int> split;                    // parts of a body's j range (batch_split)
     std::vector<size_t> off;                   // offset of system s in d_planes (doubles)
-    std::vector<size_t> acc_off, x0_off;       // offsets of its scratch (doubles)
+    std::vector<size_t> store_off;             // offset of its stage store (doubles)
     std::vector<std::vector<double>> h_full;   // host copies of the context-path systems' planes
     std::vector<std::vector<int32_t>> m_gp_nz, m_gp_nt, m_ring_nd;
     std::vector<std::vector<double>> m_gp_coef, m_ring_param, m_ring_disk;
-    double *d_planes = nullptr, *d_acc = nullptr, *d_x0 = nullptr;
+    double *d_planes = nullptr, *d_store = nullptr;
     BatchSys *d_sys = nullptr;
     int *d_order = nullptr, *d_next = nullptr;
-    int ld = 0;                                // shared-memory row stride (largest ensemble system, padded)
     eph_ctx *ctx = nullptr;                    // context path
     int64_t launches = 0;
 };
@@ -712,13 +752,21 @@ static int bfail(eph_batch *b, int code, const char *what, cudaError_t e = cudaS
     } while (0)
 
 static void batch_free(eph_batch *b) {
-    for (void *p : {(void *)b->d_planes, (void *)b->d_acc, (void *)b->d_x0, (void *)b->d_sys, (void *)b->d_order,
+    for (void *p : {(void *)b->d_planes, (void *)b->d_store, (void *)b->d_sys, (void *)b->d_order,
                     (void *)b->d_next})
         if (p) cudaFree(p);
-    b->d_planes = b->d_acc = b->d_x0 = nullptr;
+    b->d_planes = b->d_store = nullptr;
     b->d_sys = nullptr;
     b->d_order = b->d_next = nullptr;
     b->n_sys = 0;
+}
+
+static bool batch_side(eph_batch *b) {   // the side streams of an integration's launches, and their events
+    bool ok = cudaEventCreateWithFlags(&b->ev_begin, cudaEventDisableTiming) == cudaSuccess;
+    for (int g = 0; g < kShares; ++g)
+        ok = ok && cudaStreamCreateWithFlags(&b->side[g], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&b->ev_end[g], cudaEventDisableTiming) == cudaSuccess;
+    return ok;
 }
 
 extern "C" {
@@ -731,8 +779,8 @@ int eph_batch_create(int device, eph_batch **out) {
     eph_batch *b = new eph_batch();
     b->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        batch_setup(device) != cudaSuccess) {
-        delete b;
+        batch_setup(device) != cudaSuccess || !batch_side(b)) {
+        eph_batch_destroy(b);
         return EPH_ERR_CUDA;
     }
     *out = b;
@@ -743,6 +791,11 @@ int eph_batch_destroy(eph_batch *b) {
     if (!b) return EPH_ERR_ARG;
     cudaSetDevice(b->device);
     batch_free(b);
+    for (int g = 0; g < kShares; ++g) {
+        if (b->side[g]) cudaStreamDestroy(b->side[g]);
+        if (b->ev_end[g]) cudaEventDestroy(b->ev_end[g]);
+    }
+    if (b->ev_begin) cudaEventDestroy(b->ev_begin);
     if (b->ctx) eph_ctx_destroy(b->ctx);
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     else if (b->stream) cudaStreamDestroy(b->stream);
@@ -769,28 +822,24 @@ int eph_batch_upload(eph_batch *b, int32_t n_sys, const int64_t *n_body, const d
     b->n_sys = n_sys;
     b->n_body.assign(n_body, n_body + n_sys);
     b->point.assign(n_sys, 0);
+    b->split.assign(n_sys, 1);
     b->off.assign(n_sys, 0);
-    b->acc_off.assign(n_sys, 0);
-    b->x0_off.assign(n_sys, 0);
+    b->store_off.assign(n_sys, 0);
     b->h_full.assign(n_sys, {});
     b->m_gp_nz.assign(n_sys, {}); b->m_gp_nt.assign(n_sys, {}); b->m_ring_nd.assign(n_sys, {});
     b->m_gp_coef.assign(n_sys, {}); b->m_ring_param.assign(n_sys, {}); b->m_ring_disk.assign(n_sys, {});
-    const int nmax = ensemble_max_bodies();
-    size_t tot = 0, tot_acc = 0, tot_x0 = 0;
-    int ld = 0;
+    size_t tot = 0, tot_store = 0;
     for (int s = 0; s < n_sys; ++s) {
         const int n = (int)n_body[s];
-        bool pt = n <= nmax;
+        bool pt = n <= kMaxBodies;
         for (int i = 0; i < n && pt; ++i) pt = !plan_full_class(planes[s], n, i);
         b->point[s] = pt;
         if (pt) {
+            b->split[s] = batch_split(n);
             b->off[s] = tot;
-            b->acc_off[s] = tot_acc;
-            b->x0_off[s] = tot_x0;
+            b->store_off[s] = tot_store;
             tot += (size_t)EPH_NPLANES * n;
-            tot_acc += (size_t)n * kStages * kAcc;
-            tot_x0 += (size_t)12 * n;
-            ld = std::max(ld, (n + kPad - 1) / kPad * kPad);
+            tot_store += (size_t)kStore * n;
         } else {
             b->h_full[s].assign(planes[s], planes[s] + (size_t)EPH_NPLANES * n);
             const eph_models *m = models ? models[s] : nullptr;
@@ -806,14 +855,12 @@ int eph_batch_upload(eph_batch *b, int32_t n_sys, const int64_t *n_body, const d
             }
         }
     }
-    b->ld = ld;
-    if (tot) {
+        if (tot) {
         BCK(cudaMalloc(&b->d_planes, tot * sizeof(double)), "cudaMalloc(batch planes)");
-        BCK(cudaMalloc(&b->d_acc, tot_acc * sizeof(double)), "cudaMalloc(batch accumulators)");
-        BCK(cudaMalloc(&b->d_x0, tot_x0 * sizeof(double)), "cudaMalloc(batch start states)");
+        BCK(cudaMalloc(&b->d_store, tot_store * sizeof(double)), "cudaMalloc(batch stage store)");
         BCK(cudaMalloc(&b->d_sys, (size_t)n_sys * sizeof(BatchSys)), "cudaMalloc(batch table)");
         BCK(cudaMalloc(&b->d_order, (size_t)n_sys * sizeof(int)), "cudaMalloc(batch order)");
-        BCK(cudaMalloc(&b->d_next, sizeof(int)), "cudaMalloc(batch queue)");
+        BCK(cudaMalloc(&b->d_next, kShares * sizeof(int)), "cudaMalloc(batch queues)");
         for (int s = 0; s < n_sys; ++s)
             if (b->point[s])
                 BCK(cudaMemcpyAsync(b->d_planes + b->off[s], planes[s], (size_t)EPH_NPLANES * n_body[s] * sizeof(double),
@@ -830,53 +877,96 @@ int eph_batch_integrate(eph_batch *b, const double *dt, const int64_t *n_step, d
     BCK(cudaSetDevice(b->device), "cudaSetDevice");
     const int n_sys = b->n_sys;
     std::vector<BatchSys> tab(n_sys);
-    std::vector<int> order;
-    std::vector<double> work(n_sys, 0.0);
+    std::vector<int> order, share(n_sys, kShares - 1);
+    std::vector<double> stage(n_sys, 0.0), work(n_sys, 0.0);
+    int sms = 0;
+    BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device), "SM count");
     for (int s = 0; s < n_sys; ++s) {
         if (!b->point[s] || n_step[s] == 0) continue;
         BatchSys &Y = tab[s];
         const int n = (int)b->n_body[s];
         Y.n = n;
-        Y.pad = 0;
+        Y.split = b->split[s];
         // msystem::integrate: a negative step count integrates backwards (mass.cpp:401-404)
         Y.n_step = n_step[s] < 0 ? -n_step[s] : n_step[s];
         Y.dt = n_step[s] < 0 ? -dt[s] : dt[s];
         Y.t_eph = t_eph_hi[s] + t_eph_lo[s];
         Y.planes = b->d_planes + b->off[s];
-        Y.acc = b->d_acc + b->acc_off[s];
-        Y.x0 = b->d_x0 + b->x0_off[s];
-        work[s] = (double)n * (double)n * (double)Y.n_step;
+        Y.store = b->d_store + b->store_off[s];
         order.push_back(s);
     }
-    // the large systems (shared by a cluster) first, then the others; each group heaviest first, so the
-    // last systems to start are short ones
+    // CTAs per system. A system on one CTA does the least work in all, one shared by a cluster is done sooner: as
+    // long as the longest job would outlast the whole batch's work spread over the SMs (two CTAs each), it is given
+    // twice the CTAs. The choice changes no result.
+    {
+        auto job = [&](int s, int g) { return (double)stage_us((int)b->n_body[s], kSharePeers[g], b->split[s]) * (double)tab[s].n_step; };
+        double total = 0;
+        std::vector<std::pair<double, int>> heap;   // (duration, system), longest on top
+        for (int s : order) {
+            while (share[s] > 0 && (!share_fits((int)b->n_body[s], kSharePeers[share[s]], b->split[s]) || system_smem((int)b->n_body[s], kSharePeers[share[s]], b->split[s], b->mixed) > kBMaxSmem)) --share[s];
+            work[s] = job(s, share[s]);
+            total += work[s] * kSharePeers[share[s]];
+            heap.emplace_back(work[s], s);
+        }
+        std::make_heap(heap.begin(), heap.end());
+        while (!heap.empty() && heap.front().first > 1.1 * total / (2.0 * sms)) {
+            std::pop_heap(heap.begin(), heap.end());
+            const int s = heap.back().second, g = share[s] - 1;
+            heap.pop_back();
+            if (g < 0 || b->n_body[s] < b->coop_min || b->n_body[s] < kMinOwn * kSharePeers[g]) break;
+            const double d = job(s, g);
+            if (d > 0.95 * work[s]) break;
+            total += d * kSharePeers[g] - work[s] * kSharePeers[g + 1];
+            share[s] = g;
+            work[s] = d;
+            heap.emplace_back(d, s);
+            std::push_heap(heap.begin(), heap.end());
+        }
+    }
+    // one launch for each number of CTAs; in each the longest job first, so that the last to start are short ones
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) {
-        const bool ca = b->n_body[a] >= b->coop_min, cc = b->n_body[c] >= b->coop_min;
-        if (ca != cc) return ca;
+        if (share[a] != share[c]) return share[a] < share[c];
         return work[a] > work[c];
     });
-    int n_coop = 0;
-    for (int s : order) n_coop += b->n_body[s] >= b->coop_min;
     if (!order.empty()) {
         BCK(cudaMemcpyAsync(b->d_sys, tab.data(), (size_t)n_sys * sizeof(BatchSys), cudaMemcpyHostToDevice, b->stream),
             "upload batch table");
         BCK(cudaMemcpyAsync(b->d_order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream),
             "upload batch order");
-        BCK(cudaMemsetAsync(b->d_next, 0, sizeof(int), b->stream), "reset batch queue");
-        const size_t smem = ensemble_smem(b->ld);
-        int per_sm = 0, sms = 0;
-        BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ensemble_kernel<false>, kBThreads, smem), "occupancy");
-        BCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device), "SM count");
-        // whole clusters; clusters that find no room start when others finish (no CTA waits on another cluster)
-        int grid = std::min((int)order.size() * kCluster, std::max(per_sm * sms, kCluster));
-        grid = std::max(kCluster, grid / kCluster * kCluster);
-        const int nj = (int)order.size();
-        if (b->mixed)
-            ensemble_kernel<true><<<grid, kBThreads, smem, b->stream>>>(b->d_sys, b->d_order, nj, n_coop, b->d_next, b->ld);
-        else
-            ensemble_kernel<false><<<grid, kBThreads, smem, b->stream>>>(b->d_sys, b->d_order, nj, n_coop, b->d_next, b->ld);
-        BCK(cudaGetLastError(), "launch ensemble kernel");
-        b->launches++;
+        BCK(cudaMemsetAsync(b->d_next, 0, kShares * sizeof(int), b->stream), "reset batch queues");
+        BCK(cudaEventRecord(b->ev_begin, b->stream), "batch event");
+        auto kernel = b->mixed ? ensemble_kernel<true> : ensemble_kernel<false>;
+        size_t begin = 0;
+        for (int g = 0; g < kShares; ++g) {
+            // side by side: the CTAs of a later launch start as the SMs come free (no CTA waits on another cluster)
+            size_t end = begin, smem = 0;
+            const int peers = kSharePeers[g];
+            for (; end < order.size() && share[order[end]] == g; ++end)
+                smem = std::max(smem, system_smem((int)b->n_body[order[end]], peers, b->split[order[end]], b->mixed));
+            const int jobs = (int)(end - begin);
+            if (!jobs) continue;
+            cudaLaunchAttribute attr{};
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = peers;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(peers);
+            cfg.blockDim = dim3(kBThreads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = b->side[g];
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            BCK(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg), "occupancy");
+            cfg.gridDim = dim3(peers * std::max(1, std::min(jobs, clusters)));
+            BCK(cudaStreamWaitEvent(b->side[g], b->ev_begin, 0), "batch event");
+            BCK(cudaLaunchKernelEx(&cfg, kernel, (const BatchSys *)b->d_sys, (const int *)b->d_order + begin, jobs,
+                                   b->d_next + g, peers), "launch ensemble kernel");
+            BCK(cudaEventRecord(b->ev_end[g], b->side[g]), "batch event");
+            BCK(cudaStreamWaitEvent(b->stream, b->ev_end[g], 0), "batch event");
+            b->launches++;
+            begin = end;
+        }
     }
     // the other systems through the per-system kernel, while the ensemble kernel runs
     for (int s = 0; s < n_sys; ++s) {

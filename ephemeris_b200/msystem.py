@@ -208,7 +208,7 @@ class Batch:
         self.sizes = [p.shape[1] for p in pls]
 
     def set_coop_min(self, bodies: int = 0):
-        """Bodies from which a system is shared by a 4-CTA cluster (0: the default)."""
+        """Bodies from which a system may be shared by the CTAs of a cluster (0: the default)."""
         self._check(self.lib.eph_batch_set_coop_min(self.h, bodies), "batch set_coop_min")
 
     def autotune(self, dt, n_step, step_frac: float = 0.05):

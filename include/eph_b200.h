@@ -133,7 +133,7 @@ int eph_phase_times(eph_ctx *ctx, uint64_t *out, int *grid, int *phases);
  * combined integrator runs subsystems one at a time, mass_combined.cpp:286-321). Many independent systems,
  * each with its own dt, step count and ephemeris time, integrated with msystem::integrate semantics
  * (mass.cpp:399-442). Systems whose bodies are all point-like (Newtonian + 1PN only) share one persistent
- * launch, one CTA per system; any other system runs through the single-system kernel. */
+ * launch for each number of CTAs per system (1 to 16); any other system runs through the single-system kernel. */
 /* Arithmetic modes of the batched and particle paths */
 #define EPH_PREC_FP64 0
 #define EPH_PREC_MIXED 1
@@ -159,8 +159,9 @@ int eph_batch_set_stream(eph_batch *b, void *stream);
  * totals; state, separations, the Newtonian sums, the per-pair maxima and the RK12 combination stay FP64 /
  * double-double). Applies from the next integrate; systems on the single-system path are not affected. */
 int eph_batch_set_precision(eph_batch *b, int mode);
-/* Systems of at least `bodies` bodies are shared by the 4 CTAs of a thread-block cluster in the ensemble
- * launch (0: the default, 96). */
+/* Systems of at least `bodies` bodies may be shared by the CTAs (up to 16) of a thread-block cluster in the ensemble
+ * launches (0: the default, 32); how many share one follows from the batch, and changes no result. A system too
+ * large for one CTA's shared memory is shared whatever the threshold. */
 int eph_batch_set_coop_min(eph_batch *b, int bodies);
 /* Autotuner of the ensemble launch: times the uploaded batch's shared launch (step counts scaled by
  * step_frac, so the members keep their relative durations; best of 2 from the uploaded state, which is

@@ -308,7 +308,8 @@ int eph_device_planes(eph_ctx *ctx, double **d_planes) {
 
 }  // extern "C"
 
-static int run(eph_ctx *ctx, const StepParams &P) {
+// Launches the step kernel on the context's stream (no wait); `finish` waits for it and reads its status.
+static int launch(eph_ctx *ctx, const StepParams &P) {
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     if (!ctx->n) return fail(ctx, EPH_ERR_STATE, "no system uploaded");
     SysDev S;
@@ -353,6 +354,11 @@ static int run(eph_ctx *ctx, const StepParams &P) {
     CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "reset status");
     CK(launch_step(S, P, ctx->grid, ctx->stream), "launch RK12 kernel");
     ctx->launches++;
+    return EPH_OK;
+}
+
+static int finish(eph_ctx *ctx) {
+    CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     int status = 0;
     CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "read status");
     CK(cudaStreamSynchronize(ctx->stream), "RK12 kernel");
@@ -361,6 +367,25 @@ static int run(eph_ctx *ctx, const StepParams &P) {
     if (status != ST_OK) return fail(ctx, EPH_ERR_CUDA, "step kernel reported an unknown status");
     return EPH_OK;
 }
+
+static int run(eph_ctx *ctx, const StepParams &P) {
+    const int rc = launch(ctx, P);
+    return rc ? rc : finish(ctx);
+}
+
+namespace eph {
+// eph_rk12 in two halves, for work that runs beside it: launched on the context's stream after `after` (an event,
+// or null), and waited for.
+int ctx_rk12_begin(eph_ctx *ctx, double dt, long long n_step, double t_eph, cudaEvent_t after) {
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    if (after) CK(cudaStreamWaitEvent(ctx->stream, after, 0), "wait for event");
+    return launch(ctx, StepParams{MODE_INTEGRATE, 0, 0, n_step, dt, t_eph});
+}
+int ctx_rk12_end(eph_ctx *ctx) {
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return finish(ctx);
+}
+}  // namespace eph
 
 extern "C" {
 

@@ -948,7 +948,7 @@ __device__ __noinline__ void record_body(const SysDev &S, const Own &o, long lon
     }
     t[TR_GM] = o.GM;
     t[TR_PHI] = o.phi;
-    t[TR_BETA2] = o.beta2;
+    t[TR_K] = o.phi + 2 * o.beta2;
     for (int q = 0; q < 9; ++q) t[TR_CPOT + q] = o.C[q];
     t[TR_R2] = o.R2;
     const v3 gl = fast3(o.GL);

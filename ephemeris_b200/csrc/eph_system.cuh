@@ -92,10 +92,10 @@ struct SysDev {
 constexpr long long kWaitDefaultNs = 2000000000ll;   // 2 s
 
 // One stage record of a body (written after pass A, caller's body order): what a massless particle's
-// stage evaluation reads of the massive bodies.
-enum TrajField { TR_R_HI = 0, TR_R_LO = 3, TR_GM = 6, TR_PHI = 7, TR_NACC = 8, TR_BETA = 11, TR_BETA2 = 14,
-                 TR_CPOT = 15, TR_R2 = 24, TR_GL = 25, TR_FRAME = 28, TR_RADIUS = 37, TR_SR2 = 38, TR_RFRAME = 39,
-                 kTrajRec = 48 };
+// stage evaluation reads of the massive bodies. The first 16 fields are what a point-mass perturber acts with, in the
+// order in which the particle kernel reads them, 16 bytes at a time; K = phi / c^2 + 2 beta^2.
+enum TrajField { TR_R_HI = 0, TR_R_LO = 3, TR_GM = 6, TR_SR2 = 7, TR_NACC = 8, TR_BETA = 11, TR_K = 14, TR_PHI = 15,
+                 TR_CPOT = 16, TR_R2 = 25, TR_GL = 26, TR_FRAME = 29, TR_RADIUS = 38, TR_RFRAME = 39, kTrajRec = 48 };
 
 // phases of a stage evaluation, for the optional per-CTA phase timers
 // (slot PH_A_COUNT counts the pass-A sweeps instead of nanoseconds)

@@ -54,7 +54,8 @@ long long ctx_size(const eph_ctx *ctx);
 namespace eph {
 namespace {
 
-constexpr int kSThreads = 256;
+constexpr int kSThreads = 256;                 // most threads of a block that carry particles
+constexpr int kSLaunch = kSThreads + 128;      // threads of a block: four warps more evaluate perturbers
 constexpr size_t kFreeReserve = 1ull << 30;   // device memory kept free when admitting by free memory
 constexpr int kSmemSlots = 64;   // particles per block whose stage store fits shared memory
 constexpr int kSStreams = 128;   // requests in flight at once (the device runs up to 128 kernels concurrently)
@@ -62,7 +63,10 @@ constexpr int kChan = EPH_EPHEM_CHANNELS;   // x y z vx vy vz aN/c^2 (3) phi/c^2
 constexpr double kCS = 299792458.0;         // src/math/basic_math.h:10,18
 constexpr long long kMaxAttempts = 1ll << 22;
 constexpr unsigned long long kRequestNs = 300ull * 1000000000ull;   // device-time limit of one request
-enum SRow { S_RX = 0, S_RY, S_RZ, S_BX, S_BY, S_BZ, S_B2, S_PHI, S_NX, S_NY, S_NZ, S_GM, S_SR2, kSRows };
+// A perturber's record in shared memory: the channels at one time (velocity over c; K = phi / c^2 + 2 beta^2 in
+// place of the potential), then GM. 11 doubles apart, 32 lanes reading one field of 32 consecutive records meet no bank
+// conflict, and every field is a fixed offset from the record's address.
+enum SRec { S_R = 0, S_B = 3, S_N = 6, S_K = 9, S_GM = 10, kSRec = 11 };
 enum SStatus { SS_OK = 0, SS_STEP_UNDERFLOW = 1, SS_ATTEMPTS = 2, SS_DEADLINE = 3 };
 
 __device__ __forceinline__ unsigned long long now_ns() {
@@ -71,8 +75,11 @@ __device__ __forceinline__ unsigned long long now_ns() {
     return t;
 }
 
-__constant__ double q_a[EPH_RK12_NCOEF];
-__constant__ double q_abar[EPH_RK12_NCOEF];
+// The Feagin table as the request kernel uses it: c_k and the rows k = 1..25 of a (hi + lo rounded) and of the
+// second-order Abar = A A without the columns where both are zero (entries q_row[k] <= q < q_row[k + 1], ascending).
+__constant__ double2 q_ab[EPH_RK12_NCOEF];   // {Abar_kl, a_kl}
+__constant__ int q_l[EPH_RK12_NCOEF];
+__constant__ int q_row[kStages + 2];
 __constant__ double q_c[kStages + 1];
 
 struct ServeArgs {
@@ -80,13 +87,15 @@ struct ServeArgs {
     const double *coef;        // [M][n + d][kChan]
     const double *gm, *sr2;    // [M]
     const double *cheb;        // [(d + 1)^2]: c(d, k, j)
-    int M, Mpad, d;
+    int M, d;
+    int buffers;               // 2: the perturbers of the next stage are formed beside the present one's sums; 1: before them
+    int soft;                  // any sR2 is not zero
     long long n;
     double t0, knot;
     // request
     double *state;             // [12][P] in place: r hi, r lo, v hi, v lo
     double *fstore;            // [grid][kStages][3][S] (blocks of more than kSmemSlots particles)
-    int P, G;
+    int P, G, S;               // particles, lanes per particle, particles per block
     double t_start, t_end, tol, h0, hmin;
     long long *stats;          // [grid][2]: accepted, rejected
     int *status;               // [grid]
@@ -99,244 +108,256 @@ __device__ __forceinline__ double group_sum(double v, int G) {
     return v;
 }
 
-// channel values of all perturbers from the interval's coefficients and the basis values b. D > 0: degree
-// known at compile time, four items per pass with all their coefficient loads issued before any is used
-// (they come from L2); D = 0: any degree, one item at a time.
-template <int D>
-__device__ __forceinline__ void eval_items(const ServeArgs &A, double *PR, const double *cheb, double u, long long xi) {
-    const int d = D > 0 ? D : A.d;
-    // basis values B[d, x - (xi + k)], k = 0..d, at u = 2 (x - xi) - 1 from their Chebyshev form
-    constexpr int NB = D > 0 ? D + 1 : EPH_BSPLINE_MAX_DEGREE + 1;
-    double b[NB];
-    const double u2 = 2 * u;
-#pragma unroll
-    for (int k = 0; k < NB; ++k) {
-        if (k > d) break;
-        const double *c = cheb + k * (d + 1);
-        double sum = c[0] + c[1] * u, tm, tt = 1, tp = u;
+// The perturbers at time t into the shared records PR, by the warps that call it: chunks of 6 U bodies are
+// taken from the counter *take until none is left. Lanes 5 b + p (b < 6, p < 5) take channels 2 p and 2 p + 1 of body
+// b of six, so a warp reads 80 contiguous bytes per body and coefficient with 16-byte loads, and K is formed from
+// its neighbours' channels by shuffles. No barrier.
+// D > 0: degree known at compile time, U rounds of six bodies with all their coefficient loads issued before any is
+// used (they come from L2: 8 bytes at a time, a body and channel per lane, the loads and their index arithmetic were a
+// fifth of the kernel's instructions); D = 0: any degree. kRaw: the channels as they are fitted.
+template <int D, bool kRaw>
+__device__ __noinline__ void eval_rows(const double *__restrict__ coef, long long n, int deg, int M, double t0, double knot,
+                                       double *PR, const double *cheb, double t, int *take) {
+    const int lane = threadIdx.x & 31, d = D > 0 ? D : deg;
+    constexpr int U = D > 0 ? 3 : 1;
+    constexpr int NK = D > 0 ? D + 1 : EPH_BSPLINE_MAX_DEGREE + 1;
+    constexpr double inv_c = 1.0 / kCS;
+    const double x = (t - t0) / knot;
+    long long xi = (long long)floor(x);
+    xi = xi < 0 ? 0 : (xi > n - 1 ? n - 1 : xi);
+    // lane k holds the basis value B[d, x - (xi + k)], k = 0..d, at u = 2 (x - xi) - 1 from its Chebyshev form
+    const double u = 2 * (x - (double)xi) - 1, u2 = 2 * u;
+    double mine;
+    {
+        const double *c = cheb + min(lane, d) * (d + 1);
+        double tm, tt = 1, tp = u;
+        mine = c[0] + c[1] * u;
         for (int j = 2; j <= d; ++j) {
             tm = tt;
             tt = tp;
             tp = u2 * tt - tm;
-            sum += c[j] * tp;
+            mine += c[j] * tp;
         }
-        b[k] = sum;
     }
-    const long long stride = A.n + d;
-    const int total = A.M * kChan;
-    constexpr int U = D > 0 ? 4 : 1;
-    constexpr int NK = D > 0 ? D + 1 : EPH_BSPLINE_MAX_DEGREE + 1;
+    double b[NK];
+#pragma unroll
+    for (int k = 0; k < NK; ++k) b[k] = __shfl_sync(0xffffffffu, mine, min(k, d));
+    const long long stride = (n + d) * kChan;   // doubles per body
+    const int p = lane % 5, six = min(lane / 5, 5);
+    const double *at = coef + xi * kChan + 2 * p;
 #pragma unroll 1
-    for (int item0 = threadIdx.x; item0 < total; item0 += U * blockDim.x) {
-        double cf[U][NK];
+    for (;;) {
+        int chunk = 0;
+        if (lane == 0) chunk = atomicAdd(take, 1);
+        const int base = __shfl_sync(0xffffffffu, chunk, 0) * (6 * U);
+        if (base >= M) break;
+        double2 cf[U][NK];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int item = item0 + u * blockDim.x;
-            const int it = item < total ? item : total - 1;
-            const double *c = A.coef + ((size_t)(it / kChan) * stride + xi) * kChan + it % kChan;
-            if (D > 0) {
+        for (int q = 0; q < U; ++q) {
+            const int body = min(base + q * 6 + six, M - 1);
+            const double2 *c = reinterpret_cast<const double2 *>(at + body * stride);
 #pragma unroll
-                for (int k = 0; k < NK; ++k) cf[u][k] = __ldg(c + (size_t)k * kChan);
-            } else {
-                for (int k = 0; k <= d; ++k) cf[u][k] = __ldg(c + (size_t)k * kChan);
-            }
+            for (int k = 0; k < NK; ++k)
+                if (D > 0 || k <= d) cf[q][k] = __ldg(c + k * (kChan / 2));
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int item = item0 + u * blockDim.x;
-            if (item >= total) break;
-            const int body = item / kChan, ch = item % kChan;
-            double v = 0;
-            if (D > 0) {
+        for (int q = 0; q < U; ++q) {
+            const int body = base + q * 6 + lane / 5;
+            double v0 = 0, v1 = 0;
 #pragma unroll
-                for (int k = 0; k < NK; ++k) v += b[k] * cf[u][k];
-            } else {
-                for (int k = 0; k <= d; ++k) v += b[k] * cf[u][k];
+            for (int k = 0; k < NK; ++k)
+                if (D > 0 || k <= d) {
+                    v0 += b[k] * cf[q][k].x;
+                    v1 += b[k] * cf[q][k].y;
+                }
+            if (!kRaw) {
+                // channels: p = 0 (x, y), 1 (z, vx), 2 (vy, vz), 3 (a_N x, y), 4 (a_N z, phi)
+                if (p == 1) v1 *= inv_c;
+                if (p == 2) { v0 *= inv_c; v1 *= inv_c; }
+                const double bx = __shfl_sync(0xffffffffu, v1, max(lane - 3, 0));                     // of lane p = 1
+                const double byz = __shfl_sync(0xffffffffu, v0 * v0 + v1 * v1, max(lane - 2, 0));   // of lane p = 2
+                if (p == 4) v1 += 2 * (bx * bx + byz);
             }
-            const int row = ch < 3 ? S_RX + ch : ch < 6 ? S_BX + (ch - 3) : ch < 9 ? S_NX + (ch - 6) : S_PHI;
-            PR[row * A.Mpad + body] = (ch >= 3 && ch < 6) ? v / kCS : v;
+            if (lane < 30 && body < M) {
+                PR[body * kSRec + 2 * p] = v0;
+                PR[body * kSRec + 2 * p + 1] = v1;
+            }
         }
     }
 }
-
-// all perturbers at time t into the shared rows (every thread of the CTA calls it)
-__device__ void eval_perturbers(const ServeArgs &A, double *PR, const double *cheb, double t) {
-    __syncthreads();   // the previous stage's readers are done
-    const double x = (t - A.t0) / A.knot;
-    long long xi = (long long)floor(x);
-    xi = xi < 0 ? 0 : (xi > A.n - 1 ? A.n - 1 : xi);
-    const double u = 2 * (x - (double)xi) - 1;
-    if (A.d == 3) eval_items<3>(A, PR, cheb, u, xi);
-    else eval_items<0>(A, PR, cheb, u, xi);
-    __syncthreads();
-    for (int j = threadIdx.x; j < A.M; j += blockDim.x) {
-        const double bx = PR[S_BX * A.Mpad + j], by = PR[S_BY * A.Mpad + j], bz = PR[S_BZ * A.Mpad + j];
-        PR[S_B2 * A.Mpad + j] = bx * bx + by * by + bz * bz;
-    }
-    __syncthreads();
+__device__ __forceinline__ void eval_perturbers(const ServeArgs &A, double *PR, const double *cheb, double t, int *take) {
+    if (A.d == 3) eval_rows<3, false>(A.coef, A.n, 3, A.M, A.t0, A.knot, PR, cheb, t, take);
+    else eval_rows<0, false>(A.coef, A.n, A.d, A.M, A.t0, A.knot, PR, cheb, t, take);
 }
 
-// acceleration of a particle; the G lanes of its group split the perturbers and all get the total
-__device__ v3 serve_accel(const ServeArgs &A, const double *PR, const dd r[3], const dd v[3], int lane, int G) {
-    const int Mp = A.Mpad;
-    const double c2 = kCS * kCS;
-    const v3 bi = vdiv(mk(dd_val(v[0]), dd_val(v[1]), dd_val(v[2])), kCS);
-    const double beta2 = dot(bi, bi);
-    double phi = 0;
+// Reduce-scatter of 8 values over the GT lanes of a group (GT = 16 or 32): value v is complete on lanes
+// v GT/8 .. (v + 1) GT/8 - 1 of the group. 9 shuffles (GT = 32) instead of 5 per value.
+template <int GT>
+__device__ __forceinline__ double group_scatter(double (&v)[8], int lane) {
+#pragma unroll
+    for (int h = 4, bit = GT / 2; h >= 1; h >>= 1, bit >>= 1) {
+        const bool up = (lane & bit) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const double send = up ? v[k] : v[k + h], keep = up ? v[k + h] : v[k];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+        }
+    }
+#pragma unroll
+    for (int bit = GT / 16; bit >= 1; bit >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
+    return v[0];
+}
+
+// Acceleration of a particle at (r, v): every lane of its group takes the perturbers j = lane, lane + G, ... and gets
+// component c0 (GT lanes known) or all three. mass.impl:82-97 regrouped as in the ensemble and particle kernels: the
+// coefficient 4 phi_i + beta_i^2 multiplies the Newtonian sum and is applied once, and with c = r.beta_j -
+// 4 r.(beta_j - beta_i) = 4 r.beta_i - 3 r.beta_j the last term is c beta_j, less beta_i times the sum of the c (57 FP64
+// operations a perturber, not 77). A function of its own, so that the loop has the registers to itself: inlined into
+// the request loop at 128 registers it took 430 cycles a perturber and warp, with 255 registers 240.
+template <int GT, bool kSoft>
+__device__ __noinline__ v3 serve_accel(const double *PR, const double *SR2, int M, double rx, double rxl, double ry, double ryl,
+                                       double rz, double rzl, v3 bi, int lane, int G, int c0) {
+    double phi = 0, cs = 0;
     v3 na = mk(0, 0, 0), ga = mk(0, 0, 0);
-#pragma unroll 1
-    for (int j = lane; j < A.M; j += G) {
-        const v3 d = mk(sep_diff(PR[S_RX * Mp + j], 0.0, r[0].hi, r[0].lo), sep_diff(PR[S_RY * Mp + j], 0.0, r[1].hi, r[1].lo),
-                        sep_diff(PR[S_RZ * Mp + j], 0.0, r[2].hi, r[2].lo));
-        const double q = dot(d, d), sm = PR[S_SR2 * Mp + j];
-        const double rr = rsqrt((q < sm) ? sm : q);
-        const double tp_dphi = rr * PR[S_GM * Mp + j];
-        const double tp_dg = rr * rr * tp_dphi;
+    const double *R = PR + lane * kSRec;
+#pragma unroll 2
+    for (int j = lane; j < M; j += G, R += G * kSRec) {
+        const v3 d = mk((R[S_R] - rx) - rxl, (R[S_R + 1] - ry) - ryl, (R[S_R + 2] - rz) - rzl);
+        double m = dot(d, d);
+        if (kSoft) {
+            const double sm = SR2[j];
+            m = (m < sm) ? sm : m;
+        }
+        const double rr = inv_sqrt(m);
+        const double tp_dphi = rr * R[S_GM];
+        const double tp_dg = (rr * rr) * tp_dphi;
         phi -= tp_dphi;
-        na += tp_dg * d;
-        const v3 bj = mk(PR[S_BX * Mp + j], PR[S_BY * Mp + j], PR[S_BZ * Mp + j]);
-        const double rbj = dot(d, bj);
+        na = mk(fma(tp_dg, d.x, na.x), fma(tp_dg, d.y, na.y), fma(tp_dg, d.z, na.z));
+        const v3 bj = mk(R[S_B], R[S_B + 1], R[S_B + 2]), nj = mk(R[S_N], R[S_N + 1], R[S_N + 2]);
+        const double rbj = dot(d, bj), rbi = dot(d, bi), rn = dot(d, nj), bb = dot(bi, bj);
         double tp = rbj * rr;
         tp *= tp;
-        const v3 naj = mk(PR[S_NX * Mp + j], PR[S_NY * Mp + j], PR[S_NZ * Mp + j]);
-        const double delta1 = PR[S_PHI * Mp + j] + beta2 + 2 * PR[S_B2 * Mp + j] - 4 * dot(bi, bj) +
-                              (dot(d, naj) - 3 * tp) / 2;
-        const v3 b = bj - bi;
-        ga += (7 * tp_dphi / 2) * naj + (tp_dg * delta1) * d + (tp_dg * (rbj - dot(d, b) * 4)) * b;
+        const double w = tp_dg * fma(-1.5, tp, fma(0.5, rn, fma(-4.0, bb, R[S_K])));
+        const double c = tp_dg * fma(4.0, rbi, -3.0 * rbj);
+        const double h = 3.5 * tp_dphi;
+        cs += c;
+        ga.x = fma(c, bj.x, fma(w, d.x, fma(h, nj.x, ga.x)));
+        ga.y = fma(c, bj.y, fma(w, d.y, fma(h, nj.y, ga.y)));
+        ga.z = fma(c, bj.z, fma(w, d.z, fma(h, nj.z, ga.z)));
     }
-    if (G > 1) {
-        phi = group_sum(phi, G);
-        na = mk(group_sum(na.x, G), group_sum(na.y, G), group_sum(na.z, G));
-        ga = mk(group_sum(ga.x, G), group_sum(ga.y, G), group_sum(ga.z, G));
+    ga = ga - cs * bi;
+    const double beta2 = dot(bi, bi), c2i = 1.0 / (kCS * kCS);
+    if (GT >= 16) {
+        constexpr int W = GT >= 16 ? GT : 32, per = W / 8;
+        double sums[8] = {phi, na.x, na.y, na.z, ga.x, ga.y, ga.z, 0.0};
+        const double x = group_scatter<W>(sums, lane);
+        const double p = __shfl_sync(0xffffffffu, x, 0, W), n = __shfl_sync(0xffffffffu, x, per * (1 + c0), W),
+                     g = __shfl_sync(0xffffffffu, x, per * (4 + c0), W);
+        return mk((g + (4 * (p * c2i) + beta2) * n) + n, 0.0, 0.0);
     }
-    phi = phi / c2;
-    ga += (4 * phi) * na;
-    na = vdiv(na, c2);
-    return ga + c2 * na;
+    phi = group_sum(phi, G) * c2i;
+    na = mk(group_sum(na.x, G), group_sum(na.y, G), group_sum(na.z, G));
+    ga = mk(group_sum(ga.x, G), group_sum(ga.y, G), group_sum(ga.z, G));
+    return (ga + (4 * phi + beta2) * na) + na;
 }
 
-// One RK12 step of size h from the state in Xin (shared rows [12][S]) at time t, stage accelerations in F
-// (f_0 given). kFull: write the end state (r, v) to Xout and return f at it; otherwise write only the end
-// position (dd, rows [6][S]) to Xout and skip the last acceleration. Xout may be Xin.
-template <bool kFull>
-__device__ __noinline__ v3 rk_step(const ServeArgs &A, double *PR, const double *cheb, const double *Xin, double *Xout, double *F,
-                      int S, int slot, int lane, bool live, double t, double h, v3 f0) {
-    const int G = A.G;
-    if (lane == 0) {
-        F[0] = f0.x; F[S] = f0.y; F[2 * S] = f0.z;
-    }
-    __syncwarp();
-    dd r[3], v[3];
-    v3 fa = f0;
-#pragma unroll 1
-    for (int k = 1; k <= kStages; ++k) {
-        const int row = k * (k - 1) / 2;
-        double s1[3] = {0.0, 0.0, 0.0}, s2[3] = {0.0, 0.0, 0.0};
-        if (k < kStages) {
-#pragma unroll 4
-            for (int l = 0; l < k; ++l) {
-                const double ab = q_abar[row + l], a = q_a[row + l];
-                const double *Fl = F + (size_t)l * 3 * S;
-                for (int c = 0; c < 3; ++c) {
-                    const double f = Fl[(size_t)c * S];
-                    s1[c] = __fma_rn(ab, f, s1[c]);
-                    s2[c] = __fma_rn(a, f, s2[c]);
-                }
-            }
-            const double ck = q_c[k];
-            for (int c = 0; c < 3; ++c) {
-                r[c] = dd_add(dd{Xin[c * S + slot], Xin[(3 + c) * S + slot]},
-                              dd_make(h * __fma_rn(ck, Xin[(6 + c) * S + slot], h * s1[c])));
-                v[c] = dd_add(dd{Xin[(6 + c) * S + slot], Xin[(9 + c) * S + slot]}, dd_make(h * s2[c]));
-            }
-        } else {
-#pragma unroll 1
-            for (int l = 0; l < k; ++l) {
-                const double ab = q_abar[row + l], a = q_a[row + l];
-                const double *Fl = F + (size_t)l * 3 * S;
-                for (int c = 0; c < 3; ++c) {
-                    const double f = Fl[(size_t)c * S];
-                    s1[c] = __fma_rn(ab, f, s1[c]);
-                    if (a != 0) s2[c] = __dadd_rn(s2[c], __dmul_rn(a, f));
-                }
-            }
-            const dd ck = dd_make(q_c[k]), dh = dd_make(h);
-            for (int c = 0; c < 3; ++c) {
-                const dd v0 = dd{Xin[(6 + c) * S + slot], Xin[(9 + c) * S + slot]};
-                const dd sv = dd_add(dd_mul(ck, v0), dd_make(h * s1[c]));
-                r[c] = dd_add(dd{Xin[c * S + slot], Xin[(3 + c) * S + slot]}, dd_mul(dh, sv));
-                v[c] = dd_add(v0, dd_make(h * s2[c]));
-            }
-            __syncwarp();   // every lane of the group has read Xin before lane 0 overwrites it
-            if (lane == 0) {
-                for (int c = 0; c < 3; ++c) {
-                    Xout[c * S + slot] = r[c].hi;
-                    Xout[(3 + c) * S + slot] = r[c].lo;
-                    if (kFull) {
-                        Xout[(6 + c) * S + slot] = v[c].hi;
-                        Xout[(9 + c) * S + slot] = v[c].lo;
-                    }
-                }
-            }
-            __syncwarp();
-            if (!kFull) return fa;
-        }
-        eval_perturbers(A, PR, cheb, t + q_c[k] * h);
-        const v3 fk = serve_accel(A, PR, r, v, lane, G);   // every lane: the group sums shuffle over full warps
-        if (live) fa = fk;
-        if (k < kStages && lane == 0) {
-            double *Fk = F + (size_t)k * 3 * S;
-            Fk[0] = fa.x; Fk[S] = fa.y; Fk[2 * S] = fa.z;
-        }
-        __syncwarp();
-    }
-    return fa;
-}
-
-__global__ void __launch_bounds__(kSThreads, 2) serve_kernel(ServeArgs A) {
+// One request. GT: lanes per particle when known (16 and 32, requests of less than about 4700 particles: each lane
+// then carries one component of the particle's state through the stage combination), 0 for any number.
+//
+// One attempt is one RK12 step of h from X0 (phase 0: its end position to RF) and two of h/2 (phase 1: X0 to X1,
+// phase 2: X1 to X1), in second-order form: r_k = r0 + h (c_k v0 + h sum_l Abar_kl f_l), v_k = v0 + h sum_l a_kl f_l with
+// the stage accelerations f_l in F; the same code serves every stage of the three.
+//
+// What bounds it: per stage, the dependent FP64 chains of serve_accel (13 perturbers a lane with 419 of them and a warp
+// per particle) and the spline coefficients, 134 KB from L2. So the perturbers of the next stage are formed beside
+// the present stage's sums into a second set of records, one CTA barrier a stage: four warps of a block do nothing
+// else, and a warp that has its sums, or no particle, takes chunks as well. One block of 384 threads an SM: the 168
+// registers a thread let two perturbers' chains overlap; at 128 registers, with two blocks of 256 an SM, a perturber
+// took 430 cycles a warp instead of 240. Requests alone, 360 days, against a body and channel per lane, the
+// perturbers before the sums and 128 registers: 5 particles 9.2 -> 3.7 ms, 300 (100 days) 10.4 -> 5.7, 4096 (60 days)
+// 20.9 -> 12.4; 100 requests at once 285 -> 219 ms (two blocks an SM: 216). 320 threads a block: 4.1, 6.4, 13.9, 243
+// ms; 512: 4.8, 6.6, 14.8, 255.
+template <int GT, bool kSoft>
+__global__ void __launch_bounds__(kSLaunch, 1) serve_kernel(ServeArgs A) {
     extern __shared__ __align__(16) double sm[];
     __shared__ double cheb[(EPH_BSPLINE_MAX_DEGREE + 1) * (EPH_BSPLINE_MAX_DEGREE + 1)];
-    __shared__ double red[kSThreads / 32];
-    const int G = A.G, S = blockDim.x / G;
-    const int slot = threadIdx.x / G, lane = threadIdx.x % G;
-    double *PR = sm;                          // [kSRows][Mpad]
-    double *X0 = PR + kSRows * A.Mpad;        // [12][S]
-    double *X1 = X0 + 12 * S;                 // [12][S]
-    double *RF = X1 + 12 * S;                 // [6][S]
+    __shared__ double red[kSLaunch / 32];
+    __shared__ double2 ab[EPH_RK12_NCOEF];
+    __shared__ int li[EPH_RK12_NCOEF];
+    __shared__ unsigned long long s_t0;
+    __shared__ int s_late, s_take[2];
+    constexpr bool kSplit = GT >= 16;
+    constexpr int NC = kSplit ? 1 : 3;             // components per lane in the stage combination
+    const int G = GT > 0 ? GT : A.G, S = A.S;
+    const bool worker = (int)threadIdx.x < S * G;   // (whole warps)
+    const int slot = worker ? threadIdx.x / G : 0, lane = threadIdx.x % G;
+    const int c0 = kSplit ? lane % 3 : 0;          // this lane's (first) component
+    const int set = A.M * kSRec;                   // doubles of one set of records
+    double *rows = sm;                             // [buffers][M][kSRec], then sR2 [M] if any
+    double *SR2 = rows + A.buffers * set;
+    double *X0 = SR2 + (kSoft ? A.M : 0);          // [12][S]
+    double *X1 = X0 + 12 * S;                      // [12][S]
+    double *RF = X1 + 12 * S;                      // [6][S]
     // stage store [kStages][3][S]: shared memory for blocks of up to kSmemSlots particles, else global
     double *F = (S <= kSmemSlots ? RF + 6 * S : A.fstore + (size_t)blockIdx.x * kStages * 3 * S) + slot;
     const int ip = blockIdx.x * S + slot;
-    const bool live = ip < A.P;
+    const bool live = worker && ip < A.P;
     for (int q = threadIdx.x; q < (A.d + 1) * (A.d + 1); q += blockDim.x) cheb[q] = A.cheb[q];
-    for (int j = threadIdx.x; j < A.M; j += blockDim.x) {
-        PR[S_GM * A.Mpad + j] = A.gm[j];
-        PR[S_SR2 * A.Mpad + j] = A.sr2[j];
+    for (int q = threadIdx.x; q < EPH_RK12_NCOEF; q += blockDim.x) {
+        ab[q] = q_ab[q];
+        li[q] = q_l[q] * 3 * S;
     }
-    if (lane == 0)
-        for (int q = 0; q < 12; ++q) X0[q * S + slot] = live ? A.state[(size_t)q * A.P + ip] : (q < 3 ? 1e30 : 0.0);
+    for (int j = threadIdx.x; j < A.M; j += blockDim.x) {
+        for (int b = 0; b < A.buffers; ++b) rows[b * set + j * kSRec + S_GM] = A.gm[j];
+        if (kSoft) SR2[j] = A.sr2[j];
+    }
+    if (worker)
+        for (int q = lane; q < 12; q += G) X0[q * S + slot] = live ? A.state[(size_t)q * A.P + ip] : (q < 3 ? 1e30 : 0.0);
+    if (threadIdx.x == 0) {
+        s_t0 = now_ns();
+        s_take[0] = s_take[1] = 0;
+    }
     __syncthreads();
+    int cur = 0;               // rows of the present stage
+    // Acceleration of the particle at (r, v) with the perturbers of the rows in use, this lane's component(s) to fa;
+    // forms those at time t_next (if `more`) into the other rows.
+    auto stage = [&](const dd r[3], v3 v, double t_now, bool fresh, double t_next, bool more, double (&fa)[NC]) {
+        double *now = rows + cur * set;
+        if (fresh || A.buffers == 1) {   // nothing prepared: form them now
+            __syncthreads();
+            eval_perturbers(A, now, cheb, t_now, &s_take[cur]);
+        }
+        __syncthreads();   // the rows are complete, and no warp still reads the others
+        if (threadIdx.x == 0) s_take[cur] = 0;
+        const int to = cur ^ 1;
+        double *next = rows + to * set;
+        const bool ahead = more && A.buffers == 2;
+        if (ahead) cur = to;
+        if (!worker) {
+            if (ahead) eval_perturbers(A, next, cheb, t_next, &s_take[to]);
+            return;
+        }
+        const v3 bi = mk(v.x * (1.0 / kCS), v.y * (1.0 / kCS), v.z * (1.0 / kCS));
+        const v3 f = serve_accel<GT, kSoft>(now, SR2, A.M, r[0].hi, r[0].lo, r[1].hi, r[1].lo, r[2].hi, r[2].lo, bi, lane, G, c0);
+        const double fc[3] = {f.x, f.y, f.z};
+#pragma unroll
+        for (int ci = 0; ci < NC; ++ci) fa[ci] = live ? fc[ci] : 0.0;
+        if (ahead) eval_perturbers(A, next, cheb, t_next, &s_take[to]);
+    };
     const double dir = A.t_end >= A.t_start ? 1.0 : -1.0;
     double t = A.t_start;
-    // f at the start state
-    eval_perturbers(A, PR, cheb, t);
-    v3 f0 = mk(0, 0, 0);
+    double f0[NC] = {}, fm[NC] = {}, fe[NC] = {};   // f at the start, the middle and the end of the attempt
     {
-        dd r[3], v[3];
-        for (int c = 0; c < 3; ++c) {
-            r[c] = dd{X0[c * S + slot], X0[(3 + c) * S + slot]};
-            v[c] = dd{X0[(6 + c) * S + slot], X0[(9 + c) * S + slot]};
-        }
-        const v3 fs = serve_accel(A, PR, r, v, lane, G);
-        if (live) f0 = fs;
+        dd r[3];
+        for (int c = 0; c < 3; ++c) r[c] = dd{X0[c * S + slot], X0[(3 + c) * S + slot]};
+        const v3 v = mk(dd_val(dd{X0[6 * S + slot], X0[9 * S + slot]}), dd_val(dd{X0[7 * S + slot], X0[10 * S + slot]}),
+                        dd_val(dd{X0[8 * S + slot], X0[11 * S + slot]}));
+        stage(r, v, t, true, t, false, f0);
     }
     double h = fabs(A.h0);
     bool just_rejected = false;
     long long accepted = 0, rejected = 0;
     int status = SS_OK;
-    __shared__ unsigned long long s_t0;
-    __shared__ int s_late;
-    if (threadIdx.x == 0) s_t0 = now_ns();
-    __syncthreads();
 #pragma unroll 1
     for (long long attempt = 0; dir * (A.t_end - t) > 0; ++attempt) {
         if (attempt >= kMaxAttempts) { status = SS_ATTEMPTS; break; }
@@ -346,17 +367,142 @@ __global__ void __launch_bounds__(kSThreads, 2) serve_kernel(ServeArgs A) {
         const double remaining = dir * (A.t_end - t);
         const bool last = h >= remaining;
         const double hs = dir * (last ? remaining : h);
-        rk_step<false>(A, PR, cheb, X0, RF, F, S, slot, lane, live, t, hs, f0);
-        const v3 fm = rk_step<true>(A, PR, cheb, X0, X1, F, S, slot, lane, live, t, hs / 2, f0);
-        const v3 fe = rk_step<true>(A, PR, cheb, X1, X1, F, S, slot, lane, live, t + hs / 2, hs / 2, fm);
+        bool fresh = true;
+        int phase = 0, k = 1;
+#pragma unroll 1
+        for (;;) {
+            const double hp = phase == 0 ? hs : hs / 2, tp = phase == 2 ? t + hs / 2 : t;
+            const double *Xin = (phase == 2 ? X1 : X0) + slot;
+            double rh[NC] = {}, rl[NC] = {}, vv[NC] = {};
+            if (worker) {
+            if (k == 1) {
+#pragma unroll
+                for (int ci = 0; ci < NC; ++ci)
+                    if (lane < 3 || !kSplit) {
+                        if (kSplit || lane == 0) F[(c0 + ci) * S] = phase == 2 ? fm[ci] : f0[ci];
+                    }
+                __syncwarp();
+            }
+            double s1[NC], s2[NC];
+#pragma unroll
+            for (int ci = 0; ci < NC; ++ci) s1[ci] = s2[ci] = 0.0;
+            const int q1 = q_row[k + 1];
+            if (k < kStages) {
+#pragma unroll 4
+                for (int q = q_row[k]; q < q1; ++q) {
+                    const double2 a = ab[q];
+#pragma unroll
+                    for (int ci = 0; ci < NC; ++ci) {
+                        const double f = F[li[q] + (c0 + ci) * S];
+                        s1[ci] = __fma_rn(a.x, f, s1[ci]);
+                        s2[ci] = __fma_rn(a.y, f, s2[ci]);
+                    }
+                }
+                const double ck = q_c[k];
+#pragma unroll
+                for (int ci = 0; ci < NC; ++ci) {
+                    const int c = c0 + ci;
+                    const double v0 = Xin[(6 + c) * S];
+                    double e;
+                    two_sum(Xin[c * S], hp * __fma_rn(ck, v0, hp * s1[ci]), rh[ci], e);
+                    rl[ci] = e + Xin[(3 + c) * S];
+                    vv[ci] = v0 + __fma_rn(hp, s2[ci], Xin[(9 + c) * S]);
+                }
+            } else {
+#pragma unroll 1
+                for (int q = q_row[k]; q < q1; ++q) {
+                    const double2 a = ab[q];
+#pragma unroll
+                    for (int ci = 0; ci < NC; ++ci) {
+                        const double f = F[li[q] + (c0 + ci) * S];
+                        s1[ci] = __fma_rn(a.x, f, s1[ci]);
+                        if (a.y != 0) s2[ci] = __dadd_rn(s2[ci], __dmul_rn(a.y, f));
+                    }
+                }
+                const dd ck = dd_make(q_c[k]), dh = dd_make(hp);
+                dd rn[NC], vn[NC];
+#pragma unroll
+                for (int ci = 0; ci < NC; ++ci) {
+                    const int c = c0 + ci;
+                    const dd v0 = dd{Xin[(6 + c) * S], Xin[(9 + c) * S]};
+                    const dd sv = dd_add(dd_mul(ck, v0), dd_make(hp * s1[ci]));
+                    rn[ci] = dd_add(dd{Xin[c * S], Xin[(3 + c) * S]}, dd_mul(dh, sv));
+                    vn[ci] = dd_add(v0, dd_make(hp * s2[ci]));
+                    rh[ci] = rn[ci].hi;
+                    rl[ci] = rn[ci].lo;
+                    vv[ci] = dd_val(vn[ci]);
+                }
+                __syncwarp();   // every lane of the group has read Xin before it is overwritten
+                double *Xout = (phase == 0 ? RF : X1) + slot;
+#pragma unroll
+                for (int ci = 0; ci < NC; ++ci) {
+                    const int c = c0 + ci;
+                    if (kSplit ? lane < 3 : lane == 0) {
+                        Xout[c * S] = rn[ci].hi;
+                        Xout[(3 + c) * S] = rn[ci].lo;
+                        if (phase > 0) {
+                            Xout[(6 + c) * S] = vn[ci].hi;
+                            Xout[(9 + c) * S] = vn[ci].lo;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            }
+            if (k == kStages && phase == 0) {   // the whole step's end needs no acceleration
+                phase = 1;
+                k = 1;
+                continue;
+            }
+            dd r[3];
+            v3 v;
+            if (kSplit) {
+                constexpr int W = kSplit ? GT : 32;
+                double vc[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    r[c] = dd{__shfl_sync(0xffffffffu, rh[0], c, W), __shfl_sync(0xffffffffu, rl[0], c, W)};
+                    vc[c] = __shfl_sync(0xffffffffu, vv[0], c, W);
+                }
+                v = mk(vc[0], vc[1], vc[2]);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) r[c] = dd{rh[c % NC], rl[c % NC]};
+                v = mk(vv[0], vv[1 % NC], vv[2 % NC]);
+            }
+            // the next stage that needs the perturbers, and its time
+            int np = phase, nk = k + 1;
+            if (nk > kStages || (np == 0 && nk == kStages)) { ++np; nk = 1; }
+            const double nh = np == 0 ? hs : hs / 2, nt = (np == 2 ? t + hs / 2 : t) + q_c[nk] * nh;
+            double fa[NC] = {};
+            stage(r, v, tp + q_c[k] * hp, fresh, nt, np <= 2, fa);
+            fresh = false;
+            if (k < kStages) {
+#pragma unroll
+                for (int ci = 0; ci < NC; ++ci)
+                    if (worker && (kSplit ? lane < 3 : lane == 0)) F[(k * 3 + c0 + ci) * S] = fa[ci];
+                __syncwarp();
+                ++k;
+                continue;
+            }
+#pragma unroll
+            for (int ci = 0; ci < NC; ++ci) {
+                if (phase == 1) fm[ci] = fa[ci];
+                else fe[ci] = fa[ci];
+            }
+            if (phase == 2) break;
+            phase = 2;
+            k = 1;
+        }
         // error of the particle: |r_h - r_h/2| / |r_h/2 - r_star(t + h)| (the last stage evaluated the
         // ephemeris at t + h)
+        const double *PR = rows + cur * set;
         double e = 0;
         if (live && lane == 0) {
             double num = 0, den = 0;
             for (int c = 0; c < 3; ++c) {
                 const double dr = (X1[c * S + slot] - RF[c * S + slot]) + (X1[(3 + c) * S + slot] - RF[(3 + c) * S + slot]);
-                const double rs = (X1[c * S + slot] - PR[(S_RX + c) * A.Mpad]) + X1[(3 + c) * S + slot];
+                const double rs = (X1[c * S + slot] - PR[S_R + c]) + X1[(3 + c) * S + slot];
                 num += dr * dr;
                 den += rs * rs;
             }
@@ -377,10 +523,11 @@ __global__ void __launch_bounds__(kSThreads, 2) serve_kernel(ServeArgs A) {
         }
         const double hused = fabs(hs);
         if (err <= A.tol) {   // accept the two half steps
-            if (lane == 0)
-                for (int q = 0; q < 12; ++q) X0[q * S + slot] = X1[q * S + slot];
+            if (worker)
+                for (int q = lane; q < 12; q += G) X0[q * S + slot] = X1[q * S + slot];
             if (A.hlog && blockIdx.x == 0 && threadIdx.x == 0 && accepted < A.hlog_cap) A.hlog[accepted] = hs;
-            f0 = fe;
+#pragma unroll
+            for (int ci = 0; ci < NC; ++ci) f0[ci] = fe[ci];
             t = last ? A.t_end : t + hs;
             ++accepted;
         } else {
@@ -397,8 +544,8 @@ __global__ void __launch_bounds__(kSThreads, 2) serve_kernel(ServeArgs A) {
         __syncwarp();
     }
     __syncthreads();
-    if (live && lane == 0)
-        for (int q = 0; q < 12; ++q) A.state[(size_t)q * A.P + ip] = X0[q * S + slot];
+    if (live)
+        for (int q = lane; q < 12; q += G) A.state[(size_t)q * A.P + ip] = X0[q * S + slot];
     if (threadIdx.x == 0) {
         A.stats[2 * blockIdx.x] = accepted;
         A.stats[2 * blockIdx.x + 1] = rejected;
@@ -411,13 +558,13 @@ __global__ void __launch_bounds__(kSThreads) eval_kernel(ServeArgs A, double t, 
     extern __shared__ __align__(16) double sm[];
     __shared__ double cheb[(EPH_BSPLINE_MAX_DEGREE + 1) * (EPH_BSPLINE_MAX_DEGREE + 1)];
     for (int q = threadIdx.x; q < (A.d + 1) * (A.d + 1); q += blockDim.x) cheb[q] = A.cheb[q];
-    eval_perturbers(A, sm, cheb, t);
-    for (int item = threadIdx.x; item < A.M * kChan; item += blockDim.x) {
-        const int body = item / kChan, ch = item % kChan;
-        const int row = ch < 3 ? S_RX + ch : ch < 6 ? S_BX + (ch - 3) : ch < 9 ? S_NX + (ch - 6) : S_PHI;
-        const double v = sm[row * A.Mpad + body];
-        out[item] = (ch >= 3 && ch < 6) ? v * kCS : v;
-    }
+    __shared__ int take;
+    if (threadIdx.x == 0) take = 0;
+    __syncthreads();
+    if (A.d == 3) eval_rows<3, true>(A.coef, A.n, 3, A.M, A.t0, A.knot, sm, cheb, t, &take);
+    else eval_rows<0, true>(A.coef, A.n, A.d, A.M, A.t0, A.knot, sm, cheb, t, &take);
+    __syncthreads();
+    for (int item = threadIdx.x; item < A.M * kChan; item += blockDim.x) out[item] = sm[item / kChan * kSRec + item % kChan];
 }
 
 // step-end stage records of sampled steps into [samples][M][kChan]
@@ -488,33 +635,54 @@ __global__ void bspline_solve_kernel(int d, long long m, int J, int channels, lo
     }
 }
 
+using ServeKernel = void (*)(ServeArgs);
+ServeKernel serve_kernel_of(int G, bool soft) {
+    if (G == 32) return soft ? serve_kernel<32, true> : serve_kernel<32, false>;
+    if (G == 16) return soft ? serve_kernel<16, true> : serve_kernel<16, false>;
+    return soft ? serve_kernel<0, true> : serve_kernel<0, false>;
+}
+constexpr size_t kServeSmem = 216 * 1024;       // most dynamic shared memory of a block
+
 bool g_serve_ready[64];
 cudaError_t serve_setup(int device) {
     if (device >= 0 && device < 64 && g_serve_ready[device]) return cudaSuccess;
     double hi[EPH_RK12_NCOEF], lo[EPH_RK12_NCOEF], dtk[kStages + 1];
     rk12_expand(hi, lo, dtk);
-    double a[EPH_RK12_NCOEF], abar[EPH_RK12_NCOEF] = {0};
-    for (int q = 0; q < EPH_RK12_NCOEF; ++q) a[q] = hi[q] + lo[q];
-    for (int k = 1; k <= kStages; ++k)
-        for (int l = 0; l < k; ++l) {   // Abar = A A (second-order form), long double accumulation
+    auto coef = [&](int k, int j) { return (long double)hi[k * (k - 1) / 2 + j] + lo[k * (k - 1) / 2 + j]; };
+    double2 tab[EPH_RK12_NCOEF] = {};
+    int ll[EPH_RK12_NCOEF] = {}, row[kStages + 2] = {}, q = 0;
+    for (int k = 1; k <= kStages; ++k) {   // Abar = A A (second-order form), long double accumulation
+        row[k] = q;
+        for (int l = 0; l < k; ++l) {
             long double acc = 0;
-            for (int j = l + 1; j < k; ++j)
-                acc += ((long double)hi[k * (k - 1) / 2 + j] + lo[k * (k - 1) / 2 + j]) *
-                       ((long double)hi[j * (j - 1) / 2 + l] + lo[j * (j - 1) / 2 + l]);
-            abar[k * (k - 1) / 2 + l] = (double)acc;
+            bool any = hi[k * (k - 1) / 2 + l] != 0;
+            for (int j = l + 1; j < k; ++j) {
+                acc += coef(k, j) * coef(j, l);
+                any = any || (hi[k * (k - 1) / 2 + j] != 0 && hi[j * (j - 1) / 2 + l] != 0);
+            }
+            if (!any) continue;
+            tab[q] = make_double2((double)acc, hi[k * (k - 1) / 2 + l] + lo[k * (k - 1) / 2 + l]);
+            ll[q++] = l;
         }
-    cudaError_t e = cudaMemcpyToSymbol(q_a, a, sizeof(a));
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(q_abar, abar, sizeof(abar));
+    }
+    row[kStages + 1] = q;
+    cudaError_t e = cudaMemcpyToSymbol(q_ab, tab, sizeof(tab));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(q_l, ll, sizeof(ll));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(q_row, row, sizeof(row));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(q_c, dtk, sizeof(dtk));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(serve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    for (int G : {0, 16, 32})
+        for (int soft = 0; soft < 2 && e == cudaSuccess; ++soft)
+            e = cudaFuncSetAttribute(serve_kernel_of(G, soft), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kServeSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (e == cudaSuccess && device >= 0 && device < 64) g_serve_ready[device] = true;
     return e;
 }
 
-size_t serve_smem(int Mpad, int S) {
-    return (size_t)(kSRows * Mpad + 30 * S + (S <= kSmemSlots ? kStages * 3 * S : 0)) * sizeof(double);
+size_t serve_smem(int M, int S, int buffers, bool soft) {
+    return (size_t)((buffers * kSRec + (soft ? 1 : 0)) * M + 30 * S + (S <= kSmemSlots ? kStages * 3 * S : 0)) * sizeof(double);
 }
+// Sets of perturber records: two, where the second fits
+int serve_buffers(int M, int S, bool soft) { return serve_smem(M, S, 2, soft) <= kServeSmem ? 2 : 1; }
 
 }  // namespace
 }  // namespace eph
@@ -528,7 +696,8 @@ struct eph_serve {
     cudaStream_t streams[kSStreams] = {};
     int next_stream = 0;
     int sms = 148;
-    int M = 0, Mpad = 0, d = 0;
+    int M = 0, d = 0;
+    bool soft = false;                 // any sR2 is not zero
     long long n = 0;
     double t0 = 0, knot = 0;
     double *d_coef = nullptr, *d_gm = nullptr, *d_sr2 = nullptr, *d_cheb = nullptr;
@@ -608,12 +777,16 @@ static int pump(eph_serve *s) {
         }
         ServeArgs A;
         A.coef = s->d_coef; A.gm = s->d_gm; A.sr2 = s->d_sr2; A.cheb = s->d_cheb;
-        A.M = s->M; A.Mpad = s->Mpad; A.d = s->d; A.n = s->n; A.t0 = s->t0; A.knot = s->knot;
+        A.M = s->M; A.d = s->d; A.n = s->n; A.t0 = s->t0; A.knot = s->knot;
         A.state = r.d_state; A.fstore = r.d_fstore; A.P = r.P; A.G = r.G;
         A.t_start = r.t_start; A.t_end = r.t_end; A.tol = r.tol; A.h0 = r.h0;
         A.hmin = std::max(1e-9 * std::fabs(r.t_end - r.t_start), 1e-3);
         A.stats = r.d_stats; A.status = r.d_status; A.hlog = r.d_hlog; A.hlog_cap = (int)r.log_cap;
-        serve_kernel<<<r.grid, r.block, serve_smem(s->Mpad, S), st>>>(A);
+        A.S = S;
+        A.soft = s->soft;
+        A.buffers = serve_buffers(s->M, S, s->soft);
+        // a full block's warps whatever the particles: the warps without any evaluate perturbers
+        serve_kernel_of(r.G, s->soft)<<<r.grid, kSLaunch, serve_smem(s->M, S, A.buffers, s->soft), st>>>(A);
         SCK(cudaGetLastError(), "launch serve kernel");
         SCK(cudaEventRecord(r.done, st), "record event");
         r.launched = true;
@@ -640,11 +813,11 @@ int eph_serve_create(int device, int64_t n_pert, const double *gm, const double 
     eph_serve *s = new eph_serve();
     s->device = device;
     s->M = (int)n_pert;
-    s->Mpad = (int)((n_pert + 1) / 2 * 2);
     s->d = degree;
     s->n = n_intervals;
     s->t0 = t0;
     s->knot = knot;
+    for (int64_t j = 0; sr2 && j < n_pert; ++j) s->soft = s->soft || sr2[j] != 0;
     auto bail = [&](int code, const char *what, cudaError_t e) {
         sfail(s, code, what, e);
         eph_serve_destroy(s);
@@ -820,8 +993,8 @@ int eph_serve_eval(eph_serve *s, double t, double *out) {
     SCK(cudaMallocAsync((void **)&d_out, (size_t)s->M * kChan * sizeof(double), st), "cudaMallocAsync(eval)");
     ServeArgs A{};
     A.coef = s->d_coef; A.gm = s->d_gm; A.sr2 = s->d_sr2; A.cheb = s->d_cheb;
-    A.M = s->M; A.Mpad = s->Mpad; A.d = s->d; A.n = s->n; A.t0 = s->t0; A.knot = s->knot;
-    eval_kernel<<<1, kSThreads, (size_t)kSRows * s->Mpad * sizeof(double), st>>>(A, t, d_out);
+    A.M = s->M; A.d = s->d; A.n = s->n; A.t0 = s->t0; A.knot = s->knot;
+    eval_kernel<<<1, kSThreads, (size_t)kSRec * s->M * sizeof(double), st>>>(A, t, d_out);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, (size_t)s->M * kChan * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(d_out, st);

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -67,6 +68,8 @@ struct BatchSys {
     long long n_step;     // steps (>= 1)
     double dt;            // signed step
     double t_eph;         // double(t_eph) at the start
+    int accumulate;       // eph_rk12: the maxima go on from the planes' and min_distance is not inverted
+    int whole;            // also write what stays constant for such bodies (harmonics, moments of inertia, J2 change)
     double *planes;       // [EPH_NPLANES][n], in and out
     double *store;        // [kStore][n] stage accelerations and start-of-step state, when shared memory has no room
 };
@@ -584,10 +587,32 @@ __device__ void integrate_system(const BatchSys &Y, const RkTable &rk, double *s
         PLV(EPH_P_PHI, i) = c2 * rec[RB_PHI];
         const v3 be = mk(rec[RB_BETA], rec[RB_BETA + 1], rec[RB_BETA + 2]);
         PLV(EPH_P_BETA2, i) = dot(be, be);
-        PLV(EPH_P_MIN_DISTANCE, i) = 1 / sqrt(1.0 / own_row(V, OR_M, b));   // no pair seen: 1 / 0
-        PLV(EPH_P_MAX_INFLUENCE, i) = own_row(V, OR_MAXI, b);
+        double mind = sqrt(1.0 / own_row(V, OR_M, b)), maxi = own_row(V, OR_MAXI, b);   // (no pair seen: 0)
+        if (Y.accumulate) {
+            const double mind0 = PLV(EPH_P_MIN_DISTANCE, i), maxi0 = PLV(EPH_P_MAX_INFLUENCE, i);
+            checked_maximize(mind, mind0);
+            checked_maximize(maxi, maxi0);
+        }
+        PLV(EPH_P_MIN_DISTANCE, i) = Y.accumulate ? mind : 1 / mind;
+        PLV(EPH_P_MAX_INFLUENCE, i) = maxi;
+        if (Y.whole) {   // UPDATE_HARMONICS (mass.impl:48-64) of a body without tide, spin and static harmonics
+            const double gi = ((-2.0) / 3 * PLV(EPH_P_R2, i)) * -PLV(EPH_P_A, i);
+            for (int q = 0; q < 9; ++q) {
+                PLV(EPH_P_C_POTENTIAL + q, i) = 0.0;
+                PLV(EPH_P_GI + q, i) = q % 4 == 0 ? gi : 0.0;
+            }
+            PLV(EPH_P_EXJ2, i) = 0.0;
+        }
     }
 #undef PLV
+    __syncthreads();
+}
+
+__device__ __forceinline__ void load_table(RkTable &rk) {
+    for (int q = threadIdx.x; q < EPH_RK12_NCOEF; q += blockDim.x) {
+        rk.ab[q] = make_double2(b_ab_hi[q], b_a[q]);
+        rk.lo[q] = b_ab_lo[q];
+    }
     __syncthreads();
 }
 
@@ -627,6 +652,15 @@ __global__ void __launch_bounds__(kBThreads, 2)
 }
 
 constexpr size_t kBMaxSmem = 227 * 1024 - sizeof(RkTable) - 256;
+// One system on the CTAs of one cluster.
+__global__ void __launch_bounds__(kBThreads, 2) point_kernel(BatchSys Y, int peers) {
+    extern __shared__ __align__(16) double bsm[];
+    __shared__ RkTable rk;
+    load_table(rk);
+    integrate_system<false>(Y, rk, bsm, peers, peers > 1 ? (int)cg::this_cluster().block_rank() : 0);
+    if (peers > 1) cg::this_cluster().sync();   // no CTA leaves while a peer may still store to it
+}
+
 // ---- how many CTAs share a system
 constexpr int kShares = 5;
 constexpr int kSharePeers[kShares] = {16, 8, 4, 2, 1};
@@ -669,9 +703,12 @@ size_t system_smem(int n, int peers, int split, bool mixed) {
 }
 constexpr int kMaxBodies = 768;   // bodies of a system of the ensemble launch: shared memory holds it on one CTA
 
-bool g_batch_ready[64];
+std::atomic<bool> g_batch_ready[64];
+std::mutex g_batch_mu;   // contexts and batches may set a device up at the same time
 cudaError_t batch_setup(int device) {
-    if (device >= 0 && device < 64 && g_batch_ready[device]) return cudaSuccess;
+    if (device >= 0 && device < 64 && g_batch_ready[device].load(std::memory_order_acquire)) return cudaSuccess;
+    std::lock_guard<std::mutex> lock(g_batch_mu);
+    if (device >= 0 && device < 64 && g_batch_ready[device].load(std::memory_order_relaxed)) return cudaSuccess;
     double hi[EPH_RK12_NCOEF], lo[EPH_RK12_NCOEF], dtk[kStages + 1];
     rk12_expand(hi, lo, dtk);
     double ab_hi[EPH_RK12_NCOEF] = {0}, ab_lo[EPH_RK12_NCOEF] = {0}, aa[EPH_RK12_NCOEF] = {0};
@@ -703,11 +740,53 @@ cudaError_t batch_setup(int device) {
     // clusters of 16 CTAs: twice the portable size
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ensemble_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ensemble_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess && device >= 0 && device < 64) g_batch_ready[device] = true;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(point_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(point_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBMaxSmem);
+    if (e == cudaSuccess && device >= 0 && device < 64) g_batch_ready[device].store(true, std::memory_order_release);
     return e;
 }
 
 }  // namespace
+
+// ---- a single point-mass system (eph_capi.cu)
+// Scratch a context keeps for it (doubles).
+size_t point_scratch_doubles(int n) { return (size_t)kStore * n; }
+// Launches n_step steps of dt of a system of point-like bodies on `stream`, as the step kernel of eph_step.cu would
+// integrate it (accumulate: eph_rk12's maxima, else eph_integrate's).
+cudaError_t launch_point_system(int device, cudaStream_t stream, double *planes, int n, double dt, long long n_step, double t_eph,
+                                int accumulate, double *scratch) {
+    cudaError_t e = batch_setup(device);
+    if (e != cudaSuccess) return e;
+    BatchSys Y{};
+    Y.n = n;
+    Y.split = batch_split(n);
+    Y.n_step = n_step;
+    Y.dt = dt;
+    Y.t_eph = t_eph;
+    Y.accumulate = accumulate;
+    Y.whole = 1;
+    Y.planes = planes;
+    Y.store = scratch;
+    int peers = 0;   // the CTA count with the shortest stage
+    float best = 1e30f;
+    for (int p : kSharePeers) {
+        if ((p > 1 && n < kMinOwn * p) || !share_fits(n, p, Y.split) || system_smem(n, p, Y.split, false) > kBMaxSmem) continue;
+        const float t = stage_us(n, p, Y.split);
+        if (t < best) { best = t; peers = p; }
+    }
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = peers;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(peers);
+    cfg.blockDim = dim3(kBThreads);
+    cfg.dynamicSmemBytes = system_smem(n, peers, Y.split, false);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, point_kernel, Y, peers);
+}
 }  // namespace eph
 
 using namespace eph;
@@ -887,6 +966,7 @@ int eph_batch_integrate(eph_batch *b, const double *dt, const int64_t *n_step, d
         const int n = (int)b->n_body[s];
         Y.n = n;
         Y.split = b->split[s];
+        Y.accumulate = Y.whole = 0;
         // msystem::integrate: a negative step count integrates backwards (mass.cpp:401-404)
         Y.n_step = n_step[s] < 0 ? -n_step[s] : n_step[s];
         Y.dt = n_step[s] < 0 ? -dt[s] : dt[s];

@@ -33,6 +33,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -129,6 +130,22 @@ constexpr int kMaxSmem = 227 * 1024 - 4096;   // the 227 KB per-CTA maximum less
 constexpr size_t kFixedSmem = ((sizeof(Own) * kOwnMax + sizeof(Scratch) + 127) / 128) * 128;
 constexpr int kTileW = (int)((kMaxSmem - kFixedSmem) / (kTileRows * sizeof(double))) / kPad * kPad;
 static_assert(kTileW >= 512, "the staging tile must hold a 512-body system in one piece");
+// Pass A reads half as many rows as the tile has: a system of up to twice the tile's width is staged whole for its
+// sweeps, at twice the row stride, instead of in chunks that every iteration of the angular-velocity fixed point
+// copies again. Rows 6 to 11, the velocities, are free in a CTA without a delayed tide: its field items run beside
+// its sweeps there, and it takes those of the CTAs with one, as in a system of one tile. 1,001 bodies, full physics:
+// 60 -> 52 us per stage.
+constexpr int kWideW = 2 * kTileW;
+static_assert(TA_ROWS * kWideW <= kTileRows * kTileW && TA_V_HI == 6 && TA_V_LO + 3 == TA_GM, "pass-A rows at the wide stride");
+constexpr int kWideFree = (TA_GM - TA_V_HI) * kWideW;   // doubles of the free rows
+// How the bodies are staged, by the system's size. The kernel is compiled once for each: with the layout known the
+// strides and loop bounds are constants, and the code that the stage loop runs through (which a small system does
+// not stay long enough in to keep in the instruction cache) is shorter. 48 / 504 bodies, full physics: 26 -> 22 and
+// 30 -> 27 us per stage.
+enum Layout { kOneTile, kWideA, kChunks };   // one tile; pass A whole at the wide stride, pass B in chunks; chunks
+static Layout layout_of(int n, int tile) {   // a tile below the stride was asked for: chunks of that size
+    return n <= tile ? kOneTile : tile == kTileW && n <= kWideW ? kWideA : kChunks;
+}
 
 // ------------------------------------------------------------------ small helpers
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
@@ -563,8 +580,8 @@ __device__ void publish_body_warp(const SysDev &S, const Own &o, int buf, int la
 // ------------------------------------------------------------------ pass A: deform_by + angular velocity
 // One ordered pair (i = owned body o, j from the tile) of DAMPED_TIDAL_DEFORMATION_MATRIX / _NDELAY /
 // _NK2 (mass.impl:1-46), accumulated into acc = {phi, naccel[3], C[9]}.
+template <int ts>
 __device__ __forceinline__ void pair_a(const Own &o, const double *T, int j, double acc[13]) {
-    constexpr int ts = kTileW;
     v3 r = mk(sep_diff(T[(TA_R_HI + 0) * ts + j], T[(TA_R_LO + 0) * ts + j], o.r[0].hi, o.r[0].lo),
               sep_diff(T[(TA_R_HI + 1) * ts + j], T[(TA_R_LO + 1) * ts + j], o.r[1].hi, o.r[1].lo),
               sep_diff(T[(TA_R_HI + 2) * ts + j], T[(TA_R_LO + 2) * ts + j], o.r[2].hi, o.r[2].lo));
@@ -677,11 +694,12 @@ __device__ __forceinline__ void tile_a_rows(const SysDev &S, const double *pub, 
 }
 
 // Pair sums of pass A for the owned bodies in `mask` over all bodies j, by the first `nw` warps (tile
-// already staged when the whole system fits in one tile; otherwise tiles are streamed, which needs the
+// already staged (one tile, or whole at the wide stride); otherwise tiles are streamed, which needs the
 // whole CTA, nw == kWarps). Results land in own[b].sumA. One pair per iteration: a second pair chain in
 // flight per thread spills registers at the kernel's 128 per thread.
+template <Layout kL>
 __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int buf, Scratch &sc, TileState &ts,
-                        double *tile, bool staged, int nw, const int *first_all) {
+                        double *tile, int nw, const int *first_all) {
     const int na = __popc(mask);
     if (na == 0) return true;
     const int ld = S.ld, n = S.n, T = S.tile;
@@ -711,9 +729,9 @@ __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int bu
 #pragma unroll
     for (int c = 0; c < 13; ++c) acc[c] = 0;
     #pragma unroll 1
-    for (int j0 = 0; j0 < n; j0 += T) {
-        const int cnt = min(T, n - j0);
-        if (!staged) {
+    for (int j0 = 0; j0 < n; j0 += kL == kChunks ? T : n) {
+        const int cnt = kL == kChunks ? min(T, n - j0) : n;
+        if (kL == kChunks) {
             const double *src[TA_ROWS];
             tile_a_rows(S, pub, sc.has_delayed, src);
             if (!load_tile(S, sc, ts, tile, kTileW, src, TA_ROWS, j0, cnt, cnt, TA_ROWS)) return false;
@@ -721,7 +739,7 @@ __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int bu
         const int self = o.idx - j0;
 #pragma unroll 1
         for (int jj = g.tid; jj < cnt; jj += g.size)
-            if (jj != self) pair_a(o, tile, jj, acc);
+            if (jj != self) pair_a<kL == kWideA ? kWideW : kTileW>(o, tile, jj, acc);
     }
     // sums over each body's warp group: a warp reduce-scatter, then the group's warps in ascending order
     {
@@ -763,6 +781,7 @@ struct ReactStage {
     __device__ __forceinline__ double get(const double *p) const { return smem ? *p : __ldcg(p); }
 };
 constexpr int kRingTerms = kFieldMax * kRingPar * kRingDiskPar * 3;   // per-disk ring terms, [f][h][d][3]
+static_assert(kRingTerms <= kWideFree, "the ring terms must fit in the rows pass A leaves free at the wide stride");
 
 // Geopotential items (field body b, geopotential host slot e) on `nthr` threads (t = this
 // thread's index), G lanes per item: every item's lanes evaluate it together (gp_field_lanes on the
@@ -835,7 +854,7 @@ __device__ __forceinline__ v3 body_sep(const FieldBody &o, const double *pub, in
 
 // Geopotential items on warps [w_lo, w_hi), as many lanes per item as one round over the items allows
 // (more lanes: shorter chains).
-__device__ void ext_gp(const SysDev &S, const FieldBody *own, int nb, int buf, Scratch &sc, const ReactStage &st, int w_lo,
+__device__ __forceinline__ void ext_gp(const SysDev &S, const FieldBody *own, int nb, int buf, Scratch &sc, const ReactStage &st, int w_lo,
                        int w_hi) {
     if (sc.n_gp_e == 0) return;
     const double *pub = S.pub + (size_t)buf * PUB_NPLANES * S.ld;
@@ -961,7 +980,8 @@ __device__ __noinline__ void record_body(const SysDev &S, const Own &o, long lon
     for (int q = 0; q < 9; ++q) t[TR_RFRAME + q] = o.ring >= 0 ? rf[q] : 0.0;
 }
 
-__device__ bool pass_a(const SysDev &S, Own *own, int nb, int buf, bool deform_only, Scratch &sc, TileState &ts,
+template <Layout kL>
+__device__ __forceinline__ bool pass_a(const SysDev &S, Own *own, int nb, int buf, bool deform_only, Scratch &sc, TileState &ts,
                        double *tile) {
     const int ld = S.ld;
     const double *pub = S.pub + (size_t)buf * PUB_NPLANES * ld;
@@ -974,17 +994,17 @@ __device__ bool pass_a(const SysDev &S, Own *own, int nb, int buf, bool deform_o
         f.idx = o.idx; f.slot = threadIdx.x; f.GM = o.GM;
         for (int c = 0; c < 3; ++c) f.r[c] = o.r[c];
     }
-    const bool one_tile = S.n <= S.tile;
-    if (one_tile) {
+    if (kL != kChunks) {
         const double *src[TA_ROWS];
         tile_a_rows(S, pub, sc.has_delayed, src);
-        if (!load_tile(S, sc, ts, tile, kTileW, src, TA_ROWS, 0, S.n, S.n, TA_ROWS)) return false;
+        if (!load_tile(S, sc, ts, tile, kL == kWideA ? kWideW : kTileW, src, TA_ROWS, 0, S.n, S.n, TA_ROWS)) return false;
     } else {
         __syncthreads();
     }
     // The extended bodies' fields do not depend on the angular velocity, so they run beside the pass-A sweeps
-    // (one tile only: streaming tiles needs every warp): the ring items on the last warp, the geopotential
-    // items (sc.ext_overlap) on the kExtWarps - 1 warps before it. With streaming tiles they run on every warp
+    // (not with streaming tiles, which need every warp): the ring items on the last warp, the geopotential
+    // items (sc.ext_overlap) on the kExtWarps - 1 warps before it. With streaming tiles, and at the wide stride in a
+    // CTA that owns a delayed tide and could not hand them over, they run on every warp
     // after the sweeps. The per-disk ring terms and, when they fit, the reactions are staged in the rows of
     // the pass-A tile that pass A does not use.
     const bool fields = !deform_only && S.n_ext > 0 && !sc.fields_away;
@@ -992,9 +1012,11 @@ __device__ bool pass_a(const SysDev &S, Own *own, int nb, int buf, bool deform_o
     const bool gp_side = fields && sc.ext_overlap;
     const int max_iter = deform_only ? 1 : 4;   // MAX_ANGULAR_VELOCITY_ITER (mass.impl:74)
     const int nw = deform_only ? kWarps : sc.nw_a;
-    double *xa = tile + (size_t)TA_ROWS * kTileW;
+    // (staged whole at the wide stride: the velocity rows beside the sweeps, anything after them)
+    const bool beside = kL == kWideA && sc.ext_overlap;
+    double *xa = tile + (beside ? TA_V_HI * kWideW : TA_ROWS * kTileW);
     const int nf = sc.nfb;
-    const ReactStage st{kRingTerms + nf * S.n_ext * 12 <= (kTileRows - TA_ROWS) * kTileW ? xa + kRingTerms : nullptr, nf};
+    const ReactStage st{kRingTerms + nf * S.n_ext * 12 <= (beside ? kWideFree : (kTileRows - TA_ROWS) * kTileW) ? xa + kRingTerms : nullptr, nf};
     const int warp = threadIdx.x >> 5;
     if (warp < nw) {
         #pragma unroll 1
@@ -1004,7 +1026,7 @@ __device__ bool pass_a(const SysDev &S, Own *own, int nb, int buf, bool deform_o
                 // the pair sums depend on the angular velocity only for delayed tides
                 if (it == 0 || (!own[b].converged && own[b].kind == 2)) mask |= 1u << b;
             }
-            if (!sweep_a(S, own, nb, mask, buf, sc, ts, tile, one_tile, nw, it == 0 ? sc.split_a0 : nullptr)) return false;
+            if (!sweep_a<kL>(S, own, nb, mask, buf, sc, ts, tile, nw, it == 0 ? sc.split_a0 : nullptr)) return false;
             if (S.timers && threadIdx.x == 0) sc.t_phase[PH_A_COUNT] += 1;
             mark(S, sc, PH_A_SWEEP);   // thread 0 sits in a sweep warp
             // harmonics and angular velocity of the owned bodies: lane 0 of warp b updates body b
@@ -1164,7 +1186,8 @@ __device__ __forceinline__ void sweep_b_range(const Own &o, const double *tile, 
         if (jj != self) pair_b<IF, JF>(o, tile, jj, acc, x);
 }
 
-__device__ bool pass_b(const SysDev &S, Own *own, int nb, int buf, Scratch &sc, TileState &ts, double *tile) {
+template <Layout kL>
+__device__ __forceinline__ bool pass_b(const SysDev &S, Own *own, int nb, int buf, Scratch &sc, TileState &ts, double *tile) {
     const int ld = S.ld, n = S.n, T = S.tile;
     const double *pub = S.pub + (size_t)buf * PUB_NPLANES * ld;
     const double *aux = S.aux, *cst = S.cst;
@@ -1177,12 +1200,12 @@ __device__ bool pass_b(const SysDev &S, Own *own, int nb, int buf, Scratch &sc, 
     for (int c = 0; c < 9; ++c) acc[c] = 0;
     Extremes x{__longlong_as_double(0x7ff0000000000000ll), 0.0, 0.0, 0.0};   // m_min = +inf
     #pragma unroll 1
-    for (int j0 = 0; j0 < n; j0 += T) {
-        const int cnt = min(T, n - j0);
+    for (int j0 = 0; j0 < n; j0 += kL == kOneTile ? n : T) {
+        const int cnt = kL == kOneTile ? n : min(T, n - j0);
         const int cnt_full = max(0, min(cnt, S.n_full - j0));
         // rows every body needs, then rows only full-class bodies need; with one tile the positions, GM
         // and sR2 are still in the tile from pass A of this stage (`reuse`)
-        const bool reuse = n <= T;
+        constexpr bool reuse = kL == kOneTile;
         const double *src[TB_ROWS] = {
             reuse ? nullptr : pub + (PUB_R_HI + 0) * ld, reuse ? nullptr : pub + (PUB_R_HI + 1) * ld,
             reuse ? nullptr : pub + (PUB_R_HI + 2) * ld, reuse ? nullptr : pub + (PUB_R_LO + 0) * ld,
@@ -1513,11 +1536,12 @@ __device__ void rk_stage(const SysDev &S, Own *own, int nb, int s, long long i_s
 // requires) and the CTAs that handed over their fields report zero reactions. Uses the staging tile, not
 // yet filled, as scratch; ends with a CTA barrier.
 constexpr int kPlanCtas = 1024;   // CTAs the hand-off plan handles (grids are at most the SM count)
+template <Layout kL>
 __device__ void field_handoff(const SysDev &S, const StepParams &P, const Own *own, int nb, Scratch &sc, double *tile) {
     int *cta_del = reinterpret_cast<int *>(tile);   // [grid]: the CTA owns a delayed tide
     int *cta_nb = cta_del + kPlanCtas;              // [grid]: bodies of the CTA
-    const bool possible = P.mode != MODE_DEFORM && S.n_ext > 0 && S.n <= S.tile && gridDim.x <= kPlanCtas &&
-                          kRingTerms + kFieldMax * S.n_ext * 12 <= (kTileRows - TA_ROWS) * kTileW;
+    const bool possible = P.mode != MODE_DEFORM && S.n_ext > 0 && kL != kChunks && gridDim.x <= kPlanCtas &&
+                          kRingTerms + kFieldMax * S.n_ext * 12 <= (kL == kWideA ? kWideFree : (kTileRows - TA_ROWS) * kTileW);
     const int n = S.n;
     for (int c = threadIdx.x; c < (int)gridDim.x; c += blockDim.x) {
         int d = 0, k = 0;
@@ -1561,6 +1585,7 @@ __device__ void field_handoff(const SysDev &S, const StepParams &P, const Own *o
 }
 
 // ------------------------------------------------------------------ the kernel
+template <Layout kL>
 __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams P) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     Own *own = reinterpret_cast<Own *>(smem_raw);
@@ -1619,7 +1644,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams 
     }
     __syncthreads();
     load_own(S, own, nb, P);
-    field_handoff(S, P, own, nb, sc, tile);
+    field_handoff<kL>(S, P, own, nb, sc, tile);
     __syncthreads();
     if (threadIdx.x < nb) publish_body(S, own[threadIdx.x], 0);
     if (threadIdx.x == 32) {
@@ -1630,7 +1655,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams 
         bool delayed = false;
         for (int b = 0; b < nb; ++b) delayed |= own[b].kind == 2;
         sc.has_delayed = delayed;
-        const bool side = P.mode != MODE_DEFORM && S.n_ext > 0 && S.n <= S.tile && !sc.fields_away;
+        const bool side = P.mode != MODE_DEFORM && S.n_ext > 0 && (kL == kOneTile || (kL == kWideA && !delayed)) && !sc.fields_away;
         sc.ext_overlap = side;
         sc.ring_side = side && sc.n_ring_e > 0;
         sc.nw_a = sc.ext_overlap ? kWarps - kExtWarps : sc.ring_side ? kWarps - 1 : kWarps;
@@ -1641,7 +1666,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams 
         // pass-B sweep (one tile only: streaming tiles needs every warp for the copies)
         bool host = false;
         for (int b = 0; b < nb; ++b) host |= own[b].ext_slot >= 0;
-        sc.nw_b = (host && S.n <= S.tile && nb < kWarps) ? kWarps - 1 : kWarps;
+        sc.nw_b = (host && kL == kOneTile && nb < kWarps) ? kWarps - 1 : kWarps;
         split_warps(wt, nb, sc.nw_b, sc.split_b);
     }
     auto sync = [&]() {
@@ -1649,56 +1674,54 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams 
         mark(S, sc, PH_BARRIER);
         return ok;
     };
-    auto finish = [&](bool deform_only) {
-        store_own(S, own, nb, deform_only);
-        __syncthreads();
-        mark(S, sc, PH_IO);
-        if (S.timers && threadIdx.x == 0)
-            for (int p = 0; p < kPhases; ++p) S.timers[blockIdx.x * kPhases + p] = sc.t_phase[p];
-    };
     mark(S, sc, PH_IO);
 
-    if (P.mode == MODE_DEFORM || P.mode == MODE_ACCEL) {
-        if (!sync()) return;
-        if (threadIdx.x == 0) sc.traj_slot = S.traj_base;
-        if (!pass_a(S, own, nb, 0, P.mode == MODE_DEFORM, sc, ts, tile)) return;
-        if (P.mode == MODE_ACCEL) {
-            if (!sync()) return;
-            if (!pass_b(S, own, nb, 0, sc, ts, tile)) return;
+    // One loop, and one call of each pass, for all modes: MODE_DEFORM and MODE_ACCEL are one evaluation of the
+    // loaded state without a stage update. (Two copies of the passes cost registers and instruction cache.)
+    const bool integrate = P.mode == MODE_INTEGRATE, deform_only = P.mode == MODE_DEFORM;
+    const long long n_step = integrate ? P.n_step : 1;
+    const int n_stage = integrate ? kStages : 1;
+    if (integrate) {   // the loaded auxiliaries are f_0 of the first step
+        if (threadIdx.x < nb) {
+            Own &o = own[threadIdx.x];
+            stv(o.fa, (ldv(o.gacc) + ldv(o.dacc)) + ldv(o.nacc));
         }
-        finish(P.mode == MODE_DEFORM);
-        return;
+        __syncthreads();
     }
-    // MODE_INTEGRATE: the loaded auxiliaries are f_0 of the first step
-    if (threadIdx.x < nb) {
-        Own &o = own[threadIdx.x];
-        stv(o.fa, (ldv(o.gacc) + ldv(o.dacc)) + ldv(o.nacc));
-    }
-    __syncthreads();
     int buf = 0;
     #pragma unroll 1
-    for (long long step = 0; step < P.n_step; ++step) {
+    for (long long step = 0; step < n_step; ++step) {
         #pragma unroll 1
-        for (int s = 0; s < kStages; ++s) {
-            rk_stage(S, own, nb, s, step, P, buf ^ 1, sc);
-            mark(S, sc, PH_RK);
-            buf ^= 1;
+        for (int s = 0; s < n_stage; ++s) {
+            if (integrate) {
+                rk_stage(S, own, nb, s, step, P, buf ^ 1, sc);
+                mark(S, sc, PH_RK);
+                buf ^= 1;
+            }
             if (!sync()) return;
             if (threadIdx.x == 0) sc.traj_slot = S.traj_base + step * kStages + s;
-            if (!pass_a(S, own, nb, buf, false, sc, ts, tile)) return;
+            if (!pass_a<kL>(S, own, nb, buf, deform_only, sc, ts, tile)) return;
+            if (deform_only) break;
             if (!sync()) return;
-            if (!pass_b(S, own, nb, buf, sc, ts, tile)) return;
+            if (!pass_b<kL>(S, own, nb, buf, sc, ts, tile)) return;
         }
     }
-    if (P.invert_min && threadIdx.x < nb) own[threadIdx.x].mind = 1 / own[threadIdx.x].mind;
+    if (integrate && P.invert_min && threadIdx.x < nb) own[threadIdx.x].mind = 1 / own[threadIdx.x].mind;
     __syncthreads();
-    finish(false);
+    store_own(S, own, nb, deform_only);
+    __syncthreads();
+    mark(S, sc, PH_IO);
+    if (S.timers && threadIdx.x == 0)
+        for (int p = 0; p < kPhases; ++p) S.timers[blockIdx.x * kPhases + p] = sc.t_phase[p];
 }
 
 }  // namespace eph
 
 // ------------------------------------------------------------------ host launcher
 namespace eph {
+
+static const void *const kStepKernels[] = {(const void *)step_kernel<kOneTile>, (const void *)step_kernel<kWideA>,
+                                           (const void *)step_kernel<kChunks>};
 
 size_t step_fixed_smem_bytes() { return kFixedSmem; }
 // the tile is always allocated at its full stride; `tile` (bodies staged per chunk) does not change the size
@@ -1721,20 +1744,26 @@ cudaError_t upload_constants(int device) {
     cudaError_t e = cudaMemcpyToSymbol(c_rk_hi, hi, sizeof(hi));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_rk_lo, lo, sizeof(lo));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_dtk, dtk, sizeof(dtk));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    for (int l = 0; l < 3 && e == cudaSuccess; ++l)
+        e = cudaFuncSetAttribute(kStepKernels[l], cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e == cudaSuccess && device >= 0 && device < 64) g_consts_ready[device].store(true, std::memory_order_release);
     return e;
 }
 
 cudaError_t launch_step(const SysDev &S, const StepParams &P, int grid, cudaStream_t stream) {
     void *args[] = {(void *)&S, (void *)&P};
-    return cudaLaunchCooperativeKernel((void *)step_kernel, dim3(grid), dim3(kThreads), args, step_smem_bytes(S.tile),
-                                       stream);
+    return cudaLaunchCooperativeKernel(kStepKernels[layout_of(S.n, S.tile)], dim3(grid), dim3(kThreads), args,
+                                       step_smem_bytes(S.tile), stream);
 }
 
 int max_coresident_ctas(int device, int tile, int *out) {
     int per_sm = 0, sms = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, step_kernel, kThreads, step_smem_bytes(tile));
+    cudaError_t e = cudaSuccess;
+    for (int l = 0; l < 3 && e == cudaSuccess; ++l) {
+        int one = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, kStepKernels[l], kThreads, step_smem_bytes(tile));
+        per_sm = l ? std::min(per_sm, one) : one;
+    }
     if (e != cudaSuccess) return (int)e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return (int)e;

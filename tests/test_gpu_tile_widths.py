@@ -1,0 +1,36 @@
+"""Full-physics systems around the widths at which the step kernel stages the bodies differently: one tile up to 576, pass
+A whole at twice the stride up to 1152, chunks beyond. One acceleration evaluation and one RK12 step against the oracle,
+tolerances as in tests/test_gpu_paths.py."""
+import os
+
+import numpy as np
+import pytest
+
+from tests.parity import accel_error, position_error
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,step", [(576, False), (577, True), (1151, False), (1152, True), (1153, False), (1184, False)])
+def test_tile_widths(tmp_path, oracle, n, step):
+    from ephemeris_b200 import Context, Models, MSystem, synth
+    from oracle.pyoracle import Models as OModels
+    sysm = synth.make_config2(2002, n_asteroids=n - 162)
+    ms = MSystem(0)
+    assert ms.load(synth.write_system(sysm, os.path.join(str(tmp_path), "big")))
+    pl, md, dt = ms.planes(), ms.models(), ms.delta_t
+    ms.close()
+    assert pl.shape[1] == n
+    om = OModels(md.gp_nz, md.gp_nt, md.gp_coef, md.ring_ndisk, md.ring_param, md.ring_disk)
+    c = Context(0)
+    c.upload(pl, md)
+    c.accel()
+    out = c.download()
+    ref = oracle.accel(pl, om)
+    assert accel_error(out, ref) <= 1e-14
+    assert np.allclose(out[36:39], ref[36:39], rtol=1e-13, atol=0)      # the angular-velocity fixed point
+    if step:
+        c.upload(pl, md)
+        c.integrate(dt, 1)
+        assert position_error(c.download(), oracle.integrate(pl, om, dt, 1)[0]) <= 1e-12
+    c.close()

@@ -50,13 +50,17 @@ constexpr double kC = 299792458.0;                      // src/math/basic_math.h
 __constant__ double c_rk_hi[EPH_RK12_NCOEF];            // a_kj, double-double
 __constant__ double c_rk_lo[EPH_RK12_NCOEF];
 __constant__ double c_dtk[kStages + 1];                 // c_k = sum of nonzero a_kj, summed in j order
+__constant__ double c_rdtk[kStages + 1];                // 1 / c_k
 
 // ------------------------------------------------------------------ owned-body private state (shared memory)
+constexpr int kSumA = 11, kSumB = 10;   // pair sums of one body: see pair_a, pair_b
+constexpr int kSums = 12, kSumPad = 15; // width of the reductions; its stride in shared memory (odd: no bank conflicts)
 struct Own {
     int idx, kind, gp, ring;          // kind: 0 point Newtonian (k2 == 0), 1 undelayed tide, 2 delayed tide
     int converged, ext_slot, gl_fixed, full;   // ext_slot: index in the extended-body list, or -1
     int orig, pad1, pad2, pad3;               // orig: index in the caller's plane arrays
     double GM0, dGM, dJ2, R, R2, A, k2, k2r, td, sR2, rR2G4c;
+    double rad, cR;                   // rR2G4c / GM, R^3 / (2 GM) of the stage
     double Cst[9];
     double ring_GM_ratio, ring_GL_R2;
     // current stage state
@@ -68,7 +72,6 @@ struct Own {
     // auxiliaries
     double phi, nacc[3], C[9], GI[9], beta[3], beta2;
     double gacc[3], dacc[3], dtq[3], Egrad[3], mind, maxi;
-    double sumA[13];
     double Cs[9];                     // s (C_static + exJ2 terms) s^T of the stage (fixed during the fixed point)
     double fa[3];                     // f_s acceleration of the current stage
     double wnew[3], dw[3];            // stage angular velocity and its 2/3 increment (state update)
@@ -95,7 +98,10 @@ struct FieldBody {
 };
 
 struct Scratch {
-    double part[kWarps][16];          // per-warp partial sums
+    double part[kWarps][kSumPad];     // per-warp partial sums
+    int wbody[kWarps];                // owned body that each sweep warp works for
+    double red[kOwnMax][kSumPad];     // sums of the latest sweep, see group_sums
+    short row_a[TA_ROWS], row_b[TB_ROWS];   // source plane of each tile row, or -1: not copied (tile_rows)
     int split_a0[kOwnMax + 1];        // warp groups of the first pass-A sweep (all owned bodies, weighted)
     int split_b[kOwnMax + 1];         // warp groups of the pass-B sweep (all owned bodies, weighted)
     int nw_b;                         // warps of the pass-B sweep (the last one sums host reactions meanwhile)
@@ -123,18 +129,18 @@ struct Scratch {
     int flag, pad;
 };
 
-// Shared memory: the owned bodies, the scratch, then the staging tile of kTileRows rows. The tile's row stride
+// Shared memory: the owned bodies, the scratch, the staging tile of kTileRows rows, then the ring terms. The tile's row stride
 // kTileW is fixed at compile time (the widest tile that fits), so that every tile access is a fixed offset
 // from the body's column; a system of n <= kTileW bodies is staged in one tile, a larger one in chunks.
-constexpr int kMaxSmem = 227 * 1024 - 4096;   // the 227 KB per-CTA maximum less room for static arrays
+constexpr int kMaxSmem = 227 * 1024;   // the per-CTA maximum; the kernel has no static arrays
 constexpr size_t kFixedSmem = ((sizeof(Own) * kOwnMax + sizeof(Scratch) + 127) / 128) * 128;
-constexpr int kTileW = (int)((kMaxSmem - kFixedSmem) / (kTileRows * sizeof(double))) / kPad * kPad;
+constexpr int kRingTerms = kFieldMax * kRingPar * kRingDiskPar * 3;   // per-disk ring terms, [f][h][d][3], behind the tile
+constexpr int kTileW = (int)((kMaxSmem - kFixedSmem - kRingTerms * sizeof(double)) / (kTileRows * sizeof(double))) / kPad * kPad;
 static_assert(kTileW >= 512, "the staging tile must hold a 512-body system in one piece");
 // Pass A reads half as many rows as the tile has: a system of up to twice the tile's width is staged whole for its
 // sweeps, at twice the row stride, instead of in chunks that every iteration of the angular-velocity fixed point
-// copies again. Rows 6 to 11, the velocities, are free in a CTA without a delayed tide: its field items run beside
-// its sweeps there, and it takes those of the CTAs with one, as in a system of one tile. 1,001 bodies, full physics:
-// 60 -> 52 us per stage.
+// copies again. Rows 6 to 11, the velocities, are free in a CTA without a delayed tide: the reactions of its field
+// items stay there. 1,001 bodies, full physics: 60 -> 52 us per stage.
 constexpr int kWideW = 2 * kTileW;
 static_assert(TA_ROWS * kWideW <= kTileRows * kTileW && TA_V_HI == 6 && TA_V_LO + 3 == TA_GM, "pass-A rows at the wide stride");
 constexpr int kWideFree = (TA_GM - TA_V_HI) * kWideW;   // doubles of the free rows
@@ -142,6 +148,8 @@ constexpr int kWideFree = (TA_GM - TA_V_HI) * kWideW;   // doubles of the free r
 // strides and loop bounds are constants, and the code that the stage loop runs through (which a small system does
 // not stay long enough in to keep in the instruction cache) is shorter. 48 / 504 bodies, full physics: 26 -> 22 and
 // 30 -> 27 us per stage.
+constexpr int kRowAux = 256, kRowCst = 512;   // tile row sources: plane of pub, kRowAux + plane of aux, kRowCst + plane of cst
+static_assert(PUB_NPLANES < kRowAux, "planes of a row source");
 enum Layout { kOneTile, kWideA, kChunks };   // one tile; pass A whole at the wide stride, pass B in chunks; chunks
 static Layout layout_of(int n, int tile) {   // a tile below the stride was asked for: chunks of that size
     return n <= tile ? kOneTile : tile == kTileW && n <= kWideW ? kWideA : kChunks;
@@ -224,38 +232,42 @@ struct TileState {
 
 __device__ __forceinline__ void mbar_init(Scratch &sc) {
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sc.mbar)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&sc.mbar)), "n"(kWarps) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
 }
 
-// Copy `rows` planes (row r from src[r] + j0, `count` bodies rounded up to kPad; rows from `tail_from` on
-// `count_tail` bodies; a null src[r] keeps tile row r as it is) into tile rows of `stride` doubles. Every
-// thread waits for completion (bounded). Returns false on timeout.
-__device__ bool load_tile(const SysDev &S, Scratch &sc, TileState &ts, double *tile, int stride,
-                                       const double *const *src, int rows, int j0, int count, int count_tail,
-                                       int tail_from) {
+// Copy planes into tile rows of `stride` doubles: row r < nrows from the plane rows[r] names (tile_rows; -1 keeps the
+// tile row as it is), from body j0, `count` bodies rounded up to kPad; rows from `tail_from` on `count_tail` bodies. The
+// rows are dealt over the warps, whose first lanes issue them at the same time, and start with another row in each
+// CTA, which spreads the CTAs' reads over the planes: 19.9 -> 19.1 / 25.2 -> 24.4 us per stage for 48 / 504 bodies, the
+// two copies of a stage 2.6 -> 1.9 us. Every thread waits for completion (bounded). Returns false on timeout.
+__device__ __forceinline__ bool load_tile(const SysDev &S, Scratch &sc, TileState &ts, double *tile, int stride, const double *pub,
+                                       const short *rows, int nrows, int j0, int count, int count_tail, int tail_from) {
     __syncthreads();   // the previous sweep's reads of the tile are done
-    const int cpad = (count + kPad - 1) / kPad * kPad;
-    const int tpad = (count_tail + kPad - 1) / kPad * kPad;
-    const unsigned bytes = (unsigned)cpad * 8u, tbytes = (unsigned)tpad * 8u;
-    unsigned total = 0;
-    for (int r = 0; r < rows; ++r)
-        if (src[r]) total += r < tail_from ? bytes : tbytes;
     const unsigned mb = smem_addr(&sc.mbar);
-    if (threadIdx.x == 0) {
+    if ((threadIdx.x & 31) == 0) {
+        const unsigned bytes = (unsigned)((count + kPad - 1) / kPad * kPad) * 8u;
+        const unsigned tbytes = (unsigned)((count_tail + kPad - 1) / kPad * kPad) * 8u;
+        const int r0 = ((threadIdx.x >> 5) + blockIdx.x) % kWarps;
         // order the generic-proxy accesses (tile reads, other CTAs' global stores) before the copies
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("fence.proxy.async.global;" ::: "memory");
+        unsigned total = 0;
+        #pragma unroll 1
+        for (int r = r0; r < nrows; r += kWarps) total += rows[r] < 0 ? 0u : r < tail_from ? bytes : tbytes;
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(total) : "memory");
-        for (int r = 0; r < rows; ++r) {
+        #pragma unroll 1
+        for (int r = r0; r < nrows; r += kWarps) {
             const unsigned nbytes = r < tail_from ? bytes : tbytes;
-            if (nbytes == 0 || !src[r]) continue;
+            const int id = rows[r];
+            if (nbytes == 0 || id < 0) continue;
+            const double *base = id < kRowAux ? pub : id < kRowCst ? S.aux : S.cst;
             asm volatile(
                 "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                     smem_addr(tile + (size_t)r * stride)),
-                "l"(src[r] + j0), "r"(nbytes), "r"(mb)
+                "l"(base + (size_t)(id & (kRowAux - 1)) * S.ld + j0), "r"(nbytes), "r"(mb)
                 : "memory");
         }
     }
@@ -298,15 +310,6 @@ __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ double warp_cmax(double v) {   // NaN-propagating maximum
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double u = __shfl_xor_sync(0xffffffffu, v, o);
-        checked_maximize(v, u);
-    }
-    return v;
-}
-
 __device__ __forceinline__ v3 ld3(const double *p, int ld, int i) {
     return mk(__ldcg(p + i), __ldcg(p + ld + i), __ldcg(p + 2 * ld + i));
 }
@@ -378,75 +381,74 @@ __device__ __forceinline__ void part_sync(int nthreads) {
     else asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
 }
 
-__device__ __forceinline__ double combine(double a, double b, bool is_max) {
-    if (is_max) {
-        checked_maximize(a, b);
-        return a;
-    }
-    return a + b;
+// The two reductions behind both passes' sweeps, kept short: a stage runs through its code once, so every instruction
+// of it is fetched, not reused, and those fetches are the largest stall of a small system. (Out of line they cost
+// more than they save: a call that takes the kernel's parameters by reference moves them to local memory.) With the
+// one-copy pair_b, 48 / 504 bodies, full physics: 22.3 -> 19.9 / 28.5 -> 25.2 us per stage.
+//
+// Sums over the warp of 12 values per lane, into row[0..11] (the first `cnt`): a reduce-scatter that halves what a lane
+// holds, 12 -> 6 -> 3 -> 2 (or 1) -> 1 -> 1 shuffles, 13 instead of 5 per value.
+__device__ __forceinline__ void warp_sums(double a0, double a1, double a2, double a3, double a4, double a5, double a6, double a7,
+                                       double a8, double a9, double a10, double a11, double *row, int cnt) {
+    constexpr unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4, u2 = lane & 2;
+    auto half = [&](bool up, double lo, double hi, int bit) {
+        return (up ? hi : lo) + __shfl_xor_sync(all, up ? lo : hi, bit);
+    };
+    const double b0 = half(u16, a0, a6, 16), b1 = half(u16, a1, a7, 16), b2 = half(u16, a2, a8, 16);
+    const double b3 = half(u16, a3, a9, 16), b4 = half(u16, a4, a10, 16), b5 = half(u16, a5, a11, 16);
+    const double c0 = half(u8, b0, b3, 8), c1 = half(u8, b1, b4, 8), c2 = half(u8, b2, b5, 8);
+    const double d0 = half(u4, c0, c2, 4);   // lanes without bit 4: value 0 of three, the others: value 2
+    const double d1 = c1 + __shfl_xor_sync(all, c1, 4);
+    const double f = (u4 ? d0 : u2 ? d1 : d0) + __shfl_xor_sync(all, u4 ? d0 : u2 ? d0 : d1, 2);
+    const double r = f + __shfl_xor_sync(all, f, 1);
+    const int id = (u16 ? 6 : 0) + (u8 ? 3 : 0) + (u4 ? 2 : u2 ? 1 : 0);
+    if ((lane & 1) == 0 && !(u4 && u2) && id < cnt) row[id] = r;
 }
 
-// Reduce-scatter of 16 per-lane values over the warp: afterwards lanes 2c and 2c+1 hold the warp sum of
-// value c. 16 shuffles (8 + 4 + 2 + 1 + 1) instead of 5 per value.
-__device__ __forceinline__ double warp_reduce_scatter16(double (&v)[16], int lane) {
-#pragma unroll
-    for (int h = 8, bit = 16; h >= 1; h >>= 1, bit >>= 1) {
-        const bool up = (lane & bit) != 0;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const double send = up ? v[k] : v[k + h];
-            const double keep = up ? v[k + h] : v[k];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
-        }
-    }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+// Order-preserving integer keys of the extremes, whose largest wins: a NaN is above everything. m >= 0 by its
+// distance below infinity (the smallest m wins), GM/r^3 >= 0 as it is.
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ull, kNanKey = 0x7fffffffffffffffull;
+__device__ __forceinline__ unsigned long long key_of(double v) {
+    return v != v ? kNanKey : (unsigned long long)__double_as_longlong(v);
 }
 
-// Sum NV per-thread values over each group of the first `nw` warps (a warp reduce-scatter, then the
-// group's warps in order, four interleaved partial sums) into out[slot][0..NV); entries c >= max_from are
-// NaN-propagating maxima (reduced across the warp with shuffles of their own).
-template <int NV>
-__device__ __forceinline__ void group_reduce(const double (&acc)[NV], const int *first, int na, int nw, Scratch &sc,
-                                             double (*out)[16], int max_from) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    {
-        double v[16];
-#pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = (c < NV && c < max_from) ? acc[c] : 0.0;
-        const double r = warp_reduce_scatter16(v, lane);
-        if ((lane & 1) == 0 && (lane >> 1) < min(NV, max_from)) sc.part[w][lane >> 1] = r;
-    }
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        if (c < max_from) continue;
-        const double v = warp_cmax(acc[c]);
-        if (lane == 0) sc.part[w][c] = v;
-    }
-    part_sync(nw * 32);
+// Sums over each body's warps of what the first `nw` warps left in sc.part, into sc.red[body], for the bodies of
+// `mask`: a half warp per (body, value), a lane per warp, summed as a tree. With `ext` (pass B), value 10 is the key
+// of the smallest m and value 11 that of the largest GM/r^3, which carries the pair's m and GM in 12 and 13; ties go
+// to the lower warp. Called between two barriers over the nw warps.
+__device__ __forceinline__ void group_sums(Scratch &sc, int nb, unsigned mask, int nw, bool ext) {
+    constexpr unsigned all = 0xffffffffu;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = lane & 15;
+    static_assert(kWarps == 16, "a half warp holds one value of every warp");
+    const int body_w = w < nw ? sc.wbody[w] : -1;
     #pragma unroll 1
-    for (int idx = threadIdx.x; idx < na * NV; idx += nw * 32) {
-        const int slot = idx / NV, c = idx % NV;
-        const int w0 = first[slot], w1 = first[slot + 1];
-        const bool mx = c >= max_from;
-        // four interleaved partial sums over the group's warps (w0 + 4m + q), then combined in q order
-        double s0 = sc.part[w0][c], s1 = 0, s2 = 0, s3 = 0;
-        const bool h1 = w0 + 1 < w1, h2 = w0 + 2 < w1, h3 = w0 + 3 < w1;
-        if (h1) s1 = sc.part[w0 + 1][c];
-        if (h2) s2 = sc.part[w0 + 2][c];
-        if (h3) s3 = sc.part[w0 + 3][c];
-        for (int ww = w0 + 4; ww < w1; ww += 4) {
-            s0 = combine(s0, sc.part[ww][c], mx);
-            if (ww + 1 < w1) s1 = combine(s1, sc.part[ww + 1][c], mx);
-            if (ww + 2 < w1) s2 = combine(s2, sc.part[ww + 2][c], mx);
-            if (ww + 3 < w1) s3 = combine(s3, sc.part[ww + 3][c], mx);
+    for (int base = warp * 2; base < nb * kSums; base += nw * 2) {
+        const int item = base + (lane >> 4), b = item / kSums, c = item - b * kSums;
+        double v = body_w == b ? sc.part[w][c] : 0.0;
+        if (ext && c >= kSumB) {   // (uniform over the warp: base and kSums are even)
+            unsigned long long k = (unsigned long long)__double_as_longlong(v);
+            int src = w;
+            #pragma unroll
+            for (int h = 8; h >= 1; h >>= 1) {
+                const unsigned long long ok = __shfl_xor_sync(all, k, h);
+                const int os = __shfl_xor_sync(all, src, h);
+                if (ok > k || (ok == k && os < src)) { k = ok; src = os; }
+            }
+            if (w == 0) {
+                sc.red[b][c] = __longlong_as_double((long long)k);
+                if (c == kSumB + 1) {
+                    sc.red[b][12] = sc.part[src][12];
+                    sc.red[b][13] = sc.part[src][13];
+                }
+            }
+            continue;
         }
-        double r = s0;
-        if (h1) r = combine(r, s1, mx);
-        if (h2) r = combine(r, s2, mx);
-        if (h3) r = combine(r, s3, mx);
-        out[slot][c] = r;
+        #pragma unroll
+        for (int h = 8; h >= 1; h >>= 1) v += __shfl_xor_sync(all, v, h);
+        if (w == 0 && (mask >> b & 1)) sc.red[b][c] = v;
     }
-    part_sync(nw * 32);
 }
 
 // ------------------------------------------------------------------ load / publish / store
@@ -532,7 +534,7 @@ __device__ void store_own(const SysDev &S, const Own *own, int nb, bool deform_o
 }
 
 // publish the stage state of owned body o into public buffer `buf` (one thread)
-__device__ void publish_body(const SysDev &S, const Own &o, int buf) {
+__device__ __noinline__ void publish_body(const SysDev &S, const Own &o, int buf) {
     const int ld = S.ld, i = o.idx;
     double *pub = S.pub + (size_t)buf * PUB_NPLANES * ld;
     for (int c = 0; c < 3; ++c) {
@@ -578,60 +580,57 @@ __device__ void publish_body_warp(const SysDev &S, const Own &o, int buf, int la
 }
 
 // ------------------------------------------------------------------ pass A: deform_by + angular velocity
-// One ordered pair (i = owned body o, j from the tile) of DAMPED_TIDAL_DEFORMATION_MATRIX / _NDELAY /
-// _NK2 (mass.impl:1-46), accumulated into acc = {phi, naccel[3], C[9]}.
+// One ordered pair (i = owned body o, j from the tile) of DAMPED_TIDAL_DEFORMATION_MATRIX / _NDELAY / _NK2
+// (mass.impl:1-46). With g = GM_j / r^3, the deformed direction x (r itself without a delay) and the diagonal d,
+// accumulates {sum GM_j / r, sum g r (3), the symmetric sum of g (x x^T / r^2 - ...) as xx xy xz yy yz zz, sum g d}:
+// the tidal matrix is 3 k2 (the symmetric sum + the last sum on its diagonal), formed once in update_body. Three
+// reciprocal square roots per delayed pair, none of a normalised rate: with the rate vector d = td tdf_j w_rel,
+// dwt^2 = |d|^2, and the factors that multiply its direction and its dyad (y0, z02) hold dwt and dwt^2.
+// 504 bodies, full physics: 5.3 -> 5.0 us of sweeps per stage (latency bounds them: 12 warps, one pair in flight each).
 template <int ts>
-__device__ __forceinline__ void pair_a(const Own &o, const double *T, int j, double acc[13]) {
+__device__ __forceinline__ void pair_a(const Own &o, const double *T, int j, double acc[kSumA]) {
     v3 r = mk(sep_diff(T[(TA_R_HI + 0) * ts + j], T[(TA_R_LO + 0) * ts + j], o.r[0].hi, o.r[0].lo),
               sep_diff(T[(TA_R_HI + 1) * ts + j], T[(TA_R_LO + 1) * ts + j], o.r[1].hi, o.r[1].lo),
               sep_diff(T[(TA_R_HI + 2) * ts + j], T[(TA_R_LO + 2) * ts + j], o.r[2].hi, o.r[2].lo));
     const double GMj = T[TA_GM * ts + j], sR2j = T[TA_SR2 * ts + j];
-    double q = dot(r, r), sm = o.sR2 + sR2j;
-    double rr = rsqrt((q < sm) ? sm : q);   // 1/r within 1 ulp; rr2 = rr^2
-    double rr2 = rr * rr;
-    double tp_dphi = rr * GMj;
-    double tp_dg = rr2 * tp_dphi;
-    acc[0] -= tp_dphi;
+    const double q = dot(r, r), sm = o.sR2 + sR2j;
+    const double rr = inv_sqrt((q < sm) ? sm : q);
+    const double rr2 = rr * rr;
+    const double tp_dphi = rr * GMj;
+    const double tp_dg = rr2 * tp_dphi;
+    acc[0] += tp_dphi;
     acc[1] += tp_dg * r.x;
     acc[2] += tp_dg * r.y;
     acc[3] += tp_dg * r.z;
     if (o.kind == 0) return;
-    double fk = (-3 * tp_dg) * o.k2;
-    m3 M;
+    v3 x = r;
+    double diag = -1.0 / 3;
     if (o.kind == 2) {
-        v3 v = mk(sep_diff(T[(TA_V_HI + 0) * ts + j], T[(TA_V_LO + 0) * ts + j], o.v[0].hi, o.v[0].lo),
-                  sep_diff(T[(TA_V_HI + 1) * ts + j], T[(TA_V_LO + 1) * ts + j], o.v[1].hi, o.v[1].lo),
-                  sep_diff(T[(TA_V_HI + 2) * ts + j], T[(TA_V_LO + 2) * ts + j], o.v[2].hi, o.v[2].lo));
-        v3 w = mk(o.w[0], o.w[1], o.w[2]);
-        v3 dw = rr2 * cross(r, cross(w, r) - v);
-        double dwt;
-        const double dw2 = dot(dw, dw);
-        if (dw2 > 0x1p-960 && dw2 < 0x1p960) {   // inside the range where normalize needs no rescaling
-            const double rn = rsqrt(dw2);
-            dwt = dw2 * rn;
-            dw = rn * dw;
-        } else {
-            dwt = normalize(dw);
-        }
-        dwt *= o.td * T[TA_TDF * ts + j];
+        const v3 v = mk(sep_diff(T[(TA_V_HI + 0) * ts + j], T[(TA_V_LO + 0) * ts + j], o.v[0].hi, o.v[0].lo),
+                        sep_diff(T[(TA_V_HI + 1) * ts + j], T[(TA_V_LO + 1) * ts + j], o.v[1].hi, o.v[1].lo),
+                        sep_diff(T[(TA_V_HI + 2) * ts + j], T[(TA_V_LO + 2) * ts + j], o.v[2].hi, o.v[2].lo));
+        const v3 w = mk(o.w[0], o.w[1], o.w[2]);
+        const v3 d = (rr2 * (o.td * T[TA_TDF * ts + j])) * cross(r, cross(w, r) - v);
         // x0, y0, z02 of the damped deformation (mass.impl:16-20) from two reciprocal square roots: with
         // e = 1 + 4 dwt^2, s = sqrt(e), u = 1 + s, re = 1/s and ru = 1/sqrt(u/2),
         //   x0 = sqrt(u / (2e)) = (u/2) ru re,  y0 = dwt sqrt(2 / (e u)) = dwt ru re,
         //   z02 = 2 dwt^2 / (e + s) = dwt^2 re ru^2.
-        const double e = 1 + 4 * dwt * dwt;
-        const double re = rsqrt(e);
+        const double t2 = dot(d, d);
+        const double e = 1 + 4 * t2;
+        const double re = inv_sqrt(e);
         const double hu = 0.5 * (1 + e * re);
-        const double ru = rsqrt(hu);
-        const double rue = ru * re;
-        const double x0 = hu * rue, y0 = dwt * rue, z02 = (dwt * dwt) * (rue * ru);
-        v3 dr = x0 * r + y0 * cross(dw, r);
-        M = add_diag(outer(rr2 * dr, dr) - outer(z02 * dw, dw), z02 - 1.0 / 3);
-    } else {
-        M = add_diag(outer(rr2 * r, r), -(1.0 / 3));
+        const double ru = inv_sqrt(hu);
+        const double rue = ru * re, z = rue * ru;
+        x = (hu * rue) * r + rue * cross(d, r);
+        diag += t2 * z;
+        const v3 y = (tp_dg * z) * d;
+        acc[4] -= y.x * d.x; acc[5] -= y.x * d.y; acc[6] -= y.x * d.z;
+        acc[7] -= y.y * d.y; acc[8] -= y.y * d.z; acc[9] -= y.z * d.z;
     }
-    acc[4] -= fk * M.x.x; acc[5] -= fk * M.x.y; acc[6] -= fk * M.x.z;
-    acc[7] -= fk * M.y.x; acc[8] -= fk * M.y.y; acc[9] -= fk * M.y.z;
-    acc[10] -= fk * M.z.x; acc[11] -= fk * M.z.y; acc[12] -= fk * M.z.z;
+    const v3 y = (tp_dg * rr2) * x;
+    acc[4] += y.x * x.x; acc[5] += y.x * x.y; acc[6] += y.x * x.z;
+    acc[7] += y.y * x.y; acc[8] += y.y * x.z; acc[9] += y.z * x.z;
+    acc[10] += tp_dg * diag;
 }
 
 // UPDATE_HARMONICS followed by UPDATE_ANGULAR_VELOCITY (mass.impl:48-72) for owned body o, on one thread,
@@ -642,21 +641,25 @@ __device__ __forceinline__ void pair_a(const Own &o, const double *T, int j, dou
 // same sums, harmonics and w, so stopping leaves the identical state; needed for w = 0, where
 // 0 < 1e-18 * 0 never passes). Small and branch-light on purpose: it runs once per fixed-point iteration on
 // the critical path of the stage.
-__device__ void update_body(Own &o, bool first, bool deform_only) {
+__device__ void update_body(Own &o, const double *sum, bool first, bool deform_only) {
     if (first) {
-        o.phi = o.sumA[0];
-        o.nacc[0] = o.sumA[1]; o.nacc[1] = o.sumA[2]; o.nacc[2] = o.sumA[3];
+        o.phi = -sum[0];
+        o.nacc[0] = sum[1]; o.nacc[1] = sum[2]; o.nacc[2] = sum[3];
         m3 mc = ldm(o.Cst);
         mc.x.x += o.exJ2 / 2;
         mc.y.y += o.exJ2 / 2;
         mc.z.z -= o.exJ2;
         stm(o.Cs, toworld(fast9(o.s), mc));
+        o.cR = o.R * o.R2 / (2 * o.GM);
     }
     const v3 w = ldv(o.w);
-    m3 C = ldm(o.sumA + 4);
-    C = add_diag(C, dot(w, w) * o.k2r / 3);
-    C = C - outer(o.k2r * w, w);
-    C = (o.R * o.R2 / (2 * o.GM)) * C;
+    const double *q = sum + 4, k3 = o.cR * (3 * o.k2), kr = o.cR * o.k2r;
+    // cR (tidal sums + k2r (w^2 / 3 - w w^T)) + the static part; symmetric but for the static part's rounding
+    const double d = k3 * q[6] + kr * (dot(w, w) * (1.0 / 3));
+    const v3 kw = kr * w;
+    m3 C = m3{{d + (k3 * q[0] - kw.x * w.x), k3 * q[1] - kw.x * w.y, k3 * q[2] - kw.x * w.z},
+              {k3 * q[1] - kw.x * w.y, d + (k3 * q[3] - kw.y * w.y), k3 * q[4] - kw.y * w.z},
+              {k3 * q[2] - kw.x * w.z, k3 * q[4] - kw.y * w.z, d + (k3 * q[5] - kw.z * w.z)}};
     C = C + ldm(o.Cs);
     stm(o.C, C);
     const m3 GI = ((-2.0) / 3 * o.R2) * add_diag(C, -o.A);
@@ -673,37 +676,47 @@ __device__ void update_body(Own &o, bool first, bool deform_only) {
     }
     const v3 nw = mul(inverse(GI), fast3(o.GL));
     stv(o.w, nw);
-    const v3 d = nw - w;
+    const v3 dn = nw - w;
     const bool same = nw.x == w.x && nw.y == w.y && nw.z == w.z;
-    o.converged = (same || dot(d, d) < 1e-18 * dot(w, w)) ? 1 : 0;
+    o.converged = (same || dot(dn, dn) < 1e-18 * dot(w, w)) ? 1 : 0;
 }
 
-// Sources of the pass-A tile rows. Only a delayed tide reads the velocities and tidal delay factors of the
-// bodies j: a CTA without one leaves those rows out of the copy (null source).
-__device__ __forceinline__ void tile_a_rows(const SysDev &S, const double *pub, bool need_v, const double *(&src)[TA_ROWS]) {
-    const int ld = S.ld;
+// Source planes of the tile rows, fixed for the launch. Only a delayed tide reads the velocities and tidal delay
+// factors of the bodies j: a CTA without one leaves those rows out. With one tile, the positions, GM and sR2 are still
+// in the tile from pass A when pass B comes (`reuse`).
+__device__ void tile_rows(Scratch &sc, bool need_v, bool reuse) {
     for (int c = 0; c < 3; ++c) {
-        src[TA_R_HI + c] = pub + (PUB_R_HI + c) * ld;
-        src[TA_R_LO + c] = pub + (PUB_R_LO + c) * ld;
-        src[TA_V_HI + c] = need_v ? pub + (PUB_V_HI + c) * ld : nullptr;
-        src[TA_V_LO + c] = need_v ? pub + (PUB_V_LO + c) * ld : nullptr;
+        sc.row_a[TA_R_HI + c] = PUB_R_HI + c;
+        sc.row_a[TA_R_LO + c] = PUB_R_LO + c;
+        sc.row_a[TA_V_HI + c] = need_v ? PUB_V_HI + c : -1;
+        sc.row_a[TA_V_LO + c] = need_v ? PUB_V_LO + c : -1;
+        sc.row_b[TB_R_HI + c] = reuse ? -1 : PUB_R_HI + c;
+        sc.row_b[TB_R_LO + c] = reuse ? -1 : PUB_R_LO + c;
+        sc.row_b[TB_NACC + c] = kRowAux + AUX_NACC + c;
+        sc.row_b[TB_BETA + c] = kRowAux + AUX_BETA + c;
+        sc.row_b[TB_GL + c] = PUB_GL + c;
     }
-    src[TA_GM] = pub + PUB_GM * ld;
-    src[TA_SR2] = S.cst + CST_SR2 * ld;
-    src[TA_TDF] = need_v ? S.cst + CST_TDF * ld : nullptr;
+    for (int q = 0; q < 9; ++q) sc.row_b[TB_CPOT + q] = kRowAux + AUX_CPOT + q;
+    sc.row_a[TA_GM] = PUB_GM;
+    sc.row_a[TA_SR2] = kRowCst + CST_SR2;
+    sc.row_a[TA_TDF] = need_v ? kRowCst + CST_TDF : -1;
+    sc.row_b[TB_GM] = reuse ? -1 : PUB_GM;
+    sc.row_b[TB_SR2] = reuse ? -1 : kRowCst + CST_SR2;
+    sc.row_b[TB_K] = kRowAux + AUX_K;
+    sc.row_b[TB_R2] = kRowCst + CST_R2;
+    sc.row_b[TB_LUM] = kRowCst + CST_LUM;
 }
 
 // Pair sums of pass A for the owned bodies in `mask` over all bodies j, by the first `nw` warps (tile
 // already staged (one tile, or whole at the wide stride); otherwise tiles are streamed, which needs the
-// whole CTA, nw == kWarps). Results land in own[b].sumA. One pair per iteration: a second pair chain in
+// whole CTA, nw == kWarps). Results land in sc.red[b]. One pair per iteration: a second pair chain in
 // flight per thread spills registers at the kernel's 128 per thread.
 template <Layout kL>
 __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int buf, Scratch &sc, TileState &ts,
                         double *tile, int nw, const int *first_all) {
     const int na = __popc(mask);
     if (na == 0) return true;
-    const int ld = S.ld, n = S.n, T = S.tile;
-    const double *pub = S.pub + (size_t)buf * PUB_NPLANES * ld;
+    const int n = S.n, T = S.tile;
     // Warp groups: the first sweep of a stage covers every owned body (`first_all`, weighted, fixed per
     // launch); a re-sweep covers the unconverged delayed tides, which all cost the same, so the nw warps are
     // split equally: slot a owns warps [ceil(a nw / na), ceil((a + 1) nw / na)), i.e. warp w is in slot
@@ -724,47 +737,29 @@ __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int bu
     int gw0, gw1;
     bounds(my_slot, gw0, gw1);
     const Group g{my_slot, (warp - gw0) * 32 + (int)(threadIdx.x & 31), (gw1 - gw0) * 32};
-    const Own &o = own[body_of(my_slot)];
-    double acc[13];
+    const int body = body_of(my_slot);
+    const Own &o = own[body];
+    double acc[kSumA];
 #pragma unroll
-    for (int c = 0; c < 13; ++c) acc[c] = 0;
+    for (int c = 0; c < kSumA; ++c) acc[c] = 0;
     #pragma unroll 1
     for (int j0 = 0; j0 < n; j0 += kL == kChunks ? T : n) {
         const int cnt = kL == kChunks ? min(T, n - j0) : n;
         if (kL == kChunks) {
-            const double *src[TA_ROWS];
-            tile_a_rows(S, pub, sc.has_delayed, src);
-            if (!load_tile(S, sc, ts, tile, kTileW, src, TA_ROWS, j0, cnt, cnt, TA_ROWS)) return false;
+            const double *pub = S.pub + (size_t)buf * PUB_NPLANES * S.ld;
+            if (!load_tile(S, sc, ts, tile, kTileW, pub, sc.row_a, TA_ROWS, j0, cnt, cnt, TA_ROWS)) return false;
         }
         const int self = o.idx - j0;
 #pragma unroll 1
         for (int jj = g.tid; jj < cnt; jj += g.size)
             if (jj != self) pair_a<kL == kWideA ? kWideW : kTileW>(o, tile, jj, acc);
     }
-    // sums over each body's warp group: a warp reduce-scatter, then the group's warps in ascending order
-    {
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double v[16];
-#pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = c < 13 ? acc[c] : 0.0;
-        const double r = warp_reduce_scatter16(v, lane);
-        if ((lane & 1) == 0 && (lane >> 1) < 13) sc.part[w][lane >> 1] = r;
-    }
+    // sums over each body's warp group
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) sc.wbody[w] = body;
+    warp_sums(acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], acc[6], acc[7], acc[8], acc[9], acc[10], 0.0, sc.part[w], kSumA);
     part_sync(nw * 32);
-    #pragma unroll 1
-    for (int idx = threadIdx.x; idx < na * 13; idx += nw * 32) {
-        const int slot = idx / 13, c = idx % 13;
-        int w0, w1;
-        bounds(slot, w0, w1);
-        double p[kWarps];   // every load first, then the sum in warp order
-#pragma unroll
-        for (int k = 0; k < kWarps; ++k) p[k] = w0 + k < w1 ? sc.part[w0 + k][c] : 0.0;
-        double sum = p[0];
-#pragma unroll
-        for (int k = 1; k < kWarps; ++k)
-            if (w0 + k < w1) sum += p[k];
-        own[body_of(slot)].sumA[c] = sum;
-    }
+    group_sums(sc, nb, mask, nw, false);
     part_sync(nw * 32);
     return true;
 }
@@ -780,8 +775,6 @@ struct ReactStage {
     }
     __device__ __forceinline__ double get(const double *p) const { return smem ? *p : __ldcg(p); }
 };
-constexpr int kRingTerms = kFieldMax * kRingPar * kRingDiskPar * 3;   // per-disk ring terms, [f][h][d][3]
-static_assert(kRingTerms <= kWideFree, "the ring terms must fit in the rows pass A leaves free at the wide stride");
 
 // Geopotential items (field body b, geopotential host slot e) on `nthr` threads (t = this
 // thread's index), G lanes per item: every item's lanes evaluate it together (gp_field_lanes on the
@@ -995,28 +988,24 @@ __device__ __forceinline__ bool pass_a(const SysDev &S, Own *own, int nb, int bu
         for (int c = 0; c < 3; ++c) f.r[c] = o.r[c];
     }
     if (kL != kChunks) {
-        const double *src[TA_ROWS];
-        tile_a_rows(S, pub, sc.has_delayed, src);
-        if (!load_tile(S, sc, ts, tile, kL == kWideA ? kWideW : kTileW, src, TA_ROWS, 0, S.n, S.n, TA_ROWS)) return false;
+        if (!load_tile(S, sc, ts, tile, kL == kWideA ? kWideW : kTileW, pub, sc.row_a, TA_ROWS, 0, S.n, S.n, TA_ROWS)) return false;
     } else {
         __syncthreads();
     }
     // The extended bodies' fields do not depend on the angular velocity, so they run beside the pass-A sweeps
     // (not with streaming tiles, which need every warp): the ring items on the last warp, the geopotential
-    // items (sc.ext_overlap) on the kExtWarps - 1 warps before it. With streaming tiles, and at the wide stride in a
-    // CTA that owns a delayed tide and could not hand them over, they run on every warp
-    // after the sweeps. The per-disk ring terms and, when they fit, the reactions are staged in the rows of
-    // the pass-A tile that pass A does not use.
+    // items (sc.ext_overlap) on the kExtWarps - 1 warps before it. With streaming tiles they run on every warp
+    // after the sweeps. When they fit, the reactions are staged in the rows of the tile that pass A does not use.
     const bool fields = !deform_only && S.n_ext > 0 && !sc.fields_away;
     const bool ring_side = fields && sc.ring_side;
     const bool gp_side = fields && sc.ext_overlap;
     const int max_iter = deform_only ? 1 : 4;   // MAX_ANGULAR_VELOCITY_ITER (mass.impl:74)
     const int nw = deform_only ? kWarps : sc.nw_a;
-    // (staged whole at the wide stride: the velocity rows beside the sweeps, anything after them)
-    const bool beside = kL == kWideA && sc.ext_overlap;
-    double *xa = tile + (beside ? TA_V_HI * kWideW : TA_ROWS * kTileW);
     const int nf = sc.nfb;
-    const ReactStage st{kRingTerms + nf * S.n_ext * 12 <= (beside ? kWideFree : (kTileRows - TA_ROWS) * kTileW) ? xa + kRingTerms : nullptr, nf};
+    double *ring_terms = tile + (size_t)kTileRows * kTileW;
+    double *stage = tile + (kL == kWideA ? TA_V_HI * kWideW : TA_ROWS * kTileW);
+    const int room = kL != kWideA ? (kTileRows - TA_ROWS) * kTileW : sc.has_delayed ? 0 : kWideFree;
+    const ReactStage st{nf * S.n_ext * 12 <= room ? stage : nullptr, nf};
     const int warp = threadIdx.x >> 5;
     if (warp < nw) {
         #pragma unroll 1
@@ -1030,7 +1019,7 @@ __device__ __forceinline__ bool pass_a(const SysDev &S, Own *own, int nb, int bu
             if (S.timers && threadIdx.x == 0) sc.t_phase[PH_A_COUNT] += 1;
             mark(S, sc, PH_A_SWEEP);   // thread 0 sits in a sweep warp
             // harmonics and angular velocity of the owned bodies: lane 0 of warp b updates body b
-            if (warp < nb && (threadIdx.x & 31) == 0 && !own[warp].converged) update_body(own[warp], it == 0, deform_only);
+            if (warp < nb && (threadIdx.x & 31) == 0 && !own[warp].converged) update_body(own[warp], sc.red[warp], it == 0, deform_only);
             part_sync(nw * 32);
             mark(S, sc, PH_A_UPDATE);
             int all = 1;
@@ -1063,7 +1052,7 @@ __device__ __forceinline__ bool pass_a(const SysDev &S, Own *own, int nb, int bu
         const bool gp_here = ph == 0 ? (gp_side && warp >= nw) : !gp_side;
         const int gp_lo = ph == 0 ? kWarps - kExtWarps : 0;
         const int gp_hi = (ph == 0 ? ring_side : ring_after) ? kWarps - 1 : kWarps;
-        if (ring_here) ext_ring(S, sc.fb, nf, buf, sc, st, xa);
+        if (ring_here) ext_ring(S, sc.fb, nf, buf, sc, st, ring_terms);
         else if (gp_here && warp >= gp_lo && warp < gp_hi) ext_gp(S, sc.fb, nf, buf, sc, st, gp_lo, gp_hi);
     }
     if (fields) {
@@ -1086,12 +1075,12 @@ __device__ __forceinline__ bool pass_a(const SysDev &S, Own *own, int nb, int bu
         for (int c = 0; c < 3; ++c) { o.dacc[c] = 0; o.dtq[c] = 0; o.gacc[c] = 0; }
         const int i = o.idx;
         double *aux = S.aux;
-        aux[AUX_PHI * ld + i] = o.phi;
+        aux[AUX_K * ld + i] = o.phi + 2 * o.beta2;
+        o.rad = o.rR2G4c / o.GM;
         for (int c = 0; c < 3; ++c) {
             aux[(AUX_NACC + c) * ld + i] = o.nacc[c];
             aux[(AUX_BETA + c) * ld + i] = o.beta[c];
         }
-        aux[AUX_BETA2 * ld + i] = o.beta2;
         for (int q = 0; q < 9; ++q) aux[(AUX_CPOT + q) * ld + i] = o.C[q];
         // a non-finite G*L was replaced by GI*w: republish it for pass B
         if (o.gl_fixed) publish_body(S, o, buf);
@@ -1104,26 +1093,38 @@ __device__ __forceinline__ bool pass_a(const SysDev &S, Own *own, int nb, int bu
 
 // ------------------------------------------------------------------ pass B: main force
 // Extremal pairs of the per-pair maxima (RungeKutta.cu:229-230; min_distance tracks 1/r, max_influence
-// GM/r^3). The sweep uses a 1-ulp reciprocal square root; the extremes are recomputed afterwards with
-// the reference's own expressions rr2 = 1/m, rr = sqrt(rr2) (mass.impl:84-89) from the tracked pair.
+// GM/r^3). The sweep uses an ulp-accurate reciprocal square root; the extremes are recomputed afterwards with
+// the reference's own expressions rr2 = 1/m, rr = sqrt(rr2) (mass.impl:84-89) from the body's pair. A NaN sticks
+// in the reference's maxima: the sweep's comparisons pass over it, one compare each instead of three, and a thread
+// whose force sums are NaN, which a NaN pair makes them, looks for the pair afterwards (nan_extremes).
 struct Extremes {
-    double m_min;           // smallest max(r^2, sR2_i + sR2_j): the largest 1/r
-    double tq, tq_m, tq_gm; // largest GM/r^3 seen (approximate), with its m and GM_j
+    double m_min, tq, tq_m, tq_gm;   // min softened r^2; max GM/r^3 with its pair
 };
-__device__ __forceinline__ void track(Extremes &x, double m, double tp_dg, double GMj) {
-    if (x.m_min == x.m_min) x.m_min = (m != m || m < x.m_min) ? m : x.m_min;   // NaN sticks
-    if (x.tq == x.tq) {
-        if (tp_dg != tp_dg) x.tq = tp_dg;
-        else if (tp_dg > x.tq) { x.tq = tp_dg; x.tq_m = m; x.tq_gm = GMj; }
+__device__ __noinline__ void nan_extremes(const Own &o, const double *T, int lo, int hi, int self, int step, Extremes &x) {
+    constexpr int ts = kTileW;
+    #pragma unroll 1
+    for (int j = lo; j < hi; j += step) {
+        if (j == self) continue;
+        v3 r = mk(sep_diff(T[(TB_R_HI + 0) * ts + j], T[(TB_R_LO + 0) * ts + j], o.r[0].hi, o.r[0].lo),
+                  sep_diff(T[(TB_R_HI + 1) * ts + j], T[(TB_R_LO + 1) * ts + j], o.r[1].hi, o.r[1].lo),
+                  sep_diff(T[(TB_R_HI + 2) * ts + j], T[(TB_R_LO + 2) * ts + j], o.r[2].hi, o.r[2].lo));
+        const double q = dot(r, r), sm = o.sR2 + T[TB_SR2 * ts + j];
+        const double m = (q < sm) ? sm : q, rr = inv_sqrt(m), g = (rr * rr) * (rr * T[TB_GM * ts + j]);
+        if (m != m) x.m_min = m;
+        if (g != g) x.tq = g;
     }
 }
 
 // One ordered pair of RELATIVITY, ROTATIONAL_TIDAL_DEFORMATION_NANTI_FORCE, LENSE_THIRRING and
-// RADIATION_PRESSURE (mass.impl:82-125, mass.cpp:147-155) into acc = {gaccel[3], daccel[3], dtorque[3]}.
-// IF / JF: body i / body j of the full class. For a point-like body the deformation matrix, G*L,
-// luminosity and receptance are all zero, so the terms they multiply are exactly zero and skipped.
-template <bool IF, bool JF>
-__device__ __forceinline__ void pair_b(const Own &o, const double *T, int j, double acc[9], Extremes &x) {
+// RADIATION_PRESSURE (mass.impl:82-125, mass.cpp:147-155) into acc = {gaccel[3], daccel[3], dtorque[3], sum c}.
+// The 1PN terms are grouped by the vector they multiply, r, a_Nj and b = beta_j - beta_i, and what does not depend
+// on j leaves the loop: with c = g (4 r.beta_i - 3 r.beta_j), the sum of c b is (sum c beta_j) - beta_i (sum c), and
+// the terms of i alone, (4 phi_i + beta_i^2) times the sum of g r, are the Newtonian sum of pass A; both are added
+// where the pass finishes its sums. Tile row TB_K holds phi_j + 2 beta_j^2.
+// fi / fj: body i / body j of the full class. For a point-like body the deformation matrix, G*L,
+// luminosity and receptance are all zero, so the terms they multiply are exactly zero and skipped. (One copy of the
+// code with two branches, which part no warp but the one at the end of the full class; four copies were fetched.)
+__device__ __forceinline__ void pair_b(const Own &o, const double *T, int j, bool fi, bool fj, double acc[kSumB], Extremes &x) {
     constexpr int ts = kTileW;
     v3 r = mk(sep_diff(T[(TB_R_HI + 0) * ts + j], T[(TB_R_LO + 0) * ts + j], o.r[0].hi, o.r[0].lo),
               sep_diff(T[(TB_R_HI + 1) * ts + j], T[(TB_R_LO + 1) * ts + j], o.r[1].hi, o.r[1].lo),
@@ -1131,31 +1132,34 @@ __device__ __forceinline__ void pair_b(const Own &o, const double *T, int j, dou
     const double GMj = T[TB_GM * ts + j];
     const double q = dot(r, r), sm = o.sR2 + T[TB_SR2 * ts + j];
     const double m = (q < sm) ? sm : q;
-    const double rr = rsqrt(m);
+    const double rr = inv_sqrt(m);
     const double rr2 = rr * rr;
-    const double rr3 = rr * rr2;
     const double tp_dphi = rr * GMj;
     const double tp_dg = rr2 * tp_dphi;
-    track(x, m, tp_dg, GMj);
-    v3 bj = mk(T[(TB_BETA + 0) * ts + j], T[(TB_BETA + 1) * ts + j], T[(TB_BETA + 2) * ts + j]);
-    v3 bi = ldv(o.beta);
-    double rbj = dot(r, bj);
+    if (m < x.m_min) x.m_min = m;
+    if (tp_dg > x.tq) { x.tq = tp_dg; x.tq_m = m; x.tq_gm = GMj; }
+    const v3 bj = mk(T[(TB_BETA + 0) * ts + j], T[(TB_BETA + 1) * ts + j], T[(TB_BETA + 2) * ts + j]);
+    const v3 bi = ldv(o.beta);
+    const v3 naj = mk(T[(TB_NACC + 0) * ts + j], T[(TB_NACC + 1) * ts + j], T[(TB_NACC + 2) * ts + j]);
+    const double rbj = dot(r, bj);
     double tp = rbj * rr;
     tp *= tp;
-    v3 naj = mk(T[(TB_NACC + 0) * ts + j], T[(TB_NACC + 1) * ts + j], T[(TB_NACC + 2) * ts + j]);
-    double delta1 = 4 * o.phi + T[TB_PHI * ts + j] + o.beta2 + 2 * T[TB_BETA2 * ts + j] - 4 * dot(bi, bj) +
-                    (dot(r, naj) - 3 * tp) / 2;
-    v3 b = bj - bi;
-    v3 g = (7 * tp_dphi / 2) * naj + (tp_dg * delta1) * r + (tp_dg * (rbj - dot(r, b) * 4)) * b;
-    acc[0] += g.x; acc[1] += g.y; acc[2] += g.z;
-    if (!IF && !JF) return;
+    const double w = tp_dg * (((T[TB_K * ts + j] - 4 * dot(bi, bj)) + 0.5 * dot(r, naj)) - 1.5 * tp);
+    const double c = tp_dg * (4 * dot(r, bi) - 3 * rbj);
+    const double h = 3.5 * tp_dphi;
+    acc[0] += h * naj.x; acc[1] += h * naj.y; acc[2] += h * naj.z;
+    acc[0] += w * r.x; acc[1] += w * r.y; acc[2] += w * r.z;
+    acc[0] += c * bj.x; acc[1] += c * bj.y; acc[2] += c * bj.z;
+    acc[9] += c;
+    if (!fi && !fj) return;
+    const v3 b = bj - bi;
     v3 da = mk(0, 0, 0), dt = mk(0, 0, 0);
-    const double rcr32 = 2 * GMj / kC * rr3;
-    if (IF) {
+    const double g5 = tp_dg * rr2, rcr32 = (2 / kC) * tp_dg;
+    if (fi) {
         // deformation of i, Lense-Thirring of i's spin, radiation received by i
         m3 Ci = ldm(o.C);
         v3 Cr = mul(Ci, r);
-        v3 dg = (GMj * rr3 * rr2 * o.R2) * ((dot(r, Cr) * 5 * rr2) * r - (Cr + Cr));
+        v3 dg = (g5 * o.R2) * ((dot(r, Cr) * 5 * rr2) * r - (Cr + Cr));
         da = dg;
         dt = cross(r, dg);
         v3 GL = fast3(o.GL);
@@ -1163,95 +1167,93 @@ __device__ __forceinline__ void pair_b(const Own &o, const double *T, int j, dou
         da -= rcr32 * (GLb - (3 * dot(GLb, r) * rr2) * r);
         dt -= rcr32 * cross(GL, cross(r, b));
     }
-    if (JF) {
+    if (fj) {
         // deformation of j (no reaction written to j: recomputed by j's owner), j's spin, j's light
         const double *Cjp = T + TB_CPOT * ts + j;
         m3 Cj = m3{mk(Cjp[0], Cjp[ts], Cjp[2 * ts]), mk(Cjp[3 * ts], Cjp[4 * ts], Cjp[5 * ts]),
                    mk(Cjp[6 * ts], Cjp[7 * ts], Cjp[8 * ts])};
         v3 Cjr = mul(Cj, r);
-        da += (GMj * rr3 * rr2 * T[TB_R2 * ts + j]) * ((dot(r, Cjr) * 5 * rr2) * r - (Cjr + Cjr));
+        da += (g5 * T[TB_R2 * ts + j]) * ((dot(r, Cjr) * 5 * rr2) * r - (Cjr + Cjr));
         v3 GLj = mk(T[(TB_GL + 0) * ts + j], T[(TB_GL + 1) * ts + j], T[(TB_GL + 2) * ts + j]);
         da += cross(rcr32 * (GLj - (3 * dot(GLj, r) * rr2) * r), b);
-        if (IF) da += (T[TB_LUM * ts + j] * o.rR2G4c * rr3 / o.GM) * r;
+        if (fi) da += (T[TB_LUM * ts + j] * o.rad * (rr * rr2)) * r;
     }
     acc[3] += da.x; acc[4] += da.y; acc[5] += da.z;
     acc[6] += dt.x; acc[7] += dt.y; acc[8] += dt.z;
-}
-
-template <bool IF, bool JF>
-__device__ __forceinline__ void sweep_b_range(const Own &o, const double *tile, int lo, int hi, int self,
-                                              const Group &g, double acc[9], Extremes &x) {
-#pragma unroll 1
-    for (int jj = lo + g.tid; jj < hi; jj += g.size)
-        if (jj != self) pair_b<IF, JF>(o, tile, jj, acc, x);
 }
 
 template <Layout kL>
 __device__ __forceinline__ bool pass_b(const SysDev &S, Own *own, int nb, int buf, Scratch &sc, TileState &ts, double *tile) {
     const int ld = S.ld, n = S.n, T = S.tile;
     const double *pub = S.pub + (size_t)buf * PUB_NPLANES * ld;
-    const double *aux = S.aux, *cst = S.cst;
     const int nwb = sc.nw_b;
     const bool sweeper = (threadIdx.x >> 5) < nwb;
     const Group g = group_of(sc.split_b, nb);
     const Own &o = own[g.slot];
-    double acc[9];
+    double acc[kSumB];
 #pragma unroll
-    for (int c = 0; c < 9; ++c) acc[c] = 0;
+    for (int c = 0; c < kSumB; ++c) acc[c] = 0;
     Extremes x{__longlong_as_double(0x7ff0000000000000ll), 0.0, 0.0, 0.0};   // m_min = +inf
     #pragma unroll 1
     for (int j0 = 0; j0 < n; j0 += kL == kOneTile ? n : T) {
         const int cnt = kL == kOneTile ? n : min(T, n - j0);
         const int cnt_full = max(0, min(cnt, S.n_full - j0));
-        // rows every body needs, then rows only full-class bodies need; with one tile the positions, GM
-        // and sR2 are still in the tile from pass A of this stage (`reuse`)
-        constexpr bool reuse = kL == kOneTile;
-        const double *src[TB_ROWS] = {
-            reuse ? nullptr : pub + (PUB_R_HI + 0) * ld, reuse ? nullptr : pub + (PUB_R_HI + 1) * ld,
-            reuse ? nullptr : pub + (PUB_R_HI + 2) * ld, reuse ? nullptr : pub + (PUB_R_LO + 0) * ld,
-            reuse ? nullptr : pub + (PUB_R_LO + 1) * ld, reuse ? nullptr : pub + (PUB_R_LO + 2) * ld,
-            aux + (AUX_NACC + 0) * ld, aux + (AUX_NACC + 1) * ld, aux + (AUX_NACC + 2) * ld,
-            aux + (AUX_BETA + 0) * ld, aux + (AUX_BETA + 1) * ld, aux + (AUX_BETA + 2) * ld,
-            reuse ? nullptr : pub + PUB_GM * ld, reuse ? nullptr : cst + CST_SR2 * ld,
-            aux + AUX_PHI * ld, aux + AUX_BETA2 * ld,
-            pub + (PUB_GL + 0) * ld, pub + (PUB_GL + 1) * ld, pub + (PUB_GL + 2) * ld,
-            aux + (AUX_CPOT + 0) * ld, aux + (AUX_CPOT + 1) * ld, aux + (AUX_CPOT + 2) * ld,
-            aux + (AUX_CPOT + 3) * ld, aux + (AUX_CPOT + 4) * ld, aux + (AUX_CPOT + 5) * ld,
-            aux + (AUX_CPOT + 6) * ld, aux + (AUX_CPOT + 7) * ld, aux + (AUX_CPOT + 8) * ld,
-            cst + CST_R2 * ld, cst + CST_LUM * ld};
-        if (!load_tile(S, sc, ts, tile, kTileW, src, TB_ROWS, j0, cnt, cnt_full, kTileBFullRows)) return false;
+        // rows every body needs, then rows only full-class bodies need
+        if (!load_tile(S, sc, ts, tile, kTileW, pub, sc.row_b, TB_ROWS, j0, cnt, cnt_full, kTileBFullRows)) return false;
         const int self = o.idx - j0;
         if (!sweeper) continue;
-        if (o.full) {
-            sweep_b_range<true, true>(o, tile, 0, cnt_full, self, g, acc, x);
-            sweep_b_range<true, false>(o, tile, cnt_full, cnt, self, g, acc, x);
-        } else {
-            sweep_b_range<false, true>(o, tile, 0, cnt_full, self, g, acc, x);
-            sweep_b_range<false, false>(o, tile, cnt_full, cnt, self, g, acc, x);
-        }
+#pragma unroll 1
+        for (int jj = g.tid; jj < cnt; jj += g.size)
+            if (jj != self) pair_b(o, tile, jj, o.full, jj < cnt_full, acc, x);
+        const double s3 = acc[0] + acc[1] + acc[2];
+        if (s3 != s3) nan_extremes(o, tile, g.tid, cnt, self, g.size, x);
     }
-    __shared__ double red[kOwnMax][16];
     if (sweeper) {
-        // exact extremes with the reference's expressions
-        double red_in[11];
-#pragma unroll
-        for (int c = 0; c < 9; ++c) red_in[c] = acc[c];
-        {
-            const double rr2 = 1.0 / x.m_min;
-            red_in[9] = sqrt(rr2);                                // +inf -> 0 when no pair was seen
-            if (x.tq != x.tq) red_in[10] = x.tq;
-            else if (x.tq > 0) {
-                const double r2 = 1.0 / x.tq_m;
-                red_in[10] = r2 * (sqrt(r2) * x.tq_gm);
-            } else red_in[10] = 0.0;
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double *row = sc.part[w];
+        {   // the warp's extremes: their keys, and of the lowest lane with the largest GM/r^3 the pair's m and GM
+            const unsigned all = 0xffffffffu;
+            const unsigned long long km = x.m_min != x.m_min ? kNanKey : kInfBits - key_of(x.m_min), kt = key_of(x.tq);
+            const unsigned mh = __reduce_max_sync(all, (unsigned)(km >> 32)), th = __reduce_max_sync(all, (unsigned)(kt >> 32));
+            const unsigned ml = __reduce_max_sync(all, (unsigned)(km >> 32) == mh ? (unsigned)km : 0u);
+            const unsigned tl = __reduce_max_sync(all, (unsigned)(kt >> 32) == th ? (unsigned)kt : 0u);
+            const unsigned win = __ballot_sync(all, kt == ((unsigned long long)th << 32 | tl));
+            if (lane == __ffs(win) - 1) {
+                row[kSumB] = __longlong_as_double((long long)((unsigned long long)mh << 32 | ml));
+                row[kSumB + 1] = __longlong_as_double((long long)kt);
+                row[12] = x.tq_m;
+                row[13] = x.tq_gm;
+                sc.wbody[w] = g.slot;
+            }
         }
-        group_reduce<11>(red_in, sc.split_b, nb, nwb, sc, red, 9);
+        warp_sums(acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], acc[6], acc[7], acc[8], acc[9], 0.0, 0.0, row, kSumB);
+        part_sync(nwb * 32);
+        group_sums(sc, nb, ~0u, nwb, true);
+        part_sync(nwb * 32);
         if (threadIdx.x < nb) {
             Own &ob = own[threadIdx.x];
-            const double *rr = red[threadIdx.x];
-            for (int c = 0; c < 3; ++c) { ob.gacc[c] = rr[c]; ob.dacc[c] = rr[3 + c]; ob.dtq[c] = rr[6 + c]; }
-            checked_maximize(ob.mind, rr[9]);
-            checked_maximize(ob.maxi, rr[10]);
+            const double *rr = sc.red[threadIdx.x];
+            const double k = (4 * ob.phi + ob.beta2) * (kC * kC);   // (phi and the Newtonian sum are over c^2 here)
+            for (int c = 0; c < 3; ++c) {
+                ob.gacc[c] = rr[c] + (k * ob.nacc[c] - rr[9] * ob.beta[c]);
+                ob.dacc[c] = rr[3 + c];
+                ob.dtq[c] = rr[6 + c];
+            }
+        } else if (threadIdx.x >= 32 && threadIdx.x < 32 + nb) {   // the maxima, with the reference's expressions
+            Own &ob = own[threadIdx.x - 32];
+            const double *rr = sc.red[threadIdx.x - 32];
+            const unsigned long long km = (unsigned long long)__double_as_longlong(rr[kSumB]);
+            const unsigned long long kt = (unsigned long long)__double_as_longlong(rr[kSumB + 1]);
+            const double nan = __longlong_as_double(0x7ff8000000000000ll);
+            // (no pair: m = +inf, 1/r = 0)
+            checked_maximize(ob.mind, km == kNanKey ? nan : sqrt(1.0 / __longlong_as_double((long long)(kInfBits - km))));
+            double t = 0;
+            if (kt == kNanKey) t = nan;
+            else if (kt) {
+                const double r2 = 1.0 / rr[12];
+                t = r2 * (sqrt(r2) * rr[13]);
+            }
+            checked_maximize(ob.maxi, t);
         }
     } else {
         // the last warp: reactions of the owned extended bodies, the sum over all CTAs of their shares
@@ -1510,7 +1512,7 @@ __device__ void rk_stage(const SysDev &S, Own *own, int nb, int s, long long i_s
             o.r[c] = dd_add(o.r0[c], dd_mul(ddt, o.accv[k - 1][c]));
             o.v[c] = dd_add(o.v0[c], dd_make(dt * o.acca[k - 1][c]));
             o.GL[c] = dd_add(o.GL0[c], dd_make(dt * o.acct[k - 1][c]));
-            const double wc = o.accw[k - 1][c] * (1.0 / dt_k);   // xi.w /= dt_k (vec_t.h:197-203)
+            const double wc = o.accw[k - 1][c] * c_rdtk[k];   // xi.w /= dt_k (vec_t.h:197-203)
             o.wnew[c] = wc;
             o.dw[c] = (2.0 / 3) * (wc - o.w0[c]);
         }
@@ -1541,7 +1543,7 @@ __device__ void field_handoff(const SysDev &S, const StepParams &P, const Own *o
     int *cta_del = reinterpret_cast<int *>(tile);   // [grid]: the CTA owns a delayed tide
     int *cta_nb = cta_del + kPlanCtas;              // [grid]: bodies of the CTA
     const bool possible = P.mode != MODE_DEFORM && S.n_ext > 0 && kL != kChunks && gridDim.x <= kPlanCtas &&
-                          kRingTerms + kFieldMax * S.n_ext * 12 <= (kL == kWideA ? kWideFree : (kTileRows - TA_ROWS) * kTileW);
+                          kFieldMax * S.n_ext * 12 <= (kL == kWideA ? kWideFree : (kTileRows - TA_ROWS) * kTileW);
     const int n = S.n;
     for (int c = threadIdx.x; c < (int)gridDim.x; c += blockDim.x) {
         int d = 0, k = 0;
@@ -1655,7 +1657,8 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams 
         bool delayed = false;
         for (int b = 0; b < nb; ++b) delayed |= own[b].kind == 2;
         sc.has_delayed = delayed;
-        const bool side = P.mode != MODE_DEFORM && S.n_ext > 0 && (kL == kOneTile || (kL == kWideA && !delayed)) && !sc.fields_away;
+        tile_rows(sc, delayed, kL == kOneTile);
+        const bool side = P.mode != MODE_DEFORM && S.n_ext > 0 && kL != kChunks && !sc.fields_away;
         sc.ext_overlap = side;
         sc.ring_side = side && sc.n_ring_e > 0;
         sc.nw_a = sc.ext_overlap ? kWarps - kExtWarps : sc.ring_side ? kWarps - 1 : kWarps;
@@ -1725,7 +1728,7 @@ static const void *const kStepKernels[] = {(const void *)step_kernel<kOneTile>, 
 
 size_t step_fixed_smem_bytes() { return kFixedSmem; }
 // the tile is always allocated at its full stride; `tile` (bodies staged per chunk) does not change the size
-size_t step_smem_bytes(int tile) { (void)tile; return kFixedSmem + (size_t)kTileRows * kTileW * sizeof(double); }
+size_t step_smem_bytes(int tile) { (void)tile; return kFixedSmem + ((size_t)kTileRows * kTileW + kRingTerms) * sizeof(double); }
 
 // Largest tile (bodies, multiple of kPad): the tile's stride.
 int max_tile() { return kTileW; }
@@ -1744,6 +1747,9 @@ cudaError_t upload_constants(int device) {
     cudaError_t e = cudaMemcpyToSymbol(c_rk_hi, hi, sizeof(hi));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_rk_lo, lo, sizeof(lo));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_dtk, dtk, sizeof(dtk));
+    double rdtk[kStages + 1] = {};
+    for (int k = 1; k <= kStages; ++k) rdtk[k] = 1.0 / dtk[k];
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_rdtk, rdtk, sizeof(rdtk));
     for (int l = 0; l < 3 && e == cudaSuccess; ++l)
         e = cudaFuncSetAttribute(kStepKernels[l], cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
     if (e == cudaSuccess && device >= 0 && device < 64) g_consts_ready[device].store(true, std::memory_order_release);

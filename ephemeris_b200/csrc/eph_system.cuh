@@ -7,7 +7,7 @@
 //     velocity (double-double, 6), G*L/GM rounded to double (3), GM (1), body frame s rounded to
 //     double (9, geopotential hosts) and ring frame (9, ring hosts). Written by the owning CTA at the
 //     end of a stage, read by every CTA in the next one.
-//   * pass-A outputs aux[AUX_NPLANES][ld]: phi/c^2, naccel/c^2 (3), beta (3), beta^2, C_potential (9).
+//   * pass-A outputs aux[AUX_NPLANES][ld]: phi/c^2 + 2 beta^2, naccel/c^2 (3), beta (3), C_potential (9).
 //   * constants cst[CST_NPLANES][ld]: sR2, tide_delay_factor, R^2, luminosity, R, model indices.
 //   * extended-body reactions react[n_ext][ld][2][6]: for host e and body i, -GM_i an and -GM_i (r x an)
 //     of host e's geopotential (slot 0) and ring (slot 1) field at body i (written in pass A by i's
@@ -40,7 +40,7 @@ enum PubPlane {
     PUB_FRAME = 16, PUB_RFRAME = 25, PUB_NPLANES = 34
 };
 // pass-A output planes
-enum AuxPlane { AUX_PHI = 0, AUX_NACC = 1, AUX_BETA = 4, AUX_BETA2 = 7, AUX_CPOT = 8, AUX_NPLANES = 17 };
+enum AuxPlane { AUX_K = 0, AUX_NACC = 1, AUX_BETA = 4, AUX_CPOT = 7, AUX_NPLANES = 16 };
 // constant planes
 enum ConstPlane { CST_SR2 = 0, CST_TDF = 1, CST_R2 = 2, CST_LUM = 3, CST_R = 4, CST_GP = 5, CST_RING = 6,
                   CST_NPLANES = 7 };
@@ -51,9 +51,9 @@ enum TileA { TA_R_HI = 0, TA_R_LO = 3, TA_V_HI = 6, TA_V_LO = 9, TA_GM = 12, TA_
 // bodies of the full class need, staged for the full-class prefix of the tile only. Positions, GM and sR2
 // sit in the rows pass A staged them in: when the whole system fits one tile they are not copied again.
 enum TileB { TB_R_HI = TA_R_HI, TB_R_LO = TA_R_LO, TB_NACC = 6, TB_BETA = 9, TB_GM = TA_GM, TB_SR2 = TA_SR2,
-             TB_PHI = 14, TB_BETA2 = 15, TB_GL = 16, TB_CPOT = 19, TB_R2 = 28, TB_LUM = 29, TB_ROWS = 30 };
+             TB_K = 14, TB_GL = 15, TB_CPOT = 18, TB_R2 = 27, TB_LUM = 28, TB_ROWS = 29 };
 constexpr int kTileBFullRows = TB_GL;
-constexpr int kTileRows = TB_ROWS;
+constexpr int kTileRows = TB_ROWS + 1;   // twice the rows of pass A
 
 // Device bodies are ordered by class: the first n_full "full" bodies (any of tidal / rotational
 // deformation, static harmonics, spin, luminosity, radiation receptance, geopotential or ring), then the

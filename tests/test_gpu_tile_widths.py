@@ -34,3 +34,25 @@ def test_tile_widths(tmp_path, oracle, n, step):
         c.integrate(dt, 1)
         assert position_error(c.download(), oracle.integrate(pl, om, dt, 1)[0]) <= 1e-12
     c.close()
+
+
+def test_nan_sticks_in_the_maxima(oracle):
+    """One body without a position: the maxima of every body are NaN, those of a pair the comparisons must not pass over."""
+    from ephemeris_b200 import PLANES, Context
+    from oracle.pyoracle import Models
+    from tests.test_gpu_batch_shapes import _system
+    pl = _system(40, seed=3)
+    rows = [PLANES["MIN_DISTANCE"], PLANES["MAX_INFLUENCE"]]
+    for bad in (None, 33):
+        p = pl.copy()
+        if bad is not None:
+            p[PLANES["R_HI"], bad] = np.nan
+        c = Context(0)
+        c.upload(p)
+        c.accel()
+        out = c.download()[rows]
+        c.close()
+        ref = oracle.accel(p, Models.empty())[rows]
+        assert np.array_equal(np.isnan(out), np.isnan(ref))
+        assert np.isnan(out).all() == (bad is not None)
+        assert np.allclose(out, ref, rtol=1e-13, atol=0, equal_nan=True)

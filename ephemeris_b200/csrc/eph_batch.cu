@@ -356,7 +356,8 @@ __device__ __forceinline__ void send_all(double *p, int count, int peers, int ra
 // many CTAs per system as the batch needs to finish together. Stage times on one B200, one system alone, before
 // (one thread per body, power-of-two lane groups, at most 4 CTAs) and now: 8 bodies 6.5 / 2.9 us, 33 9.3 / 4.6,
 // 95 28.7 / 7.8, 128 16.6 / 7.5, 300 80.3 / 13.3 us.
-template <bool MIXED>
+// kEval: one evaluation of the accelerations of the loaded state (eph_accel) instead of steps.
+template <bool MIXED, bool kEval = false>
 __device__ void integrate_system(const BatchSys &Y, const RkTable &rk, double *smem, int peers, int rank) {
     const int n = Y.n;
     const int lo = (int)((long long)rank * n / peers);
@@ -408,6 +409,7 @@ __device__ void integrate_system(const BatchSys &Y, const RkTable &rk, double *s
         own_row(V, OR_DGM, b) = PLV(EPH_P_DGM, i);
         own_row(V, OR_M, b) = __longlong_as_double(0x7ff0000000000000ll);   // msystem::integrate resets the
         own_row(V, OR_MAXI, b) = 0.0;                                         // maxima (mass.cpp:406)
+        if (kEval) continue;
         // the loaded auxiliaries are f_0 of the first step (RungeKutta.impl:110-116)
         const v3 fa = (mk(PLV(EPH_P_GACCEL, i), PLV(EPH_P_GACCEL + 1, i), PLV(EPH_P_GACCEL + 2, i)) +
                        mk(PLV(EPH_P_DACCEL, i), PLV(EPH_P_DACCEL + 1, i), PLV(EPH_P_DACCEL + 2, i))) +
@@ -420,74 +422,76 @@ __device__ void integrate_system(const BatchSys &Y, const RkTable &rk, double *s
     const double dt = Y.dt;
     int buf = 0;   // parity of the state records in use
 #pragma unroll 1
-    for (long long step = 0; step < Y.n_step; ++step) {
+    for (long long step = 0; step < (kEval ? 1 : Y.n_step); ++step) {
 #pragma unroll 1
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = kEval ? kStages - 1 : 0; s < kStages; ++s) {
             const int k = s + 1;
             const double t = Y.t_eph + dt * (b_dtk[k] + (double)step);
-            const bool last = k == kStages && step + 1 == Y.n_step;
-            double *A = V.A[buf ^ 1];
-            // At s == 0 x0 = x (RungeKutta.impl:113-121). Then the state of stage k (RungeKutta.impl:148-186):
-            // r = r0 + dt (c_k v0 + dt sum_l Abar_kl f_l), the sums in double-double, v = v0 + dt sum_l a_kl f_l.
+            const bool last = kEval || (k == kStages && step + 1 == Y.n_step);
+            double *A = V.A[kEval ? buf : buf ^ 1];
+            if (!kEval) {
+                // At s == 0 x0 = x (RungeKutta.impl:113-121). Then the state of stage k (RungeKutta.impl:148-186):
+                // r = r0 + dt (c_k v0 + dt sum_l Abar_kl f_l), the sums in double-double, v = v0 + dt sum_l a_kl f_l.
 #pragma unroll 1
-            for (int idx = threadIdx.x; idx < 3 * cnt; idx += blockDim.x) {
-                const int b = idx / 3, c = idx - 3 * b, i = lo + b, ld = V.ld;
-                double *x0 = V.store + (size_t)(3 * kStages + c) * ld + b;
-                dd r0, v0;
-                if (s == 0) {
-                    const double *a = V.A[buf] + (size_t)i * kRecA;
-                    r0 = dd{a[RA_R_HI + c], a[RA_R_LO + c]};
-                    v0 = dd{own_row(V, OR_V_HI + c, b), own_row(V, OR_V_LO + c, b)};
-                    x0[0] = r0.hi;
-                    x0[3 * ld] = r0.lo;
-                    x0[6 * ld] = v0.hi;
-                    x0[9 * ld] = v0.lo;
-                } else {
-                    r0 = dd{x0[0], x0[3 * ld]};
-                    v0 = dd{x0[6 * ld], x0[9 * ld]};
-                }
-                // r0 + dt c_k v0 does not wait for the sum
-                const dd rv = dd_add(r0, dd_mul(dd_make(dt), dd_mul(dd{b_ck_hi[k], b_ck_lo[k]}, v0)));
-                // sum_l Abar_kl f_l as a compensated dot product (Ogita, Rump and Oishi 2005, Dot2: the result of
-                // twice the working precision): one dependent addition per term instead of a double-double one
-                double s1 = 0, e1 = 0, s2 = 0;
-                const double *f = V.store + c * ld + b;
-                const int row = k * (k - 1) / 2;
+                for (int idx = threadIdx.x; idx < 3 * cnt; idx += blockDim.x) {
+                    const int b = idx / 3, c = idx - 3 * b, i = lo + b, ld = V.ld;
+                    double *x0 = V.store + (size_t)(3 * kStages + c) * ld + b;
+                    dd r0, v0;
+                    if (s == 0) {
+                        const double *a = V.A[buf] + (size_t)i * kRecA;
+                        r0 = dd{a[RA_R_HI + c], a[RA_R_LO + c]};
+                        v0 = dd{own_row(V, OR_V_HI + c, b), own_row(V, OR_V_LO + c, b)};
+                        x0[0] = r0.hi;
+                        x0[3 * ld] = r0.lo;
+                        x0[6 * ld] = v0.hi;
+                        x0[9 * ld] = v0.lo;
+                    } else {
+                        r0 = dd{x0[0], x0[3 * ld]};
+                        v0 = dd{x0[6 * ld], x0[9 * ld]};
+                    }
+                    // r0 + dt c_k v0 does not wait for the sum
+                    const dd rv = dd_add(r0, dd_mul(dd_make(dt), dd_mul(dd{b_ck_hi[k], b_ck_lo[k]}, v0)));
+                    // sum_l Abar_kl f_l as a compensated dot product (Ogita, Rump and Oishi 2005, Dot2: the result of
+                    // twice the working precision): one dependent addition per term instead of a double-double one
+                    double s1 = 0, e1 = 0, s2 = 0;
+                    const double *f = V.store + c * ld + b;
+                    const int row = k * (k - 1) / 2;
 #pragma unroll 4
-                for (int l = 0; l < k; ++l) {
-                    const double2 ab = rk.ab[row + l];
-                    const double fl = f[3 * l * ld], h = ab.x;
-                    const double p = __dmul_rn(h, fl), pe = __fma_rn(rk.lo[row + l], fl, __fma_rn(h, fl, -p));
-                    double sum, se;
-                    two_sum(s1, p, sum, se);
-                    s1 = sum;
-                    e1 = __dadd_rn(e1, __dadd_rn(se, pe));
-                    s2 = __dadd_rn(s2, __dmul_rn(ab.y, fl));
+                    for (int l = 0; l < k; ++l) {
+                        const double2 ab = rk.ab[row + l];
+                        const double fl = f[3 * l * ld], h = ab.x;
+                        const double p = __dmul_rn(h, fl), pe = __fma_rn(rk.lo[row + l], fl, __fma_rn(h, fl, -p));
+                        double sum, se;
+                        two_sum(s1, p, sum, se);
+                        s1 = sum;
+                        e1 = __dadd_rn(e1, __dadd_rn(se, pe));
+                        s2 = __dadd_rn(s2, __dmul_rn(ab.y, fl));
+                    }
+                    dd sf;
+                    two_sum_quick(s1, e1, sf.hi, sf.lo);
+                    const dd r = dd_add(rv, dd_mul(dd_make(dt), dd_mul(dd_make(dt), sf)));
+                    const dd v = dd_add(v0, dd_make(dt * s2));
+                    double *a = A + (size_t)i * kRecA;
+                    a[RA_R_HI + c] = r.hi;
+                    a[RA_R_LO + c] = r.lo;
+                    own_row(V, OR_V_HI + c, b) = v.hi;
+                    own_row(V, OR_V_LO + c, b) = v.lo;
+                    if (c == 0) {
+                        const double gm = own_row(V, OR_GM0, b) + own_row(V, OR_DGM, b) * t;
+                        a[RA_GM] = gm;
+                    }
                 }
-                dd sf;
-                two_sum_quick(s1, e1, sf.hi, sf.lo);
-                const dd r = dd_add(rv, dd_mul(dd_make(dt), dd_mul(dd_make(dt), sf)));
-                const dd v = dd_add(v0, dd_make(dt * s2));
-                double *a = A + (size_t)i * kRecA;
-                a[RA_R_HI + c] = r.hi;
-                a[RA_R_LO + c] = r.lo;
-                own_row(V, OR_V_HI + c, b) = v.hi;
-                own_row(V, OR_V_LO + c, b) = v.lo;
-                if (c == 0) {
-                    const double gm = own_row(V, OR_GM0, b) + own_row(V, OR_DGM, b) * t;
-                    a[RA_GM] = gm;
+                if (k == kStages)
+                    for (int b = threadIdx.x; b < cnt; b += blockDim.x) orthogonalize_frame(pl, n, lo + b);
+                buf ^= 1;
+                if (peers > 1) {
+                    __syncthreads();
+                    send_all(A + (size_t)lo * kRecA, cnt * (kRecA / 2), peers, rank);
                 }
+                // The state records alternate between two arrays when a cluster shares the system: a peer that is
+                // still in the previous stage's pass B reads the other one, so one barrier per exchange is enough
+                sync();
             }
-            if (k == kStages)
-                for (int b = threadIdx.x; b < cnt; b += blockDim.x) orthogonalize_frame(pl, n, lo + b);
-            buf ^= 1;
-            if (peers > 1) {
-                __syncthreads();
-                send_all(A + (size_t)lo * kRecA, cnt * (kRecA / 2), peers, rank);
-            }
-            // The state records alternate between two arrays when a cluster shares the system: a peer that is
-            // still in the previous stage's pass B reads the other one, so one barrier per exchange is enough
-            sync();
             // pass A (DAMPED_TIDAL_DEFORMATION_MATRIX_NK2, mass.impl:38-46), then PREPARE_RELATIVITY
             // (mass.impl:76-80), one thread per (body, value)
             for_units([&](int i, int j0, int j1, double *part) {
@@ -652,12 +656,14 @@ __global__ void __launch_bounds__(kBThreads, 2)
 }
 
 constexpr size_t kBMaxSmem = 227 * 1024 - sizeof(RkTable) - 256;
-// One system on the CTAs of one cluster.
+// One system on the CTAs of one cluster: its steps, or one evaluation of its accelerations (eph_accel of 33 bodies,
+// with the read-back: 73 -> 45 us; of 300: 109 -> 78 us).
+template <bool kEval>
 __global__ void __launch_bounds__(kBThreads, 2) point_kernel(BatchSys Y, int peers) {
     extern __shared__ __align__(16) double bsm[];
     __shared__ RkTable rk;
-    load_table(rk);
-    integrate_system<false>(Y, rk, bsm, peers, peers > 1 ? (int)cg::this_cluster().block_rank() : 0);
+    if (!kEval) load_table(rk);
+    integrate_system<false, kEval>(Y, rk, bsm, peers, peers > 1 ? (int)cg::this_cluster().block_rank() : 0);
     if (peers > 1) cg::this_cluster().sync();   // no CTA leaves while a peer may still store to it
 }
 
@@ -740,8 +746,10 @@ cudaError_t batch_setup(int device) {
     // clusters of 16 CTAs: twice the portable size
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ensemble_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ensemble_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(point_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(point_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBMaxSmem);
+    for (auto k : {point_kernel<false>, point_kernel<true>}) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBMaxSmem);
+    }
     if (e == cudaSuccess && device >= 0 && device < 64) g_batch_ready[device].store(true, std::memory_order_release);
     return e;
 }
@@ -752,7 +760,7 @@ cudaError_t batch_setup(int device) {
 // Scratch a context keeps for it (doubles).
 size_t point_scratch_doubles(int n) { return (size_t)kStore * n; }
 // Launches n_step steps of dt of a system of point-like bodies on `stream`, as the step kernel of eph_step.cu would
-// integrate it (accumulate: eph_rk12's maxima, else eph_integrate's).
+// integrate it (accumulate: eph_rk12's maxima, else eph_integrate's); n_step 0: one evaluation of its accelerations.
 cudaError_t launch_point_system(int device, cudaStream_t stream, double *planes, int n, double dt, long long n_step, double t_eph,
                                 int accumulate, double *scratch) {
     cudaError_t e = batch_setup(device);
@@ -785,7 +793,7 @@ cudaError_t launch_point_system(int device, cudaStream_t stream, double *planes,
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, point_kernel, Y, peers);
+    return n_step ? cudaLaunchKernelEx(&cfg, point_kernel<false>, Y, peers) : cudaLaunchKernelEx(&cfg, point_kernel<true>, Y, peers);
 }
 }  // namespace eph
 

@@ -43,6 +43,8 @@ struct eph_ctx {
     int ld = 0, tile = 0;                // plane stride (n rounded up to kPad), bodies per smem tile
     int n_full = 0;                      // full-class bodies (device order)
     bool point_ok = false;               // a system of ordinary point-like bodies (point_system_ok)
+    bool point_accel_ok = false;         // and no oblateness change is loaded: so is one evaluation of it
+    bool ran_point = false;              // the latest launch was of the point-mass kernel, which has no status
     double *d_point = nullptr;           // scratch of launch_point_system
     size_t point_cap = 0;                // its size (doubles)
     int *d_orig = nullptr;               // [n] device order -> caller order
@@ -212,6 +214,8 @@ static int prepare_constants(eph_ctx *ctx, const double *h_planes) {
     }
     ctx->h_orig = orig;
     ctx->point_ok = point_system_ok(h_planes, n, ctx->n_full);
+    ctx->point_accel_ok = ctx->point_ok && std::all_of(h_planes + (size_t)EPH_P_EXJ2 * n, h_planes + (size_t)(EPH_P_EXJ2 + 1) * n,
+                                                       [](double x) { return x == 0; });
     if ((int)ext.size() > kMaxExt) return fail(ctx, EPH_ERR_ARG, "too many bodies with geopotential or ring models");
     ctx->n_ext = (int)ext.size();
     cudaError_t e = cudaMemcpy(ctx->d_cst, cst.data(), cst.size() * sizeof(double), cudaMemcpyHostToDevice);
@@ -343,7 +347,9 @@ int eph_device_planes(eph_ctx *ctx, double **d_planes) {
 static int launch(eph_ctx *ctx, const StepParams &P) {
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     if (!ctx->n) return fail(ctx, EPH_ERR_STATE, "no system uploaded");
-    if (P.mode == MODE_INTEGRATE && ctx->point_ok && !ctx->d_traj && !ctx->d_timers && ctx->req_grid == 0 && ctx->req_per_cta == 0) {
+    ctx->ran_point = false;
+    if (((P.mode == MODE_INTEGRATE && ctx->point_ok) || (P.mode == MODE_ACCEL && ctx->point_accel_ok && ctx->point_ok)) &&
+        !ctx->stall_barrier && !ctx->d_traj && !ctx->d_timers && ctx->req_grid == 0 && ctx->req_per_cta == 0) {
         const size_t need = point_scratch_doubles(ctx->n);
         if (need > ctx->point_cap) {
             if (ctx->d_point) cudaFree(ctx->d_point);
@@ -352,9 +358,9 @@ static int launch(eph_ctx *ctx, const StepParams &P) {
             CK(cudaMalloc(&ctx->d_point, need * sizeof(double)), "cudaMalloc(point system)");
             ctx->point_cap = need;
         }
-        CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "reset status");
-        CK(launch_point_system(ctx->device, ctx->stream, ctx->d_planes, ctx->n, P.dt, P.n_step, P.t_eph, !P.reset_minmax,
-                               ctx->d_point), "launch point-mass kernel");
+        CK(launch_point_system(ctx->device, ctx->stream, ctx->d_planes, ctx->n, P.dt, P.mode == MODE_ACCEL ? 0 : P.n_step, P.t_eph,
+                               !P.reset_minmax, ctx->d_point), "launch point-mass kernel");
+        ctx->ran_point = true;
         ctx->launches++;
         return EPH_OK;
     }
@@ -405,6 +411,10 @@ static int launch(eph_ctx *ctx, const StepParams &P) {
 
 static int finish(eph_ctx *ctx) {
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
+    if (ctx->ran_point) {
+        CK(cudaStreamSynchronize(ctx->stream), "point-mass kernel");
+        return EPH_OK;
+    }
     int status = 0;
     CK(cudaMemcpyAsync(&status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "read status");
     CK(cudaStreamSynchronize(ctx->stream), "RK12 kernel");

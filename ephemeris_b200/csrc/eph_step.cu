@@ -99,10 +99,10 @@ struct FieldBody {
 
 struct Scratch {
     double part[kWarps][kSumPad];     // per-warp partial sums
-    int wbody[kWarps];                // owned body that each sweep warp works for
+    int wbody[kWarps];                // owned body that each sweep warp works for (pass A: its job)
     double red[kOwnMax][kSumPad];     // sums of the latest sweep, see group_sums
     short row_a[TA_ROWS], row_b[TB_ROWS];   // source plane of each tile row, or -1: not copied (tile_rows)
-    int split_a0[kOwnMax + 1];        // warp groups of the first pass-A sweep (all owned bodies, weighted)
+    int split_a0[kOwnMax + 1];        // warp groups of the first pass-A sweep (sc.job_a, weighted)
     int split_b[kOwnMax + 1];         // warp groups of the pass-B sweep (all owned bodies, weighted)
     int nw_b;                         // warps of the pass-B sweep (the last one sums host reactions meanwhile)
     double ext[kOwnMax][kMaxExt][3];  // other hosts' fields on the owned bodies (geopotential, or ring)
@@ -126,7 +126,9 @@ struct Scratch {
     unsigned long long mbar;          // mbarrier of the tile copies
     unsigned long long bar_target;    // grid-barrier arrivals that complete the next barrier
     long long traj_slot;              // stage-record slot of the current stage evaluation
-    int flag, pad;
+    int flag;
+    unsigned char njob_a;             // jobs of the first pass-A sweep: one owned body, or two point-like ones together:
+    unsigned char job_a[kOwnMax];     // body + 16 (second body + 1), 0 there without one
 };
 
 // Shared memory: the owned bodies, the scratch, the staging tile of kTileRows rows, then the ring terms. The tile's row stride
@@ -136,7 +138,7 @@ constexpr int kMaxSmem = 227 * 1024;   // the per-CTA maximum; the kernel has no
 constexpr size_t kFixedSmem = ((sizeof(Own) * kOwnMax + sizeof(Scratch) + 127) / 128) * 128;
 constexpr int kRingTerms = kFieldMax * kRingPar * kRingDiskPar * 3;   // per-disk ring terms, [f][h][d][3], behind the tile
 constexpr int kTileW = (int)((kMaxSmem - kFixedSmem - kRingTerms * sizeof(double)) / (kTileRows * sizeof(double))) / kPad * kPad;
-static_assert(kTileW >= 512, "the staging tile must hold a 512-body system in one piece");
+static_assert(kTileW >= 576, "the staging tile must hold a 512-body system in one piece");
 // Pass A reads half as many rows as the tile has: a system of up to twice the tile's width is staged whole for its
 // sweeps, at twice the row stride, instead of in chunks that every iteration of the angular-velocity fixed point
 // copies again. Rows 6 to 11, the velocities, are free in a CTA without a delayed tide: the reactions of its field
@@ -418,15 +420,18 @@ __device__ __forceinline__ unsigned long long key_of(double v) {
 // `mask`: a half warp per (body, value), a lane per warp, summed as a tree. With `ext` (pass B), value 10 is the key
 // of the smallest m and value 11 that of the largest GM/r^3, which carries the pair's m and GM in 12 and 13; ties go
 // to the lower warp. Called between two barriers over the nw warps.
-__device__ __forceinline__ void group_sums(Scratch &sc, int nb, unsigned mask, int nw, bool ext) {
+template <bool ext, bool kTwos>
+__device__ __forceinline__ void group_sums(Scratch &sc, int nb, unsigned mask, int nw) {
     constexpr unsigned all = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = lane & 15;
     static_assert(kWarps == 16, "a half warp holds one value of every warp");
-    const int body_w = w < nw ? sc.wbody[w] : -1;
+    const int work = w < nw ? sc.wbody[w] : -1;
+    const int body_w = kTwos && work >= 0 ? work & 15 : work, second_w = kTwos && work >= 0 ? (work >> 4) - 1 : -1;
+    const int cols = kTwos && second_w >= 0 ? 4 : kSums;   // a warp of two bodies: four values of the first, then four of the second
     #pragma unroll 1
     for (int base = warp * 2; base < nb * kSums; base += nw * 2) {
         const int item = base + (lane >> 4), b = item / kSums, c = item - b * kSums;
-        double v = body_w == b ? sc.part[w][c] : 0.0;
+        double v = c >= cols ? 0.0 : body_w == b ? sc.part[w][c] : kTwos && second_w == b ? sc.part[w][4 + c] : 0.0;
         if (ext && c >= kSumB) {   // (uniform over the warp: base and kSums are even)
             unsigned long long k = (unsigned long long)__double_as_longlong(v);
             int src = w;
@@ -633,6 +638,31 @@ __device__ __forceinline__ void pair_a(const Own &o, const double *T, int j, dou
     acc[10] += tp_dg * diag;
 }
 
+// The pairs of two point-like bodies (kind 0) with body j: what the pair reads of j, 16 of 24 shared-memory wavefronts
+// of a warp's pair, is read once for both, and the two chains interleave. acc = {sum GM_j / r, sum g r} of each. A
+// body takes part in its own sum with GM = 0 at unit distance. 800 point masses 23.0 -> 21.9 us per stage, 800 and 1,001
+// bodies with full physics 39.9 -> 38.3 and 46.6 -> 43.9.
+template <int ts>
+__device__ __forceinline__ void pair_a2(const Own &o, const Own &p, const double *T, int j, int self_o, int self_p, double acc[8]) {
+    const v3 hi = mk(T[(TA_R_HI + 0) * ts + j], T[(TA_R_HI + 1) * ts + j], T[(TA_R_HI + 2) * ts + j]);
+    const v3 lo = mk(T[(TA_R_LO + 0) * ts + j], T[(TA_R_LO + 1) * ts + j], T[(TA_R_LO + 2) * ts + j]);
+    const double GMj = T[TA_GM * ts + j], sR2j = T[TA_SR2 * ts + j];
+    auto one = [&](const Own &q, bool self, double *a) {
+        const v3 r = mk(sep_diff(hi.x, lo.x, q.r[0].hi, q.r[0].lo), sep_diff(hi.y, lo.y, q.r[1].hi, q.r[1].lo),
+                        sep_diff(hi.z, lo.z, q.r[2].hi, q.r[2].lo));
+        const double d = dot(r, r), sm = q.sR2 + sR2j;
+        const double rr = inv_sqrt(self ? 1.0 : (d < sm) ? sm : d);
+        const double tp_dphi = rr * (self ? 0.0 : GMj);
+        const double tp_dg = (rr * rr) * tp_dphi;
+        a[0] += tp_dphi;
+        a[1] += tp_dg * r.x;
+        a[2] += tp_dg * r.y;
+        a[3] += tp_dg * r.z;
+    };
+    one(o, j == self_o, acc);
+    one(p, j == self_p, acc + 4);
+}
+
 // UPDATE_HARMONICS followed by UPDATE_ANGULAR_VELOCITY (mass.impl:48-72) for owned body o, on one thread,
 // from the pass-A sums in o.sumA. The first iteration of a stage (`first`) also sets the potential and the
 // Newtonian acceleration and rotates the static harmonics into the world frame once for the stage (they do
@@ -714,11 +744,12 @@ __device__ void tile_rows(Scratch &sc, bool need_v, bool reuse) {
 template <Layout kL>
 __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int buf, Scratch &sc, TileState &ts,
                         double *tile, int nw, const int *first_all) {
-    const int na = __popc(mask);
+    constexpr bool kTwos = kL != kOneTile;   // point-like bodies may go in twos (sc.job_a)
+    const int na = kTwos && first_all ? sc.njob_a : __popc(mask);
     if (na == 0) return true;
     const int n = S.n, T = S.tile;
-    // Warp groups: the first sweep of a stage covers every owned body (`first_all`, weighted, fixed per
-    // launch); a re-sweep covers the unconverged delayed tides, which all cost the same, so the nw warps are
+    // Warp groups: the first sweep of a stage covers every owned body (the jobs of sc.job_a in `first_all`, weighted,
+    // fixed per launch); a re-sweep covers the unconverged delayed tides, which all cost the same, so the nw warps are
     // split equally: slot a owns warps [ceil(a nw / na), ceil((a + 1) nw / na)), i.e. warp w is in slot
     // floor(w na / nw). Every thread works its group out itself: no shared list, no barrier.
     auto bounds = [&](int slot, int &w0, int &w1) {
@@ -737,7 +768,8 @@ __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int bu
     int gw0, gw1;
     bounds(my_slot, gw0, gw1);
     const Group g{my_slot, (warp - gw0) * 32 + (int)(threadIdx.x & 31), (gw1 - gw0) * 32};
-    const int body = body_of(my_slot);
+    const int job = kTwos && first_all ? sc.job_a[my_slot] : body_of(my_slot);
+    const int body = kTwos ? job & 15 : job, second = kTwos ? (job >> 4) - 1 : -1;
     const Own &o = own[body];
     double acc[kSumA];
 #pragma unroll
@@ -750,16 +782,23 @@ __device__ bool sweep_a(const SysDev &S, Own *own, int nb, unsigned mask, int bu
             if (!load_tile(S, sc, ts, tile, kTileW, pub, sc.row_a, TA_ROWS, j0, cnt, cnt, TA_ROWS)) return false;
         }
         const int self = o.idx - j0;
+        constexpr int stride = kL == kWideA ? kWideW : kTileW;
+        if (kTwos && second >= 0) {
+            const Own &p = own[second];
 #pragma unroll 1
-        for (int jj = g.tid; jj < cnt; jj += g.size)
-            if (jj != self) pair_a<kL == kWideA ? kWideW : kTileW>(o, tile, jj, acc);
+            for (int jj = g.tid; jj < cnt; jj += g.size) pair_a2<stride>(o, p, tile, jj, self, p.idx - j0, acc);
+        } else {
+#pragma unroll 1
+            for (int jj = g.tid; jj < cnt; jj += g.size)
+                if (jj != self) pair_a<stride>(o, tile, jj, acc);
+        }
     }
     // sums over each body's warp group
     const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) sc.wbody[w] = body;
+    if ((threadIdx.x & 31) == 0) sc.wbody[w] = job;
     warp_sums(acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], acc[6], acc[7], acc[8], acc[9], acc[10], 0.0, sc.part[w], kSumA);
     part_sync(nw * 32);
-    group_sums(sc, nb, mask, nw, false);
+    group_sums<false, kTwos>(sc, nb, mask, nw);
     part_sync(nw * 32);
     return true;
 }
@@ -1050,7 +1089,7 @@ __device__ __forceinline__ bool pass_a(const SysDev &S, Own *own, int nb, int bu
         }
         const bool ring_here = warp == kWarps - 1 && (ph == 0 ? ring_side : ring_after);
         const bool gp_here = ph == 0 ? (gp_side && warp >= nw) : !gp_side;
-        const int gp_lo = ph == 0 ? kWarps - kExtWarps : 0;
+        const int gp_lo = ph == 0 ? nw : 0;
         const int gp_hi = (ph == 0 ? ring_side : ring_after) ? kWarps - 1 : kWarps;
         if (ring_here) ext_ring(S, sc.fb, nf, buf, sc, st, ring_terms);
         else if (gp_here && warp >= gp_lo && warp < gp_hi) ext_gp(S, sc.fb, nf, buf, sc, st, gp_lo, gp_hi);
@@ -1228,7 +1267,7 @@ __device__ __forceinline__ bool pass_b(const SysDev &S, Own *own, int nb, int bu
         }
         warp_sums(acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], acc[6], acc[7], acc[8], acc[9], 0.0, 0.0, row, kSumB);
         part_sync(nwb * 32);
-        group_sums(sc, nb, ~0u, nwb, true);
+        group_sums<true, false>(sc, nb, ~0u, nwb);
         part_sync(nwb * 32);
         if (threadIdx.x < nb) {
             Own &ob = own[threadIdx.x];
@@ -1650,8 +1689,7 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams 
     __syncthreads();
     if (threadIdx.x < nb) publish_body(S, own[threadIdx.x], 0);
     if (threadIdx.x == 32) {
-        // warp groups of the sweeps over all owned bodies: delayed-tide pass-A pairs cost ~8x a point pair,
-        // full-class pass-B pairs ~2x. During the pass-A sweeps the last warp evaluates the ring items and
+        // warp groups of the sweeps over all owned bodies: full-class pass-B pairs cost ~2x a point pair. During the pass-A sweeps the last warp evaluates the ring items and
         // the kExtWarps - 1 warps before it the geopotential items.
         int wt[kOwnMax];
         bool delayed = false;
@@ -1662,8 +1700,31 @@ __global__ void __launch_bounds__(kThreads, 1) step_kernel(SysDev S, StepParams 
         sc.ext_overlap = side;
         sc.ring_side = side && sc.n_ring_e > 0;
         sc.nw_a = sc.ext_overlap ? kWarps - kExtWarps : sc.ring_side ? kWarps - 1 : kWarps;
-        for (int b = 0; b < nb; ++b) wt[b] = own[b].kind == 2 ? 8 : 1;
-        split_warps(wt, nb, P.mode == MODE_DEFORM ? kWarps : sc.nw_a, sc.split_a0);
+        const int nw_a = P.mode == MODE_DEFORM ? kWarps : sc.nw_a;
+        if (kL == kOneTile) {
+            for (int b = 0; b < nb; ++b) wt[b] = own[b].kind == 2 ? 8 : 1;
+            split_warps(wt, nb, nw_a, sc.split_a0);
+        } else {
+            // Beyond one tile, point-like bodies go in twos when there are more pairs than threads. (The code costs a
+            // system of one tile more than it gains: 504 bodies 24.4 -> 25.5 us per stage, 48 19.1 -> 19.7.) A delayed
+            // pair beside them counts as four single ones, else as eight (1,001 bodies: 43.9 us per stage, with eight
+            // 45.7).
+            const bool twos = nb * S.n > nw_a * 32;
+            int nj = 0, open = -1;
+            for (int b = 0; b < nb; ++b) {
+                if (twos && own[b].kind == 0 && open >= 0) {
+                    sc.job_a[open] |= 16 * (b + 1);
+                    wt[open] = 3;
+                    open = -1;
+                    continue;
+                }
+                if (own[b].kind == 0) open = nj;
+                sc.job_a[nj] = b;
+                wt[nj++] = own[b].kind == 2 ? 8 : 2;
+            }
+            sc.njob_a = nj;
+            split_warps(wt, nj, nw_a, sc.split_a0);
+        }
         for (int b = 0; b < nb; ++b) wt[b] = own[b].full ? 2 : 1;
         // a CTA that owns geopotential / ring hosts sums their reactions on its last warp during the
         // pass-B sweep (one tile only: streaming tiles needs every warp for the copies)

@@ -1036,35 +1036,33 @@ int eph_bspline_fit_batch(int device, int d, int64_t n, int64_t mn, int channels
     };
     const std::vector<double> rw = pack(f.rw_hi, f.rw_lo), lu = pack(f.lu_hi, f.lu_lo), rd = pack(f.rd_hi, f.rd_lo);
     const size_t n_smp = (size_t)n_series * (mn + 1) * channels, n_coef = (size_t)n_series * m * channels;
-    double *d_smp = nullptr, *d_coef = nullptr, *d_y = nullptr, *d_bval = nullptr, *d_rw = nullptr, *d_lu = nullptr, *d_rd = nullptr;
-    long long *d_jmin = nullptr;
-    int *d_cnt = nullptr;
-    int rc = EPH_OK;
-    cudaError_t e = cudaSuccess;
-    auto alloc = [&](void **p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+    // One allocation, and one copy for the matrix's tables: the allocations and frees of nine arrays took longer than
+    // the kernel (419 bodies, 365 knots: 5.9 -> 4.0 ms with everything, at the same sizes of the copies).
+    std::vector<char> tab;
+    auto put = [&](const void *p, size_t bytes) {   // the table's offset, 256-byte aligned
+        const size_t at = (tab.size() + 255) / 256 * 256;
+        tab.resize(at + bytes);
+        memcpy(tab.data() + at, p, bytes);
+        return at;
     };
-    alloc((void **)&d_smp, n_smp * sizeof(double));
-    alloc((void **)&d_coef, n_coef * sizeof(double));
-    alloc((void **)&d_y, (size_t)2 * m * T * sizeof(double));
-    alloc((void **)&d_bval, f.bval.size() * sizeof(double));
-    alloc((void **)&d_rw, rw.size() * sizeof(double));
-    alloc((void **)&d_lu, lu.size() * sizeof(double));
-    alloc((void **)&d_rd, rd.size() * sizeof(double));
-    alloc((void **)&d_jmin, f.jmin.size() * sizeof(long long));
-    alloc((void **)&d_cnt, f.cnt.size() * sizeof(int));
-    if (e != cudaSuccess) rc = e == cudaErrorMemoryAllocation ? EPH_ERR_OOM : EPH_ERR_CUDA;
-    if (!rc) {
-        std::vector<long long> jm(f.jmin.begin(), f.jmin.end());
-        if ((e = cudaMemcpy(d_smp, samples, n_smp * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
-            (e = cudaMemcpy(d_bval, f.bval.data(), f.bval.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
-            (e = cudaMemcpy(d_rw, rw.data(), rw.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
-            (e = cudaMemcpy(d_lu, lu.data(), lu.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
-            (e = cudaMemcpy(d_rd, rd.data(), rd.size() * sizeof(double), cudaMemcpyHostToDevice)) != cudaSuccess ||
-            (e = cudaMemcpy(d_jmin, jm.data(), jm.size() * sizeof(long long), cudaMemcpyHostToDevice)) != cudaSuccess ||
-            (e = cudaMemcpy(d_cnt, f.cnt.data(), f.cnt.size() * sizeof(int), cudaMemcpyHostToDevice)) != cudaSuccess)
-            rc = EPH_ERR_CUDA;
-    }
+    const std::vector<long long> jm(f.jmin.begin(), f.jmin.end());
+    const size_t o_bval = put(f.bval.data(), f.bval.size() * sizeof(double)), o_rw = put(rw.data(), rw.size() * sizeof(double)),
+                 o_lu = put(lu.data(), lu.size() * sizeof(double)), o_rd = put(rd.data(), rd.size() * sizeof(double)),
+                 o_jmin = put(jm.data(), jm.size() * sizeof(long long)), o_cnt = put(f.cnt.data(), f.cnt.size() * sizeof(int));
+    auto round = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t o_smp = round(tab.size()), o_coef = o_smp + round(n_smp * sizeof(double)), o_y = o_coef + round(n_coef * sizeof(double));
+    char *base = nullptr;
+    int rc = EPH_OK;
+    cudaError_t e = cudaMalloc((void **)&base, o_y + (size_t)2 * m * T * sizeof(double));
+    if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? EPH_ERR_OOM : EPH_ERR_CUDA;
+    double *d_smp = (double *)(base + o_smp), *d_coef = (double *)(base + o_coef), *d_y = (double *)(base + o_y);
+    const double *d_bval = (double *)(base + o_bval), *d_rw = (double *)(base + o_rw), *d_lu = (double *)(base + o_lu),
+                 *d_rd = (double *)(base + o_rd);
+    const long long *d_jmin = (long long *)(base + o_jmin);
+    const int *d_cnt = (int *)(base + o_cnt);
+    if (cudaMemcpy(base, tab.data(), tab.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(d_smp, samples, n_smp * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+        rc = EPH_ERR_CUDA;
     if (!rc) {
         const int threads = 128;
         bspline_solve_kernel<<<(unsigned)((T + threads - 1) / threads), threads>>>(
@@ -1074,9 +1072,7 @@ int eph_bspline_fit_batch(int device, int d, int64_t n, int64_t mn, int channels
             (e = cudaMemcpy(coefs, d_coef, n_coef * sizeof(double), cudaMemcpyDeviceToHost)) != cudaSuccess)
             rc = EPH_ERR_CUDA;
     }
-    for (void *p : {(void *)d_smp, (void *)d_coef, (void *)d_y, (void *)d_bval, (void *)d_rw, (void *)d_lu, (void *)d_rd,
-                    (void *)d_jmin, (void *)d_cnt})
-        if (p) cudaFree(p);
+    cudaFree(base);
     return rc;
 }
 

@@ -384,7 +384,7 @@ __device__ __forceinline__ void part_sync(int nthreads) {
 }
 
 // The two reductions behind both passes' sweeps, kept short: a stage runs through its code once, so every instruction
-// of it is fetched, not reused, and those fetches are the largest stall of a small system. (Out of line they cost
+// of it is fetched, not reused, and those fetches stall a small system more than its arithmetic. (Out of line they cost
 // more than they save: a call that takes the kernel's parameters by reference moves them to local memory.) With the
 // one-copy pair_b, 48 / 504 bodies, full physics: 22.3 -> 19.9 / 28.5 -> 25.2 us per stage.
 //

@@ -754,7 +754,8 @@ int eph_particles_integrate(eph_particles *p, double dt, int64_t n_step, double 
     // msystem::integrate: maxima reset before, min_distance inverted after (mass.cpp:406,436)
     double *d_pl = nullptr;
     eph_device_planes(p->ctx, &d_pl);
-    PCK(cudaMemset(d_pl + (size_t)EPH_P_MIN_DISTANCE * p->n_pert, 0, 2 * p->n_pert * sizeof(double)), "reset maxima");
+    // On the set's stream, which the perturbers' stream waits for: nothing orders the default stream before either.
+    PCK(cudaMemsetAsync(d_pl + (size_t)EPH_P_MIN_DISTANCE * p->n_pert, 0, 2 * p->n_pert * sizeof(double), p->stream), "reset maxima");
     PCK(cudaEventRecord(p->ev_begin, p->stream), "event");
     auto begin = [&](int64_t steps, double *traj) {   // a round of perturbers, on the context's stream
         ctx_record_stages(p->ctx, traj, 1);
@@ -809,11 +810,12 @@ int eph_particles_integrate(eph_particles *p, double dt, int64_t n_step, double 
         ready = next;
     }
     std::vector<double> md(p->n_pert);
-    PCK(cudaMemcpy(md.data(), d_pl + (size_t)EPH_P_MIN_DISTANCE * p->n_pert, p->n_pert * sizeof(double),
-                   cudaMemcpyDeviceToHost), "maxima");
+    double *d_md = d_pl + (size_t)EPH_P_MIN_DISTANCE * p->n_pert;
+    PCK(cudaMemcpyAsync(md.data(), d_md, md.size() * sizeof(double), cudaMemcpyDeviceToHost, p->stream), "maxima");
+    PCK(cudaStreamSynchronize(p->stream), "maxima");
     for (auto &x : md) x = 1 / x;
-    PCK(cudaMemcpy(d_pl + (size_t)EPH_P_MIN_DISTANCE * p->n_pert, md.data(), p->n_pert * sizeof(double),
-                   cudaMemcpyHostToDevice), "maxima");
+    PCK(cudaMemcpyAsync(d_md, md.data(), md.size() * sizeof(double), cudaMemcpyHostToDevice, p->stream), "maxima");
+    PCK(cudaStreamSynchronize(p->stream), "maxima");
     return EPH_OK;
 }
 

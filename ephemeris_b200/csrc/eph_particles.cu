@@ -757,22 +757,34 @@ int eph_particles_integrate(eph_particles *p, double dt, int64_t n_step, double 
     // On the set's stream, which the perturbers' stream waits for: nothing orders the default stream before either.
     PCK(cudaMemsetAsync(d_pl + (size_t)EPH_P_MIN_DISTANCE * p->n_pert, 0, 2 * p->n_pert * sizeof(double), p->stream), "reset maxima");
     PCK(cudaEventRecord(p->ev_begin, p->stream), "event");
-    auto begin = [&](int64_t steps, double *traj) {   // a round of perturbers, on the context's stream
+    double th = *t_eph_hi, tl = *t_eph_lo;   // time at the start of the next round of perturbers
+    // A round of perturbers on the context's stream: begin launches it, end waits for it. No way out of this function
+    // leaves one in flight, or the context recording.
+    struct Round {
+        eph_ctx *ctx;
+        bool open = false;
+        int end() {
+            open = false;
+            const int r = ctx_rk12_end(ctx);
+            ctx_record_stages(ctx, nullptr, 0);
+            return r;
+        }
+        ~Round() {
+            if (open) end();
+        }
+    } pert{p->ctx};
+    auto begin = [&](int64_t steps, double *traj) {
         ctx_record_stages(p->ctx, traj, 1);
-        const int r = ctx_rk12_begin(p->ctx, dt, steps, *t_eph_hi + *t_eph_lo, p->ev_begin);
+        pert.open = true;
+        const int r = ctx_rk12_begin(p->ctx, dt, steps, th + tl, p->ev_begin);
         if (r) return r;
         ++p->launches;
-        dd_advance(t_eph_hi, t_eph_lo, dt * (double)steps);
+        dd_advance(&th, &tl, dt * (double)steps);
         return (int)EPH_OK;
-    };
-    auto end = [&]() {
-        const int r = ctx_rk12_end(p->ctx);
-        ctx_record_stages(p->ctx, nullptr, 0);
-        return r;
     };
     int64_t ready = std::min<int64_t>(n_step, chunk);   // steps of the round whose records are complete
     rc = begin(ready, p->d_traj[0]);
-    if (!rc) rc = end();
+    if (!rc) rc = pert.end();
     if (rc) return pfail(p, rc, eph_last_error(p->ctx));
     for (int64_t done = 0, round = 0; done < n_step; ++round) {
         const int64_t next = std::min<int64_t>(n_step - done - ready, chunk);
@@ -793,19 +805,19 @@ int eph_particles_integrate(eph_particles *p, double dt, int64_t n_step, double 
         A.next = p->d_next;
         PCK(cudaMemsetAsync(p->d_next, 0, sizeof(int), p->stream), "reset queue");
         PCK(cudaEventRecord(p->ev0, p->stream), "event");
-        kernel_of(p->general, p->mixed)<<<p->grid, kPThreads, part_smem((int)p->n_pert), p->stream>>>(A);
-        PCK(cudaGetLastError(), "launch particle kernel");
+        void *args[] = {&A};   // (the launch's own status: cudaGetLastError may still hold an earlier call's error)
+        PCK(cudaLaunchKernel((const void *)kernel_of(p->general, p->mixed), dim3(p->grid), dim3(kPThreads), args,
+                             part_smem((int)p->n_pert), p->stream), "launch particle kernel");
         ++p->launches;
         PCK(cudaEventRecord(p->ev1, p->stream), "event");
-        if (next > 0 && (rc = end())) {
-            cudaStreamSynchronize(p->stream);
-            return pfail(p, rc, eph_last_error(p->ctx));
-        }
+        rc = next > 0 ? pert.end() : (int)EPH_OK;
         PCK(cudaStreamSynchronize(p->stream), "particle kernel");
         float ms = 0;
         PCK(cudaEventElapsedTime(&ms, p->ev0, p->ev1), "event time");
         p->kernel_ms += ms;
         p->started = true;
+        dd_advance(t_eph_hi, t_eph_lo, dt * (double)ready);   // the particles' time; a round that fails later leaves it
+        if (rc) return pfail(p, rc, eph_last_error(p->ctx));
         done += ready;
         ready = next;
     }

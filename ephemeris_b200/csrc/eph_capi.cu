@@ -43,6 +43,7 @@ struct eph_ctx {
     int ld = 0, tile = 0;                // plane stride (n rounded up to kPad), bodies per smem tile
     int n_full = 0;                      // full-class bodies (device order)
     bool point_ok = false;               // a system of ordinary point-like bodies (point_system_ok)
+    bool planes_shared = false;          // the caller holds d_planes (eph_device_planes) and may write to it at any time
     bool point_accel_ok = false;         // and no oblateness change is loaded: so is one evaluation of it
     bool ran_point = false;              // the latest launch was of the point-mass kernel, which has no status
     double *d_point = nullptr;           // scratch of launch_point_system
@@ -251,6 +252,7 @@ int eph_upload_system(eph_ctx *ctx, int64_t n64, const double *planes, const eph
     if ((size_t)n > ctx->cap_n) {
         free_system(ctx);
         CK(cudaMalloc(&ctx->d_planes, (size_t)EPH_NPLANES * n * sizeof(double)), "cudaMalloc(planes)");
+        ctx->planes_shared = false;
         const int ld = (n + kPad - 1) / kPad * kPad;
         CK(cudaMalloc(&ctx->d_pub, (size_t)2 * PUB_NPLANES * ld * sizeof(double)), "cudaMalloc(public state)");
         CK(cudaMalloc(&ctx->d_aux, (size_t)AUX_NPLANES * ld * sizeof(double)), "cudaMalloc(aux)");
@@ -336,7 +338,7 @@ int eph_device_planes(eph_ctx *ctx, double **d_planes) {
     if (!ctx || !d_planes) return fail(ctx, EPH_ERR_ARG, "eph_device_planes: bad arguments");
     if (!ctx->n) return fail(ctx, EPH_ERR_STATE, "no system uploaded");
     *d_planes = ctx->d_planes;
-    ctx->point_ok = false;   // the caller may write to them
+    ctx->planes_shared = true;   // until the planes are allocated anew: what point_system_ok saw need not hold any more
     return EPH_OK;
 }
 
@@ -349,7 +351,8 @@ static int launch(eph_ctx *ctx, const StepParams &P) {
     if (!ctx->n) return fail(ctx, EPH_ERR_STATE, "no system uploaded");
     ctx->ran_point = false;
     if (((P.mode == MODE_INTEGRATE && ctx->point_ok) || (P.mode == MODE_ACCEL && ctx->point_accel_ok && ctx->point_ok)) &&
-        !ctx->stall_barrier && !ctx->d_traj && !ctx->d_timers && ctx->req_grid == 0 && ctx->req_per_cta == 0) {
+        !ctx->planes_shared && !ctx->stall_barrier && !ctx->d_traj && !ctx->d_timers && ctx->req_grid == 0 &&
+        ctx->req_per_cta == 0) {
         const size_t need = point_scratch_doubles(ctx->n);
         if (need > ctx->point_cap) {
             if (ctx->d_point) cudaFree(ctx->d_point);

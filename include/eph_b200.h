@@ -67,7 +67,8 @@ int eph_upload_system(eph_ctx *ctx, int64_t n, const double *planes, const eph_m
 int eph_upload_planes_device(eph_ctx *ctx, const double *d_planes);
 /* Copy the whole body state back (cuda_rungekutta_kernel_config::save, RungeKutta.cu:124-133). */
 int eph_download_system(eph_ctx *ctx, double *planes);
-/* Device copy of the planes [EPH_NPLANES][n] (valid until the next upload of a larger system). */
+/* Device copy of the planes [EPH_NPLANES][n] (valid until the next upload of a larger system). The caller may write to
+ * it between calls; from here until that upload the context uses the step kernel, also for small point-mass systems. */
 int eph_device_planes(eph_ctx *ctx, double **d_planes);
 
 /* msystem::Cuda_RungeKutta12(dt, n_step) (RungeKutta.cu:391-412): n_step Feagin RK12 steps of dt

@@ -79,3 +79,58 @@ def test_two_calls_are_one():
     pl = _system(97, seed=23)
     assert np.array_equal(_go(pl, [("integrate", 600.0, 5)], False)[0][0:100],
                           _go(pl, [("integrate", 600.0, 2), ("integrate", 600.0, 3)], False)[0][0:100])
+
+
+@pytest.mark.parametrize("then", ["nothing", "upload", "costs", "autotune", "larger", "accel"])
+def test_planes_the_caller_holds_stay_on_the_step_kernel(then):
+    """The caller may write to planes whose address it has, until a larger system is uploaded: whatever else is called
+    in between, a spin written there turns the frames (the step kernel's results, bit for bit)."""
+    import torch
+    from ephemeris_b200 import Context, PLANES as P
+    pl = _system(40, seed=24)
+    spun = pl.copy()
+    spun[P["W"] + 2, 5] = 1e-4
+    spun[P["GL_HI"] + 2, 5] = 1e-4 * spun[P["GI"] + 8, 5]
+
+    def through(c):                                     # writes `spun` to the context's planes, as its owner may
+        ptr = c.device_planes_ptr() if then == "larger" else held
+        src = Context(0)
+        src.upload(spun)
+        torch.cuda.synchronize()
+        _copy(ptr, src.device_planes_ptr(), spun.nbytes)
+        src.close()
+
+    c = Context(0)
+    c.upload(_system(30, seed=24) if then == "larger" else pl)
+    held = c.device_planes_ptr()
+    if then in ("upload", "larger"):
+        c.upload(pl)
+    elif then == "costs":
+        c.set_body_costs(None)
+    elif then == "autotune":
+        c.autotune(600.0, 1, 1, False)
+        c.set_launch(0, 0)
+    elif then == "accel":
+        c.accel()
+    through(c)
+    c.integrate(600.0, 2)
+    out = c.download()
+    c.close()
+    r = Context(0)
+    r.upload(pl)
+    r.set_launch(0, 8)
+    held = r.device_planes_ptr()
+    through(r)
+    r.integrate(600.0, 2)
+    ref = r.download()
+    r.close()
+    assert not np.array_equal(ref[P["S_HI"]:P["S_HI"] + 9, 5], pl[P["S_HI"]:P["S_HI"] + 9, 5])
+    assert np.array_equal(out, ref)
+
+
+def _copy(dst, src, nbytes):
+    from cuda.bindings import runtime
+    err, = runtime.cudaMemcpy(dst, src, nbytes, runtime.cudaMemcpyKind.cudaMemcpyDeviceToDevice)
+    assert int(err) == 0
+    err, = runtime.cudaDeviceSynchronize()
+    assert int(err) == 0

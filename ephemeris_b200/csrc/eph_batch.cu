@@ -35,6 +35,7 @@
 #include "eph_math.cuh"
 #include "eph_plan.h"
 #include "eph_rk12_host.h"
+#include "eph_share.h"
 #include "eph_system.cuh"
 #include "../../include/eph_b200.h"
 #include "../../include/eph_planes.h"
@@ -42,11 +43,7 @@
 namespace eph {
 namespace {
 
-constexpr int kBThreads = 256;          // threads per ensemble CTA
-constexpr int kCoopMin = 32;            // default: bodies from which a system may be shared by a cluster
 constexpr double kCB = 299792458.0;     // src/math/basic_math.h:10,18
-constexpr int kStore = 3 * kStages + 12;   // stored values per body: f_j of every stage, r0 and v0 (hi, lo)
-constexpr int kMaxSplit = 32;           // most parts a body's j range is cut into
 
 // The Feagin table in second-order form: v_j = v0 + dt sum_l a_jl f_l, so sum_j a_kj v_j = c_k v0 +
 // dt sum_l Abar_kl f_l with Abar = A A. Entry k(k-1)/2 + l: Abar_kl as hi + lo, a_kl rounded. The CTAs read the
@@ -61,6 +58,7 @@ struct RkTable {
     double2 ab[EPH_RK12_NCOEF];   // {Abar hi, a}
     double lo[EPH_RK12_NCOEF];    // Abar lo
 };
+static_assert(sizeof(RkTable) == kRkTableBytes, "static shared memory that eph_share.h leaves room for");
 
 struct BatchSys {
     int n;                // bodies
@@ -73,16 +71,6 @@ struct BatchSys {
     double *planes;       // [EPH_NPLANES][n], in and out
     double *store;        // [kStore][n] stage accelerations and start-of-step state, when shared memory has no room
 };
-
-// What a pair term reads of a body lies in records of 64 bytes, 80 apart, so that a thread fetches a body j with four
-// 16-byte shared-memory loads; the lanes of a warp work on different bodies i and the same j, which makes every
-// one of them a broadcast.
-enum RecA { RA_R_HI = 0, RA_R_LO = 3, RA_GM = 6, RA_SR2 = 7, kRecA = 10 };          // state of the stage
-enum RecB { RB_NACC = 0, RB_BETA = 3, RB_K = 6, RB_PHI = 7, kRecB = 10 };           // pass-A outputs; K = phi + 2 beta^2
-// The mixed-precision form reads single-precision copies instead of RecB.
-enum RecF { RF_NACC = 0, RF_GM = 3, RF_BETA = 4, RF_PHI = 7, RF_BETA2 = 8, kRecF = 12 };
-enum OwnRow { OR_V_HI = 0, OR_V_LO = 3, OR_M = 6, OR_MAXI = 7, OR_GM0 = 8, OR_DGM = 9, kOwnRows = 10 };
-constexpr int kPartA = 4, kPartB = 6;   // values of a unit's sums: {phi, a_N}; {gaccel, m_min, tq, j of tq}
 
 // One CTA's share of a system: the bodies [lo, lo + cnt) of n, and its shared memory. Every CTA of a cluster has
 // the same layout for the arrays that its peers write (A, and what pass B reads of all bodies: B, or F in mixed
@@ -101,16 +89,6 @@ struct View {
 __device__ __forceinline__ double &own_row(const View &V, int r, int b) { return V.own[r * V.cnt + b]; }
 __device__ __forceinline__ double *rec_b(const View &V, int i) { return V.B + (size_t)(i - V.b0) * kRecB; }
 
-// Shared memory (doubles) of each CTA when `peers` share a system of n bodies: room for the largest share. The
-// stage store is in it while two CTAs still fit an SM; larger shares keep it in global memory (L2).
-constexpr int kPairSmem = (113 * 1024 - (int)sizeof(RkTable) - 128) / 8;
-__host__ __device__ inline int batch_smem_doubles(int n, int peers, int split, bool mixed, bool *store_in_smem) {
-    const int most = (n + peers - 1) / peers;
-    const int base = n * ((peers > 1 ? 2 : 1) * kRecA + (mixed ? kRecF / 2 : kRecB)) +
-                     most * (split * kPartB + kOwnRows + (mixed ? kRecB : 0));
-    *store_in_smem = base + most * kStore <= kPairSmem;
-    return *store_in_smem ? base + most * kStore : base;
-}
 template <bool MIXED>
 __device__ __forceinline__ View make_view(const BatchSys &Y, double *smem, int lo, int cnt, int peers) {
     const bool coop = peers > 1;
@@ -655,7 +633,6 @@ __global__ void __launch_bounds__(kBThreads, 2)
     }
 }
 
-constexpr size_t kBMaxSmem = 227 * 1024 - sizeof(RkTable) - 256;
 // One system on the CTAs of one cluster: its steps, or one evaluation of its accelerations (eph_accel of 33 bodies,
 // with the read-back: 73 -> 45 us; of 300: 109 -> 78 us).
 template <bool kEval>
@@ -667,54 +644,42 @@ __global__ void __launch_bounds__(kBThreads, 2) point_kernel(BatchSys Y, int pee
     if (peers > 1) cg::this_cluster().sync();   // no CTA leaves while a peer may still store to it
 }
 
-// ---- how many CTAs share a system
-constexpr int kShares = 5;
-constexpr int kSharePeers[kShares] = {16, 8, 4, 2, 1};
-constexpr int kMinOwn = 12;  // bodies per CTA below which sharing a system further does not pay
-
-// Time of one stage (us) of a system of n bodies on `peers` CTAs, its j ranges cut into `split` parts: a model
-// of measurements on one B200 (single systems of 8-400 bodies on 1-16 CTAs): 2.6 us for the state update and the
-// phases per body, 1.3 us for the two cluster exchanges, and per unit of a thread 0.36 us a pair (both passes;
-// FP64 latency at 8 warps) and 0.3 us.
-float stage_us(int n, int peers, int split) {
-    const int per_thread = ((n + peers - 1) / peers * split + kBThreads - 1) / kBThreads;
-    return 2.6f + (peers > 1 ? 1.3f : 0.0f) + (float)per_thread * (0.36f * (float)((n + split - 1) / split) + 0.3f);
-}
-// Parts that each body's j range is cut into: the number that keeps the threads busiest over the CTA counts the
-// system may be shared by. It depends on n alone, so that a system's sums are the same however it is shared.
-constexpr int kMaxPerThread = 4;   // units per thread, by the shared memory of their sums
-int batch_split(int n) {
-    int best = 1;
-    float best_cost = 1e30f;
-    for (int g = 1; g <= kMaxSplit && g <= n; ++g) {
-        float cost = 0;
-        for (int peers : kSharePeers) {
-            const int cnt = (n + peers - 1) / peers;
-            if ((peers > 1 && n < kMinOwn * peers) || cnt * g > kMaxPerThread * kBThreads) continue;
-            cost += stage_us(n, peers, g) / stage_us(n, peers, std::max(1, std::min(n, kBThreads / cnt)));
-        }
-        // (the same CTA counts enter every candidate's mean)
-        int counted = 0;
-        for (int peers : kSharePeers)
-            counted += !((peers > 1 && n < kMinOwn * peers) || (n + peers - 1) / peers * g > kMaxPerThread * kBThreads);
-        if (counted && cost / counted < best_cost) { best_cost = cost / counted; best = g; }
+// CTA counts whose clusters the present device, or the part of it that the process may use, can hold, each CTA with the
+// most shared memory it may take. Above 8 CTAs that is not a matter of course.
+unsigned device_shares() {
+    unsigned set = 1u << (kShares - 1);
+    for (int g = 0; g < kShares - 1; ++g) {
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kSharePeers[g];
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kSharePeers[g]);
+        cfg.blockDim = dim3(kBThreads);
+        cfg.dynamicSmemBytes = kBMaxSmem;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, point_kernel<false>, &cfg) == cudaSuccess && clusters > 0) set |= 1u << g;
     }
-    return best;
+    cudaGetLastError();   // (a size that the device refuses)
+    return set;
 }
-bool share_fits(int n, int peers, int split) { return (n + peers - 1) / peers * split <= kMaxPerThread * kBThreads; }
-
-size_t system_smem(int n, int peers, int split, bool mixed) {
-    bool in_smem;
-    return batch_smem_doubles(n, peers, split, mixed, &in_smem) * sizeof(double);
-}
-constexpr int kMaxBodies = 768;   // bodies of a system of the ensemble launch: shared memory holds it on one CTA
 
 std::atomic<bool> g_batch_ready[64];
+unsigned g_batch_shares[64];
 std::mutex g_batch_mu;   // contexts and batches may set a device up at the same time
-cudaError_t batch_setup(int device) {
-    if (device >= 0 && device < 64 && g_batch_ready[device].load(std::memory_order_acquire)) return cudaSuccess;
+cudaError_t batch_setup(int device, unsigned *shares) {
+    const bool kept = device >= 0 && device < 64;
+    if (kept && g_batch_ready[device].load(std::memory_order_acquire)) {
+        *shares = g_batch_shares[device];
+        return cudaSuccess;
+    }
     std::lock_guard<std::mutex> lock(g_batch_mu);
-    if (device >= 0 && device < 64 && g_batch_ready[device].load(std::memory_order_relaxed)) return cudaSuccess;
+    if (kept && g_batch_ready[device].load(std::memory_order_relaxed)) {
+        *shares = g_batch_shares[device];
+        return cudaSuccess;
+    }
     double hi[EPH_RK12_NCOEF], lo[EPH_RK12_NCOEF], dtk[kStages + 1];
     rk12_expand(hi, lo, dtk);
     double ab_hi[EPH_RK12_NCOEF] = {0}, ab_lo[EPH_RK12_NCOEF] = {0}, aa[EPH_RK12_NCOEF] = {0};
@@ -750,8 +715,13 @@ cudaError_t batch_setup(int device) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBMaxSmem);
     }
-    if (e == cudaSuccess && device >= 0 && device < 64) g_batch_ready[device].store(true, std::memory_order_release);
-    return e;
+    if (e != cudaSuccess) return e;
+    *shares = device_shares();
+    if (kept) {
+        g_batch_shares[device] = *shares;
+        g_batch_ready[device].store(true, std::memory_order_release);
+    }
+    return cudaSuccess;
 }
 
 }  // namespace
@@ -761,13 +731,18 @@ cudaError_t batch_setup(int device) {
 size_t point_scratch_doubles(int n) { return (size_t)kStore * n; }
 // Launches n_step steps of dt of a system of point-like bodies on `stream`, as the step kernel of eph_step.cu would
 // integrate it (accumulate: eph_rk12's maxima, else eph_integrate's); n_step 0: one evaluation of its accelerations.
+// cudaErrorNotSupported: the device's clusters are too small for it, nothing was launched.
 cudaError_t launch_point_system(int device, cudaStream_t stream, double *planes, int n, double dt, long long n_step, double t_eph,
                                 int accumulate, double *scratch) {
-    cudaError_t e = batch_setup(device);
+    unsigned shares = 0;
+    cudaError_t e = batch_setup(device, &shares);
     if (e != cudaSuccess) return e;
+    const int split = batch_split(n), g = shortest_stage(n, split, false, shares);
+    if (g < 0) return cudaErrorNotSupported;
+    const int peers = kSharePeers[g];
     BatchSys Y{};
     Y.n = n;
-    Y.split = batch_split(n);
+    Y.split = split;
     Y.n_step = n_step;
     Y.dt = dt;
     Y.t_eph = t_eph;
@@ -775,13 +750,6 @@ cudaError_t launch_point_system(int device, cudaStream_t stream, double *planes,
     Y.whole = 1;
     Y.planes = planes;
     Y.store = scratch;
-    int peers = 0;   // the CTA count with the shortest stage
-    float best = 1e30f;
-    for (int p : kSharePeers) {
-        if ((p > 1 && n < kMinOwn * p) || !share_fits(n, p, Y.split) || system_smem(n, p, Y.split, false) > kBMaxSmem) continue;
-        const float t = stage_us(n, p, Y.split);
-        if (t < best) { best = t; peers = p; }
-    }
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = peers;
@@ -789,7 +757,7 @@ cudaError_t launch_point_system(int device, cudaStream_t stream, double *planes,
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(peers);
     cfg.blockDim = dim3(kBThreads);
-    cfg.dynamicSmemBytes = system_smem(n, peers, Y.split, false);
+    cfg.dynamicSmemBytes = system_smem(n, peers, split, false);
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
@@ -805,6 +773,7 @@ struct eph_batch {
     cudaStream_t own_stream = nullptr;
     cudaStream_t side[kShares] = {};   // the launches of one integration run beside each other
     cudaEvent_t ev_begin = nullptr, ev_end[kShares] = {};
+    unsigned shares = 0;               // CTA counts that the device can hold as clusters (batch_setup)
     int mixed = 0;                     // 1: EIH 1PN terms of the ensemble kernel in FP32 (eph_batch_set_precision)
     int coop_min = kCoopMin;           // bodies from which a system is shared by a cluster (eph_batch_set_coop_min)
     std::mutex mu;
@@ -866,7 +835,7 @@ int eph_batch_create(int device, eph_batch **out) {
     eph_batch *b = new eph_batch();
     b->device = device;
     if (cudaSetDevice(device) != cudaSuccess || cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        batch_setup(device) != cudaSuccess || !batch_side(b)) {
+        batch_setup(device, &b->shares) != cudaSuccess || !batch_side(b)) {
         eph_batch_destroy(b);
         return EPH_ERR_CUDA;
     }
@@ -920,9 +889,12 @@ int eph_batch_upload(eph_batch *b, int32_t n_sys, const int64_t *n_body, const d
         const int n = (int)n_body[s];
         bool pt = n <= kMaxBodies;
         for (int i = 0; i < n && pt; ++i) pt = !plan_full_class(planes[s], n, i);
+        if (pt) {   // (in either precision, which may be chosen after the upload)
+            b->split[s] = batch_split(n);
+            pt = fewest_ctas(n, b->split[s], false, b->shares) >= 0 && fewest_ctas(n, b->split[s], true, b->shares) >= 0;
+        }
         b->point[s] = pt;
         if (pt) {
-            b->split[s] = batch_split(n);
             b->off[s] = tot;
             b->store_off[s] = tot_store;
             tot += (size_t)EPH_NPLANES * n;
@@ -991,7 +963,7 @@ int eph_batch_integrate(eph_batch *b, const double *dt, const int64_t *n_step, d
         double total = 0;
         std::vector<std::pair<double, int>> heap;   // (duration, system), longest on top
         for (int s : order) {
-            while (share[s] > 0 && (!share_fits((int)b->n_body[s], kSharePeers[share[s]], b->split[s]) || system_smem((int)b->n_body[s], kSharePeers[share[s]], b->split[s], b->mixed) > kBMaxSmem)) --share[s];
+            share[s] = fewest_ctas((int)b->n_body[s], b->split[s], b->mixed, b->shares);
             work[s] = job(s, share[s]);
             total += work[s] * kSharePeers[share[s]];
             heap.emplace_back(work[s], s);
@@ -999,12 +971,12 @@ int eph_batch_integrate(eph_batch *b, const double *dt, const int64_t *n_step, d
         std::make_heap(heap.begin(), heap.end());
         while (!heap.empty() && heap.front().first > 1.1 * total / (2.0 * sms)) {
             std::pop_heap(heap.begin(), heap.end());
-            const int s = heap.back().second, g = share[s] - 1;
+            const int s = heap.back().second, g = more_ctas((int)b->n_body[s], b->split[s], b->mixed, b->shares, share[s]);
             heap.pop_back();
-            if (g < 0 || b->n_body[s] < b->coop_min || b->n_body[s] < kMinOwn * kSharePeers[g]) break;
+            if (g < 0 || b->n_body[s] < b->coop_min) break;
             const double d = job(s, g);
             if (d > 0.95 * work[s]) break;
-            total += d * kSharePeers[g] - work[s] * kSharePeers[g + 1];
+            total += d * kSharePeers[g] - work[s] * kSharePeers[share[s]];
             share[s] = g;
             work[s] = d;
             heap.emplace_back(d, s);
@@ -1046,7 +1018,8 @@ int eph_batch_integrate(eph_batch *b, const double *dt, const int64_t *n_step, d
             cfg.numAttrs = 1;
             int clusters = 0;
             BCK(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg), "occupancy");
-            cfg.gridDim = dim3(peers * std::max(1, std::min(jobs, clusters)));
+            if (clusters <= 0) return bfail(b, EPH_ERR_CUDA, "no room for a cluster of the ensemble kernel");
+            cfg.gridDim = dim3(peers * std::min(jobs, clusters));
             BCK(cudaStreamWaitEvent(b->side[g], b->ev_begin, 0), "batch event");
             BCK(cudaLaunchKernelEx(&cfg, kernel, (const BatchSys *)b->d_sys, (const int *)b->d_order + begin, jobs,
                                    b->d_next + g, peers), "launch ensemble kernel");

@@ -361,11 +361,14 @@ static int launch(eph_ctx *ctx, const StepParams &P) {
             CK(cudaMalloc(&ctx->d_point, need * sizeof(double)), "cudaMalloc(point system)");
             ctx->point_cap = need;
         }
-        CK(launch_point_system(ctx->device, ctx->stream, ctx->d_planes, ctx->n, P.dt, P.mode == MODE_ACCEL ? 0 : P.n_step, P.t_eph,
-                               !P.reset_minmax, ctx->d_point), "launch point-mass kernel");
-        ctx->ran_point = true;
-        ctx->launches++;
-        return EPH_OK;
+        const cudaError_t e = launch_point_system(ctx->device, ctx->stream, ctx->d_planes, ctx->n, P.dt,
+                                                  P.mode == MODE_ACCEL ? 0 : P.n_step, P.t_eph, !P.reset_minmax, ctx->d_point);
+        if (e != cudaErrorNotSupported) {   // (no room for its clusters on this device: the step kernel)
+            CK(e, "launch point-mass kernel");
+            ctx->ran_point = true;
+            ctx->launches++;
+            return EPH_OK;
+        }
     }
     SysDev S;
     S.n = ctx->n;

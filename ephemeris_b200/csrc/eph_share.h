@@ -20,7 +20,7 @@ constexpr int kBThreads = 256;          // threads per ensemble CTA
 constexpr int kCoopMin = 32;            // default: bodies from which a system may be shared by a cluster
 constexpr int kStore = 3 * kStages + 12;   // stored values per body: f_j of every stage, r0 and v0 (hi, lo)
 constexpr int kMaxSplit = 32;           // most parts a body's j range is cut into
-constexpr int kMaxBodies = 768;         // bodies of a system of the ensemble launch
+constexpr int kMaxBodies = 768;         // bodies of a system of the ensemble launch (16 CTAs hold any such)
 
 // What a pair term reads of a body lies in records of 64 bytes, 80 apart, so that a thread fetches a body j with four
 // 16-byte shared-memory loads; the lanes of a warp work on different bodies i and the same j, which makes every
@@ -69,7 +69,10 @@ inline bool share_fits(int n, int peers, int split, bool mixed) {
     return units_fit(n, peers, split) && system_smem(n, peers, split, mixed) <= kBMaxSmem;
 }
 // Parts that each body's j range is cut into: the number that keeps the threads busiest over the CTA counts the
-// system may be shared by. It depends on n alone, so that a system's sums are the same however it is shared.
+// system may be shared by and on which its units fit. It depends on n alone, so that a system's sums are the same however
+// it is shared. Where many parts win, the units do not fit one CTA: 85, 96, 101 to 140 and more than 144 bodies take
+// two or more CTAs in any batch. On one CTA by memory alone they are slower: 96 bodies in a full batch 5.1 ms against
+// 4.0 on two, 128 5.7 against 4.4, 200 9.0 against 6.4.
 inline int batch_split(int n) {
     int best = 1;
     float best_cost = 1e30f;
@@ -80,7 +83,6 @@ inline int batch_split(int n) {
             if ((peers > 1 && n < kMinOwn * peers) || cnt * g > kMaxPerThread * kBThreads) continue;
             cost += stage_us(n, peers, g) / stage_us(n, peers, std::max(1, std::min(n, kBThreads / cnt)));
         }
-        // (the same CTA counts enter every candidate's mean)
         int counted = 0;
         for (int peers : kSharePeers)
             counted += !((peers > 1 && n < kMinOwn * peers) || (n + peers - 1) / peers * g > kMaxPerThread * kBThreads);

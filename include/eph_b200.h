@@ -161,8 +161,9 @@ int eph_batch_set_stream(eph_batch *b, void *stream);
  * double-double). Applies from the next integrate; systems on the single-system path are not affected. */
 int eph_batch_set_precision(eph_batch *b, int mode);
 /* Systems of at least `bodies` bodies may be shared by the CTAs (up to 16) of a thread-block cluster in the ensemble
- * launches (0: the default, 32); how many share one follows from the batch, and changes no result. A system too
- * large for one CTA's shared memory is shared whatever the threshold. */
+ * launches (0: the default, 32); how many share one follows from the batch, and changes no result. A system whose
+ * partial sums are too many for one CTA (85, 96, 101 to 140, more than 144 bodies) is shared whatever the threshold,
+ * by as few CTAs as hold them. */
 int eph_batch_set_coop_min(eph_batch *b, int bodies);
 /* Autotuner of the ensemble launch: times the uploaded batch's shared launch (step counts scaled by
  * step_frac, so the members keep their relative durations; best of 2 from the uploaded state, which is

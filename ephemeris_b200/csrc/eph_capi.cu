@@ -165,10 +165,12 @@ static int choose_shape(eph_ctx *ctx) {
 }
 
 // Whether a system may run on the point-mass kernel of eph_batch.cu, one cluster instead of the whole GPU: up to
-// kPointMax point-like bodies (a stage of 33 takes 4.6 us there and 13.3 us in the step kernel, of 200 10 and 13.9, of
-// 300 13.3 and 14.5, of 400 19.7 and 15), with masses and moments of inertia for which the step kernel's harmonics and
-// angular velocity stay exactly zero (any other body it turns into NaN or infinite ones there).
-constexpr int kPointMax = 300;
+// kPointMax point-like bodies with masses and moments of inertia for which the step kernel's harmonics and angular
+// velocity stay exactly zero (any other body it turns into NaN or infinite ones there).
+// One evaluation: 17 us of 33 bodies there and 42 in the step kernel, 26 and 48 of 300 (launch and wait, no read-back).
+// Steps, up to kPointSteps bodies: a stage of 33 takes 4.9 us there and 11.2 in the step kernel, of 200 10.8 and 12.3, of
+// 288 (18 bodies a CTA) 12.4 and 12.8, of 289 (19) 12.85 in both, of 300 13.5 and 13.4.
+constexpr int kPointMax = 300, kPointSteps = 288;
 static bool point_system_ok(const double *pl, int n, int n_full) {
     if (n_full > 0 || n < 2 || n > kPointMax) return false;   // (a lone body drifts as the reference's sums have it, bit for bit)
     for (int i = 0; i < n; ++i) {
@@ -182,6 +184,12 @@ static bool point_system_ok(const double *pl, int n, int n_full) {
             if (!std::isfinite(P(EPH_P_S_HI + q)) || !std::isfinite(P(EPH_P_S_LO + q))) return false;
     }
     return true;
+}
+
+// Whether a launch goes to the point-mass kernel unless a launch shape is requested.
+static bool point_route(const eph_ctx *ctx, int mode) {
+    if (!ctx->point_ok || ctx->planes_shared || ctx->stall_barrier || ctx->d_traj || ctx->d_timers) return false;
+    return mode == MODE_INTEGRATE ? ctx->n <= kPointSteps : mode == MODE_ACCEL && ctx->point_accel_ok;
 }
 
 static int prepare_constants(eph_ctx *ctx, const double *h_planes) {
@@ -350,9 +358,7 @@ static int launch(eph_ctx *ctx, const StepParams &P) {
     CK(cudaSetDevice(ctx->device), "cudaSetDevice");
     if (!ctx->n) return fail(ctx, EPH_ERR_STATE, "no system uploaded");
     ctx->ran_point = false;
-    if (((P.mode == MODE_INTEGRATE && ctx->point_ok) || (P.mode == MODE_ACCEL && ctx->point_accel_ok && ctx->point_ok)) &&
-        !ctx->planes_shared && !ctx->stall_barrier && !ctx->d_traj && !ctx->d_timers && ctx->req_grid == 0 &&
-        ctx->req_per_cta == 0) {
+    if (point_route(ctx, P.mode) && ctx->req_grid == 0 && ctx->req_per_cta == 0) {
         const size_t need = point_scratch_doubles(ctx->n);
         if (need > ctx->point_cap) {
             if (ctx->d_point) cudaFree(ctx->d_point);

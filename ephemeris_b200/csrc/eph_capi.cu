@@ -567,8 +567,10 @@ int eph_get_ownership(const eph_ctx *ctx, int32_t *bodies, int *grid) {
 namespace {
 struct TuneKey {
     int device, n, n_full, n_delayed, n_ext;
+    bool point;   // the heuristic's steps run on the point-mass kernel: a shape of the step kernel has that to beat
     bool operator<(const TuneKey &o) const {
-        return std::tie(device, n, n_full, n_delayed, n_ext) < std::tie(o.device, o.n, o.n_full, o.n_delayed, o.n_ext);
+        return std::tie(device, n, n_full, n_delayed, n_ext, point) <
+               std::tie(o.device, o.n, o.n_full, o.n_delayed, o.n_ext, o.point);
     }
 };
 struct TuneChoice {
@@ -611,7 +613,7 @@ int eph_autotune(eph_ctx *ctx, double dt, int n_step, int reps, int use_cache, i
     int n_delayed = 0;
     for (int i = 0; i < n; ++i)
         n_delayed += h_planes[(size_t)EPH_P_K2 * n + i] != 0 && h_planes[(size_t)EPH_P_TIDE_DELAY * n + i] != 0;
-    const TuneKey key{ctx->device, n, ctx->n_full, n_delayed, ctx->n_ext};
+    const TuneKey key{ctx->device, n, ctx->n_full, n_delayed, ctx->n_ext, point_route(ctx, MODE_INTEGRATE)};
     // every trial integrates from the uploaded state, which is restored afterwards
     double *d_save = nullptr;
     CK(cudaMalloc(&d_save, h_planes.size() * sizeof(double)), "cudaMalloc(autotune)");

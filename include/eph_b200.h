@@ -100,14 +100,15 @@ int eph_set_stream(eph_ctx *ctx, void *stream);
  * The reference fixes its shape in code (RungeKutta.cu:80-88); eph_autotune picks one by timing. */
 #define EPH_MAX_BODIES_PER_CTA 8
 int eph_set_launch(eph_ctx *ctx, int grid, int bodies_per_cta);
-/* Current launch shape. */
+/* Current launch shape of the step kernel. (Where none was requested, a small point-mass system runs on the point-mass
+ * kernel, one thread-block cluster; asking for a shape, this one too, brings it to the step kernel.) */
 int eph_get_launch(const eph_ctx *ctx, int *grid, int *bodies_per_cta);
 /* Autotuner (the reference fixes its launch shape in code, RungeKutta.cu:80-88): times candidate launch
  * shapes (bodies per CTA, hence the grid) and ownership cost models (the weight of a delayed-tide body) of
  * the step kernel on the uploaded system, n_step RK12 steps of dt each, best of `reps` after a warm-up run,
  * every trial starting from the uploaded state; keeps the fastest through eph_set_launch /
- * eph_set_body_costs and caches it per (device, bodies, body classes), so that with use_cache a later call on
- * a system of the same key times only the cached choice. Leaves the uploaded state as it was. Returns the
+ * eph_set_body_costs and caches it per (device, bodies, body classes, whether the heuristic runs on the point-mass
+ * kernel), so that with use_cache a later call on a system of the same key times only the cached choice. Leaves the uploaded state as it was. Returns the
  * chosen shape and the per-RK12-step times of the choice and of the built-in heuristic. */
 int eph_autotune(eph_ctx *ctx, double dt, int n_step, int reps, int use_cache, int *grid, int *bodies_per_cta,
                  double *ms_per_step_tuned, double *ms_per_step_default);

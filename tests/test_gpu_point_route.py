@@ -134,3 +134,25 @@ def _copy(dst, src, nbytes):
     assert int(err) == 0
     err, = runtime.cudaDeviceSynchronize()
     assert int(err) == 0
+
+
+@pytest.mark.parametrize("n", [41, 77, 143, 200])
+def test_tuned_shapes_are_kept_apart(n):
+    """A system with a mass rate stays on the step kernel, and a shape tuned for it is one of that kernel: a later system
+    of the same size that may run on the point-mass kernel is tuned by itself and stays there."""
+    from ephemeris_b200 import Context, PLANES as P
+    pl = _system(n, seed=25)
+    barred = pl.copy()
+    barred[P["DGM"], 1] = 1e-3
+    c = Context(0)
+    c.upload(barred)
+    c.autotune(600.0, 2, 2, True)
+    c.close()
+    c = Context(0)
+    c.upload(pl)
+    c.autotune(600.0, 2, 2, True)
+    c.integrate(600.0, 2)
+    out = c.download()
+    c.close()
+    assert np.array_equal(out, _go(pl, [("integrate", 600.0, 2)], False)[0])
+    assert not np.array_equal(out, _go(pl, [("integrate", 600.0, 2)], True)[0])

@@ -914,7 +914,7 @@ int eph_batch_upload(eph_batch *b, int32_t n_sys, const int64_t *n_body, const d
             }
         }
     }
-        if (tot) {
+    if (tot) {
         BCK(cudaMalloc(&b->d_planes, tot * sizeof(double)), "cudaMalloc(batch planes)");
         BCK(cudaMalloc(&b->d_store, tot_store * sizeof(double)), "cudaMalloc(batch stage store)");
         BCK(cudaMalloc(&b->d_sys, (size_t)n_sys * sizeof(BatchSys)), "cudaMalloc(batch table)");

@@ -375,79 +375,77 @@ __global__ void __launch_bounds__(kSLaunch, 1) serve_kernel(ServeArgs A) {
             const double *Xin = (phase == 2 ? X1 : X0) + slot;
             double rh[NC] = {}, rl[NC] = {}, vv[NC] = {};
             if (worker) {
-            if (k == 1) {
+                if (k == 1) {
 #pragma unroll
-                for (int ci = 0; ci < NC; ++ci)
-                    if (lane < 3 || !kSplit) {
-                        if (kSplit || lane == 0) F[(c0 + ci) * S] = phase == 2 ? fm[ci] : f0[ci];
-                    }
-                __syncwarp();
-            }
-            double s1[NC], s2[NC];
+                    for (int ci = 0; ci < NC; ++ci)
+                        if (kSplit ? lane < 3 : lane == 0) F[(c0 + ci) * S] = phase == 2 ? fm[ci] : f0[ci];
+                    __syncwarp();
+                }
+                double s1[NC], s2[NC];
 #pragma unroll
-            for (int ci = 0; ci < NC; ++ci) s1[ci] = s2[ci] = 0.0;
-            const int q1 = q_row[k + 1];
-            if (k < kStages) {
+                for (int ci = 0; ci < NC; ++ci) s1[ci] = s2[ci] = 0.0;
+                const int q1 = q_row[k + 1];
+                if (k < kStages) {
 #pragma unroll 4
-                for (int q = q_row[k]; q < q1; ++q) {
-                    const double2 a = ab[q];
+                    for (int q = q_row[k]; q < q1; ++q) {
+                        const double2 a = ab[q];
 #pragma unroll
-                    for (int ci = 0; ci < NC; ++ci) {
-                        const double f = F[li[q] + (c0 + ci) * S];
-                        s1[ci] = __fma_rn(a.x, f, s1[ci]);
-                        s2[ci] = __fma_rn(a.y, f, s2[ci]);
-                    }
-                }
-                const double ck = q_c[k];
-#pragma unroll
-                for (int ci = 0; ci < NC; ++ci) {
-                    const int c = c0 + ci;
-                    const double v0 = Xin[(6 + c) * S];
-                    double e;
-                    two_sum(Xin[c * S], hp * __fma_rn(ck, v0, hp * s1[ci]), rh[ci], e);
-                    rl[ci] = e + Xin[(3 + c) * S];
-                    vv[ci] = v0 + __fma_rn(hp, s2[ci], Xin[(9 + c) * S]);
-                }
-            } else {
-#pragma unroll 1
-                for (int q = q_row[k]; q < q1; ++q) {
-                    const double2 a = ab[q];
-#pragma unroll
-                    for (int ci = 0; ci < NC; ++ci) {
-                        const double f = F[li[q] + (c0 + ci) * S];
-                        s1[ci] = __fma_rn(a.x, f, s1[ci]);
-                        if (a.y != 0) s2[ci] = __dadd_rn(s2[ci], __dmul_rn(a.y, f));
-                    }
-                }
-                const dd ck = dd_make(q_c[k]), dh = dd_make(hp);
-                dd rn[NC], vn[NC];
-#pragma unroll
-                for (int ci = 0; ci < NC; ++ci) {
-                    const int c = c0 + ci;
-                    const dd v0 = dd{Xin[(6 + c) * S], Xin[(9 + c) * S]};
-                    const dd sv = dd_add(dd_mul(ck, v0), dd_make(hp * s1[ci]));
-                    rn[ci] = dd_add(dd{Xin[c * S], Xin[(3 + c) * S]}, dd_mul(dh, sv));
-                    vn[ci] = dd_add(v0, dd_make(hp * s2[ci]));
-                    rh[ci] = rn[ci].hi;
-                    rl[ci] = rn[ci].lo;
-                    vv[ci] = dd_val(vn[ci]);
-                }
-                __syncwarp();   // every lane of the group has read Xin before it is overwritten
-                double *Xout = (phase == 0 ? RF : X1) + slot;
-#pragma unroll
-                for (int ci = 0; ci < NC; ++ci) {
-                    const int c = c0 + ci;
-                    if (kSplit ? lane < 3 : lane == 0) {
-                        Xout[c * S] = rn[ci].hi;
-                        Xout[(3 + c) * S] = rn[ci].lo;
-                        if (phase > 0) {
-                            Xout[(6 + c) * S] = vn[ci].hi;
-                            Xout[(9 + c) * S] = vn[ci].lo;
+                        for (int ci = 0; ci < NC; ++ci) {
+                            const double f = F[li[q] + (c0 + ci) * S];
+                            s1[ci] = __fma_rn(a.x, f, s1[ci]);
+                            s2[ci] = __fma_rn(a.y, f, s2[ci]);
                         }
                     }
+                    const double ck = q_c[k];
+#pragma unroll
+                    for (int ci = 0; ci < NC; ++ci) {
+                        const int c = c0 + ci;
+                        const double v0 = Xin[(6 + c) * S];
+                        double e;
+                        two_sum(Xin[c * S], hp * __fma_rn(ck, v0, hp * s1[ci]), rh[ci], e);
+                        rl[ci] = e + Xin[(3 + c) * S];
+                        vv[ci] = v0 + __fma_rn(hp, s2[ci], Xin[(9 + c) * S]);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int q = q_row[k]; q < q1; ++q) {
+                        const double2 a = ab[q];
+#pragma unroll
+                        for (int ci = 0; ci < NC; ++ci) {
+                            const double f = F[li[q] + (c0 + ci) * S];
+                            s1[ci] = __fma_rn(a.x, f, s1[ci]);
+                            if (a.y != 0) s2[ci] = __dadd_rn(s2[ci], __dmul_rn(a.y, f));
+                        }
+                    }
+                    const dd ck = dd_make(q_c[k]), dh = dd_make(hp);
+                    dd rn[NC], vn[NC];
+#pragma unroll
+                    for (int ci = 0; ci < NC; ++ci) {
+                        const int c = c0 + ci;
+                        const dd v0 = dd{Xin[(6 + c) * S], Xin[(9 + c) * S]};
+                        const dd sv = dd_add(dd_mul(ck, v0), dd_make(hp * s1[ci]));
+                        rn[ci] = dd_add(dd{Xin[c * S], Xin[(3 + c) * S]}, dd_mul(dh, sv));
+                        vn[ci] = dd_add(v0, dd_make(hp * s2[ci]));
+                        rh[ci] = rn[ci].hi;
+                        rl[ci] = rn[ci].lo;
+                        vv[ci] = dd_val(vn[ci]);
+                    }
+                    __syncwarp();   // every lane of the group has read Xin before it is overwritten
+                    double *Xout = (phase == 0 ? RF : X1) + slot;
+#pragma unroll
+                    for (int ci = 0; ci < NC; ++ci) {
+                        const int c = c0 + ci;
+                        if (kSplit ? lane < 3 : lane == 0) {
+                            Xout[c * S] = rn[ci].hi;
+                            Xout[(3 + c) * S] = rn[ci].lo;
+                            if (phase > 0) {
+                                Xout[(6 + c) * S] = vn[ci].hi;
+                                Xout[(9 + c) * S] = vn[ci].lo;
+                            }
+                        }
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
-            }
             }
             if (k == kStages && phase == 0) {   // the whole step's end needs no acceleration
                 phase = 1;

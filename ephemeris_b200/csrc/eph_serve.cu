@@ -13,14 +13,14 @@
 // * Requests. A request is P particles (double-double position and velocity), a time span and a
 //   tolerance. It runs as one kernel launch of ceil(P G / 256) CTAs on one of the server's streams, G
 //   lanes per particle: the smallest power of two (at most 32) that spreads the request over one block per
-//   SM, so that a request's latency is that of one block's sequential stages (G = 32 below ~1200
-//   particles; 16 at 4096). Each CTA integrates its particles with
+//   SM, so that a request's latency is that of one block's sequential stages (G = 32 up to 2352
+//   particles, 16 up to 4704, 1 from 37633). Each CTA integrates its particles with
 //   a shared adaptive step: one RK12 step of h and two of h/2 (step doubling); the error is the largest
 //   |r_h - r_h/2| / |r_h/2 - r_0| over the CTA's particles (body 0 of the ephemeris is the central star);
 //   a step is accepted when it is at most tol, and the two half steps are kept; the next step is
-//   h * clamp(0.9 (tol / err)^(1/13), 0.2, 4). The reference has no adaptive integrator (its RK12 table
-//   has no embedded pair, RungeKutta.impl:38-104); step doubling with the same 25-stage method is the
-//   estimator.
+//   h * clamp(0.8 (tol / err)^(1/13), 0.25, 2), no larger right after a rejection. The reference has no
+//   adaptive integrator (its RK12 table has no embedded pair, RungeKutta.impl:38-104); step doubling with
+//   the same 25-stage method is the estimator.
 // * Admission. Requests queue on the host and launch while their device memory (state, stage store)
 //   fits: by default while the device's free memory (cudaMemGetInfo at admission) stays above a 1 GiB
 //   reserve, or within a fixed budget set by the caller; finished requests release their memory when their
@@ -276,7 +276,8 @@ __device__ __noinline__ v3 serve_accel(const double *PR, const double *SR2, int 
 // took 430 cycles a warp instead of 240. Requests alone, 360 days, against a body and channel per lane, the
 // perturbers before the sums and 128 registers: 5 particles 9.2 -> 3.7 ms, 300 (100 days) 10.4 -> 5.7, 4096 (60 days)
 // 20.9 -> 12.4; 100 requests at once 285 -> 219 ms (two blocks an SM: 216). 320 threads a block: 4.1, 6.4, 13.9, 243
-// ms; 512: 4.8, 6.6, 14.8, 255.
+// ms; 512: 4.8, 6.6, 14.8, 255. Requests of more blocks than SMs (30 days, one block an SM where there were two): 20,000
+// particles 61.8 -> 47.5 ms, 40,000 149 -> 119, 75,776 165.5 -> 155, 150,000 275 -> 246, 1,000,000 1563 -> 1474.
 template <int GT, bool kSoft>
 __global__ void __launch_bounds__(kSLaunch, 1) serve_kernel(ServeArgs A) {
     extern __shared__ __align__(16) double sm[];

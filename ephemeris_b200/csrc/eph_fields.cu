@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "eph_launch.cuh"
 #include "eph_models.cuh"
 #include "../../include/eph_b200.h"
 
@@ -83,10 +84,9 @@ extern "C" int eph_geopotential_field(int device, const double *coef, int nz, in
     if (rc == EPH_OK) {
         const int threads = 128;
         const long long blocks = (count * (lanes == 8 ? 8 : 1) + threads - 1) / threads;
-        if (lanes == 1) eph::gp_field_kernel<<<(unsigned)blocks, threads>>>(d_coef, nz, nt, R, count, d_r, d_out);
-        else if (lanes == 0) eph::gp_field_item_kernel<<<(unsigned)blocks, threads>>>(d_coef, nz, nt, R, count, d_r, d_out);
-        else eph::gp_field_lanes_kernel<<<(unsigned)blocks, threads>>>(d_coef, nz, nt, R, count, d_r, d_out);
-        if (cudaGetLastError() != cudaSuccess || cudaMemcpy(out, d_out, vb, cudaMemcpyDeviceToHost) != cudaSuccess)
+        auto kernel = lanes == 1 ? eph::gp_field_kernel : lanes == 0 ? eph::gp_field_item_kernel : eph::gp_field_lanes_kernel;
+        if (eph::launch_kernel(kernel, (unsigned)blocks, threads, 0, nullptr, d_coef, nz, nt, R, count, d_r, d_out) != cudaSuccess ||
+            cudaMemcpy(out, d_out, vb, cudaMemcpyDeviceToHost) != cudaSuccess)
             rc = EPH_ERR_CUDA;
     }
     cudaFree(d_coef);

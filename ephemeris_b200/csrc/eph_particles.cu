@@ -27,6 +27,7 @@
 #include <mutex>
 #include <vector>
 
+#include "eph_launch.cuh"
 #include "eph_math.cuh"
 #include "eph_models.cuh"
 #include "eph_rk12_host.h"
@@ -805,9 +806,8 @@ int eph_particles_integrate(eph_particles *p, double dt, int64_t n_step, double 
         A.next = p->d_next;
         PCK(cudaMemsetAsync(p->d_next, 0, sizeof(int), p->stream), "reset queue");
         PCK(cudaEventRecord(p->ev0, p->stream), "event");
-        void *args[] = {&A};   // (the launch's own status: cudaGetLastError may still hold an earlier call's error)
-        PCK(cudaLaunchKernel((const void *)kernel_of(p->general, p->mixed), dim3(p->grid), dim3(kPThreads), args,
-                             part_smem((int)p->n_pert), p->stream), "launch particle kernel");
+        PCK(launch_kernel(kernel_of(p->general, p->mixed), p->grid, kPThreads, part_smem((int)p->n_pert), p->stream, A),
+            "launch particle kernel");
         ++p->launches;
         PCK(cudaEventRecord(p->ev1, p->stream), "event");
         rc = next > 0 ? pert.end() : (int)EPH_OK;

@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "eph_bspline.h"
+#include "eph_launch.cuh"
 #include "eph_math.cuh"
 #include "eph_rk12_host.h"
 #include "eph_system.cuh"
@@ -785,8 +786,8 @@ static int pump(eph_serve *s) {
         A.soft = s->soft;
         A.buffers = serve_buffers(s->M, S, s->soft);
         // a full block's warps whatever the particles: the warps without any evaluate perturbers
-        serve_kernel_of(r.G, s->soft)<<<r.grid, kSLaunch, serve_smem(s->M, S, A.buffers, s->soft), st>>>(A);
-        SCK(cudaGetLastError(), "launch serve kernel");
+        SCK(launch_kernel(serve_kernel_of(r.G, s->soft), r.grid, kSLaunch, serve_smem(s->M, S, A.buffers, s->soft), st, A),
+            "launch serve kernel");
         SCK(cudaEventRecord(r.done, st), "record event");
         r.launched = true;
         s->in_use += r.bytes;
@@ -993,8 +994,7 @@ int eph_serve_eval(eph_serve *s, double t, double *out) {
     ServeArgs A{};
     A.coef = s->d_coef; A.gm = s->d_gm; A.sr2 = s->d_sr2; A.cheb = s->d_cheb;
     A.M = s->M; A.d = s->d; A.n = s->n; A.t0 = s->t0; A.knot = s->knot;
-    eval_kernel<<<1, kSThreads, (size_t)kSRec * s->M * sizeof(double), st>>>(A, t, d_out);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_kernel(eval_kernel, 1, kSThreads, (size_t)kSRec * s->M * sizeof(double), st, A, t, d_out);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d_out, (size_t)s->M * kChan * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(d_out, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1064,10 +1064,9 @@ int eph_bspline_fit_batch(int device, int d, int64_t n, int64_t mn, int channels
         rc = EPH_ERR_CUDA;
     if (!rc) {
         const int threads = 128;
-        bspline_solve_kernel<<<(unsigned)((T + threads - 1) / threads), threads>>>(
-            d, m, f.J, channels, n_series, (long long)(mn + 1) * channels, d_smp, d_jmin, d_cnt, d_bval, d_rw, d_lu, d_rd,
-            d_y, d_coef);
-        if ((e = cudaGetLastError()) != cudaSuccess ||
+        e = launch_kernel(bspline_solve_kernel, (unsigned)((T + threads - 1) / threads), threads, 0, nullptr, d, m, f.J, channels,
+                          n_series, (long long)(mn + 1) * channels, d_smp, d_jmin, d_cnt, d_bval, d_rw, d_lu, d_rd, d_y, d_coef);
+        if (e != cudaSuccess ||
             (e = cudaMemcpy(coefs, d_coef, n_coef * sizeof(double), cudaMemcpyDeviceToHost)) != cudaSuccess)
             rc = EPH_ERR_CUDA;
     }
@@ -1119,8 +1118,7 @@ int eph_record_samples(eph_ctx *ctx, double dt, int64_t n_step, int64_t stride, 
         ctx_record_stages(ctx, nullptr, 0);
         if (rc) break;
         const int take = (int)(c / stride);
-        gather_samples<<<256, 256>>>(d_traj, (int)n, take, stride - 1, (int)stride, d_out);
-        cudaError_t e = cudaGetLastError();
+        cudaError_t e = launch_kernel(gather_samples, 256, 256, 0, nullptr, d_traj, (int)n, take, stride - 1, (int)stride, d_out);
         if (e == cudaSuccess) e = cudaMemcpy(out + (size_t)written * n * kChan, d_out, (size_t)take * n * kChan * sizeof(double),
                                              cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) { rc = EPH_ERR_CUDA; break; }

@@ -64,3 +64,45 @@ def test_a_call_that_fails_leaves_the_time_and_the_set(tmp_path):
         p.close()
     assert got[0][2] == got[1][2]
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+def test_an_error_that_was_reported_fails_no_later_call(tmp_path):
+    """After a call that reported an error, every entry point that launches a kernel on the default stream or a stream of
+    its own runs as before."""
+    import torch
+    from ephemeris_b200 import Context, EphError, Server, bspline_fit_batch
+    sysm = _points(5)
+    pl, md, _, n = _combined(tmp_path, sysm, _cloud(sysm, 10, 9), "points")
+    pl = np.ascontiguousarray(pl[:, :n])
+    c = Context(0)
+    c.upload(pl, md)
+
+    def broken():
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="relaxed")
+            c.set_stream(stream.cuda_stream)
+            with pytest.raises(EphError):
+                c.integrate(4320.0, 1)
+            c.set_stream(None)
+            with pytest.raises(RuntimeError):
+                graph.capture_end()
+
+    broken()
+    samples, _ = c.record_samples(4320.0, 20, 1)
+    c.close()
+    c = Context(0)
+    c.upload(pl, md)
+    assert np.array_equal(samples, c.record_samples(4320.0, 20, 1)[0])
+    broken()
+    coefs = bspline_fit_batch(np.ascontiguousarray(samples.transpose(1, 0, 2)), 10, 3)
+    assert np.isfinite(coefs).all()
+    srv = Server(coefs, pl[39], 8640.0)
+    broken()
+    assert np.isfinite(srv.eval(8640.0)).all()
+    broken()
+    state = np.concatenate([pl[0:12, 1:2] + np.array([[1e10], [0], [0]] + [[0]] * 9)])
+    out, accepted, _ = srv.result(srv.submit(state, 0.0, 8640.0, tol=1e-12, h0=8640.0))
+    assert accepted >= 1 and np.isfinite(out).all()
+    srv.close()
+    c.close()
